@@ -179,9 +179,25 @@ __device__ float node_dmin(const PotRec *PO, int s, int n, const float *mc) {
     return (float)(bm + sqrt(bm * bm + sx / (n * 1.0)));
 }
 
-// leaves: mass and mass centre from their points (src/potential.c:101-113)
-__global__ void k_bh_leaf(const KNode<3> *nodes, int32_t nn, const PotRec *PO, double mp,
-                          BHNode *B) {
+// Mass and mass centre of every node (src/potential.c:101-123) in one pass
+// without levels: a thread per leaf sums its points, then climbs.  The first
+// of two siblings to reach their parent stops there; the second has both
+// children's values and merges them in the reference's order (left and right
+// have fixed places), so which one arrives last does not show in the result.
+// What bounds it is the longest climb: one fence, one atomic and two L2 reads
+// a level.  Two kernels per build level took 3.4 of 5.7 ms at 3,001 records,
+// nearly all of it launches and one thread walking a big node's points.
+__device__ __forceinline__ void bh_merge(const BHNode *B, const KNode<3> &x, BHNode &b) {
+    const BHNode *L = B + x.left, *R = L + 1;
+    const float lm = __ldcg(&L->m), rm = __ldcg(&R->m);
+    b.m = fadd(lm, rm);
+    for (int j = 0; j < 3; j++)
+        b.mc[j] = b.m ? __fdiv_rn(fadd(fmul(__ldcg(&R->mc[j]), rm), fmul(__ldcg(&L->mc[j]), lm)),
+                                  b.m)
+                      : 0.f;
+}
+__global__ void k_bh_climb(const KNode<3> *nodes, int32_t nn, const PotRec *PO, double mp,
+                           BHNode *B, int32_t *arrived) {
     int a = blockIdx.x * blockDim.x + threadIdx.x;
     if (a >= nn) return;
     const KNode<3> &x = nodes[a];
@@ -194,78 +210,87 @@ __global__ void k_bh_leaf(const KNode<3> *nodes, int32_t nn, const PotRec *PO, d
     for (int j = 0; j < 3; j++) b.mc[j] = pos[j] ? (float)(pos[j] / (double)x.n) : 0.f;
     b.dmin = node_dmin(PO, x.start, x.n, b.mc);
     B[a] = b;
-}
-// internal nodes of one build level (src/potential.c:115-123)
-__global__ void k_bh_internal(const KNode<3> *nodes, int32_t first, int32_t count,
-                              const PotRec *PO, BHNode *B) {
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= count) return;
-    int a = first + k;
-    const KNode<3> &x = nodes[a];
-    if (x.div < 0 || x.n > RSG_BH_BIG) return;
-    const BHNode &L = B[x.left], &R = B[x.left + 1];
-    BHNode b;
-    b.m = fadd(L.m, R.m);
-    for (int j = 0; j < 3; j++)
-        b.mc[j] = b.m ? __fdiv_rn(fadd(fmul(R.mc[j], R.m), fmul(L.mc[j], L.m)), b.m) : 0.f;
-    b.dmin = node_dmin(PO, x.start, x.n, b.mc);
-    B[a] = b;
+    for (int q = x.parent; q >= 0; q = nodes[q].parent) {
+        __threadfence();
+        if (atomicAdd(&arrived[q], 1) == 0) return;
+        __threadfence();
+        bh_merge(B, nodes[q], b);
+        B[q].m = b.m;
+        for (int j = 0; j < 3; j++) B[q].mc[j] = b.mc[j];
+    }
 }
 
-// Batched form: one warp per internal node of at most RSG_BH_BIG points,
-// the sum of squared distances reduced by shuffles.
-__global__ void k_bh_internal_warp(const KNode<3> *nodes, int32_t first, int32_t count,
-                                   const PotRec *PO, BHNode *B) {
-    int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (k >= count) return;
-    int a = first + k;
+// Opening radius of every internal node of at most RSG_BH_BIG points
+// (src/potential.c:71-82), one warp per node: lanes compute the squared
+// distances; the plain form adds them in point order (every lane runs the
+// same chain over the lanes' values), the batched form lane by lane and
+// then by shuffles.
+template <int EXACT>
+__global__ void __launch_bounds__(256) k_bh_dmin(const KNode<3> *nodes, int32_t nn,
+                                                 const PotRec *PO, BHNode *B) {
+    const int a = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (a >= nn) return;
     const KNode<3> &x = nodes[a];
     if (x.div < 0 || x.n > RSG_BH_BIG) return;
-    const BHNode &L = B[x.left], &R = B[x.left + 1];
-    BHNode b;
-    b.m = fadd(L.m, R.m);
-    for (int j = 0; j < 3; j++)
-        b.mc[j] = b.m ? __fdiv_rn(fadd(fmul(R.mc[j], R.m), fmul(L.mc[j], L.m)), b.m) : 0.f;
+    const float mc[3] = {B[a].mc[0], B[a].mc[1], B[a].mc[2]};
     double sx = 0, bm = 0;
-    for (int i = lane; i < x.n; i += 32) {
-        double dx = d2d(b.mc, PO[x.start + i].pos);
-        if (bm < dx) bm = dx;
-        sx += dx;
+    if (EXACT) {
+        for (int i0 = 0; i0 < x.n; i0 += 32) {
+            double dx = 0;
+            if (i0 + lane < x.n) dx = d2d(mc, PO[x.start + i0 + lane].pos);
+            if (bm < dx) bm = dx;
+            const int m = min(32, x.n - i0);
+            if (m == 32) {
+#pragma unroll
+                for (int t = 0; t < 32; t++) sx += __shfl_sync(0xffffffffu, dx, t);
+            } else {
+                for (int t = 0; t < m; t++) sx += __shfl_sync(0xffffffffu, dx, t);
+            }
+        }
+    } else {
+        for (int i = lane; i < x.n; i += 32) {
+            double dx = d2d(mc, PO[x.start + i].pos);
+            if (bm < dx) bm = dx;
+            sx += dx;
+        }
     }
     for (int o = 16; o; o >>= 1) {
-        sx += __shfl_xor_sync(0xffffffffu, sx, o);
+        if (!EXACT) sx += __shfl_xor_sync(0xffffffffu, sx, o);
         bm = fmax(bm, __shfl_xor_sync(0xffffffffu, bm, o));
     }
     if (lane == 0) {
         bm = sqrt(bm) / 2.0;
-        b.dmin = (float)(bm + sqrt(bm * bm + sx / (x.n * 1.0)));
-        B[a] = b;
+        B[a].dmin = (float)(bm + sqrt(bm * bm + sx / (x.n * 1.0)));
     }
+}
+
+// Internal nodes of more than RSG_BH_BIG points, listed with their sizes.
+__global__ void k_bh_big_flags(const KNode<3> *nodes, int32_t nn, int32_t *f) {
+    int a = blockIdx.x * blockDim.x + threadIdx.x;
+    if (a < nn) f[a] = nodes[a].div >= 0 && nodes[a].n > RSG_BH_BIG;
+}
+__global__ void k_bh_big_sizes(const KNode<3> *nodes, const int32_t *node, int32_t nn,
+                               int32_t *n) {
+    int j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j < nn) n[j] = nodes[node[j]].n;
 }
 
 // Batched form, internal nodes of more than Tuning::bh_huge points: one
 // block per chunk of `chunk` points forms the chunk's sum and maximum of
 // squared distances to the node's mass centre (part[item]); one thread per
 // node adds the chunks in order.  item = (node, chunk); the chunks of node j
-// of a level are items first[j] .. first[j + 1].
-__device__ __forceinline__ BHNode bh_merge(const BHNode &L, const BHNode &R) {
-    BHNode b;
-    b.m = fadd(L.m, R.m);
-    for (int j = 0; j < 3; j++)
-        b.mc[j] = b.m ? __fdiv_rn(fadd(fmul(R.mc[j], R.m), fmul(L.mc[j], L.m)), b.m) : 0.f;
-    return b;
-}
+// are items first[j] .. first[j + 1].
 __global__ void __launch_bounds__(256) k_bh_huge_part(const KNode<3> *nodes, const int2 *item,
                                                       int chunk, const PotRec *PO,
                                                       const BHNode *B, double2 *part) {
     __shared__ double s_s[8], m_s[8];
     const int2 it = item[blockIdx.x];
     const KNode<3> &x = nodes[it.x];
-    const BHNode b = bh_merge(B[x.left], B[x.left + 1]);
+    const float mc[3] = {B[it.x].mc[0], B[it.x].mc[1], B[it.x].mc[2]};
     const int i0 = it.y * chunk, i1 = min(x.n, i0 + chunk);
     double sx = 0, bm = 0;
     for (int i = i0 + threadIdx.x; i < i1; i += 256) {
-        double dx = d2d(b.mc, PO[x.start + i].pos);
+        double dx = d2d(mc, PO[x.start + i].pos);
         if (bm < dx) bm = dx;
         sx += dx;
     }
@@ -291,77 +316,68 @@ __global__ void k_bh_huge_fin(const KNode<3> *nodes, const int32_t *node, const 
     int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= nn) return;
     int a = node[j];
-    const KNode<3> &x = nodes[a];
-    BHNode b = bh_merge(B[x.left], B[x.left + 1]);
     double sx = 0, bm = 0;
     for (int c = first[j]; c < first[j + 1]; c++) {
         sx += part[c].x;
         bm = fmax(bm, part[c].y);
     }
     bm = sqrt(bm) / 2.0;
-    b.dmin = (float)(bm + sqrt(bm * bm + sx / (x.n * 1.0)));
-    B[a] = b;
-}
-__global__ void k_bh_huge_flags(const KNode<3> *nodes, int32_t nn, int huge, int32_t *f) {
-    int a = blockIdx.x * blockDim.x + threadIdx.x;
-    if (a < nn) f[a] = nodes[a].div >= 0 && nodes[a].n > huge;
-}
-__global__ void k_bh_huge_sizes(const KNode<3> *nodes, const int32_t *node, int32_t nn,
-                                int32_t *n) {
-    int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j < nn) n[j] = nodes[node[j]].n;
+    B[a].dmin = (float)(bm + sqrt(bm * bm + sx / (nodes[a].n * 1.0)));
 }
 
-// Large internal nodes: the block computes every point's squared distance
-// to the mass centre; the maximum is a reduction and the sum is added by one
-// thread in point order, as _compute_dmin does.
-__global__ void __launch_bounds__(256) k_bh_internal_big(const KNode<3> *nodes, int32_t first,
-                                                         int32_t count, const PotRec *PO, BHNode *B,
-                                                         int exact, int huge) {
-    __shared__ double dx_s[256];
-    __shared__ BHNode bs;
+// Large internal nodes (the list `node`), one block each: every point's
+// squared distance to the mass centre, their maximum a reduction.  The plain
+// form's sum is added in point order, as _compute_dmin does: the first warp
+// runs the chain over one buffer of distances while the other warps fill the
+// next, so that the chain's additions, not the loads, set its length.
+#define RSG_BHB 512  // points per buffer
+__global__ void __launch_bounds__(256) k_bh_dmin_big(const KNode<3> *nodes, const int32_t *node,
+                                                     const PotRec *PO, BHNode *B, int exact) {
+    __shared__ double dx_s[2][RSG_BHB];
     __shared__ double mx_s[8];
-    int a = first + blockIdx.x;
+    const int a = node[blockIdx.x];
     const KNode<3> &x = nodes[a];
-    if (x.div < 0 || x.n <= RSG_BH_BIG) return;
-    if (!exact && x.n > huge) return;  // k_bh_huge_*
-    if (threadIdx.x == 0) {
-        const BHNode &L = B[x.left], &R = B[x.left + 1];
-        bs.m = fadd(L.m, R.m);
-        for (int j = 0; j < 3; j++)
-            bs.mc[j] = bs.m ? __fdiv_rn(fadd(fmul(R.mc[j], R.m), fmul(L.mc[j], L.m)), bs.m) : 0.f;
-    }
-    __syncthreads();
+    const float mc[3] = {B[a].mc[0], B[a].mc[1], B[a].mc[2]};
+    const int s = x.start, n = x.n;
     double sx = 0, bm = 0;
-    for (int b0 = 0; b0 < x.n; b0 += 256) {
-        int i = b0 + threadIdx.x;
-        double dx = 0;
-        if (i < x.n) {
-            dx = d2d(bs.mc, PO[x.start + i].pos);
+    if (exact) {
+        auto fill = [&](int b0, int first, int step) {
+            for (int i = first; i < RSG_BHB && b0 + i < n; i += step) {
+                const double dx = d2d(mc, PO[s + b0 + i].pos);
+                if (bm < dx) bm = dx;
+                dx_s[(b0 / RSG_BHB) & 1][i] = dx;
+            }
+        };
+        fill(0, threadIdx.x, 256);
+        __syncthreads();
+        for (int b0 = 0; b0 < n; b0 += RSG_BHB) {
+            if (threadIdx.x >= 32) {
+                fill(b0 + RSG_BHB, threadIdx.x - 32, 224);
+            } else {
+                const double *d = dx_s[(b0 / RSG_BHB) & 1];
+                const int m = min(RSG_BHB, n - b0);
+                int t = 0;
+                for (; t + 16 <= m; t += 16) {
+#pragma unroll
+                    for (int u = 0; u < 16; u++) sx += d[t + u];
+                }
+                for (; t < m; t++) sx += d[t];
+            }
+            __syncthreads();
+        }
+    } else {
+        for (int i = threadIdx.x; i < n; i += 256) {
+            double dx = d2d(mc, PO[s + i].pos);
             if (bm < dx) bm = dx;
-        }
-        if (!exact) {
             sx += dx;
-            continue;
         }
-        dx_s[threadIdx.x] = dx;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            int m = min(256, x.n - b0);
-            for (int t = 0; t < m; t++) sx += dx_s[t];
-        }
-        __syncthreads();
-    }
-    if (!exact) {
         for (int o = 16; o; o >>= 1) sx += __shfl_down_sync(0xffffffffu, sx, o);
-        __syncthreads();
-        if ((threadIdx.x & 31) == 0) dx_s[threadIdx.x >> 5] = sx;
+        if ((threadIdx.x & 31) == 0) dx_s[0][threadIdx.x >> 5] = sx;
         __syncthreads();
         if (threadIdx.x == 0) {
             sx = 0;
-            for (int w = 0; w < 8; w++) sx += dx_s[w];
+            for (int w = 0; w < 8; w++) sx += dx_s[0][w];
         }
-        __syncthreads();
     }
     for (int o = 16; o; o >>= 1) bm = fmax(bm, __shfl_down_sync(0xffffffffu, bm, o));
     if ((threadIdx.x & 31) == 0) mx_s[threadIdx.x >> 5] = bm;
@@ -369,9 +385,7 @@ __global__ void __launch_bounds__(256) k_bh_internal_big(const KNode<3> *nodes, 
     if (threadIdx.x == 0) {
         for (int w = 1; w < 8; w++) bm = fmax(bm, mx_s[w]);
         bm = sqrt(bm) / 2.0;
-        BHNode b = bs;
-        b.dmin = (float)(bm + sqrt(bm * bm + sx / (x.n * 1.0)));
-        B[a] = b;
+        B[a].dmin = (float)(bm + sqrt(bm * bm + sx / (n * 1.0)));
     }
 }
 
@@ -1927,64 +1941,66 @@ void bh_potential(Arena &ar, PotRec *PO, int64_t npo, const int32_t *rs, const i
         return;
     }
     BHNode *B = ar.get<BHNode>(F.nnodes);
-    launch(k_bh_leaf, nblk(F.nnodes, T), T, 0, st, F.nodes, F.nnodes, PO, mp, B);
-    // batched form: the nodes of more than bh_huge points, by level, and
-    // their chunks (node ids ascend with the level index in the forest)
-    const int huge = tuning().bh_huge, chunk = tuning().bh_chunk;
-    std::vector<int32_t> hn_node, hn_first(1, 0);  // per huge node: id, first item
-    std::vector<int2> hitem;
-    int2 *d_item = nullptr;
-    int32_t *d_hnode = nullptr, *d_hfirst = nullptr;
-    double2 *d_part = nullptr;
-    if (!exact) {
-        int32_t *hf = ar.get<int32_t>(F.nnodes), *hid = ar.get<int32_t>(F.nnodes);
-        launch(k_bh_huge_flags, nblk(F.nnodes, T), T, 0, st, F.nodes, F.nnodes, huge, hf);
-        int32_t nh = select_idx(ar, hf, hid, F.nnodes, st);
-        if (nh) {
-            int32_t *hsz = ar.get<int32_t>(nh);
-            launch(k_bh_huge_sizes, nblk(nh, T), T, 0, st, F.nodes, hid, nh, hsz);
-            std::vector<int32_t> sz(nh);
-            hn_node.resize(nh);
-            RSG_CUDA(cudaMemcpyAsync(hn_node.data(), hid, 4 * nh, cudaMemcpyDeviceToHost, st));
-            RSG_CUDA(cudaMemcpyAsync(sz.data(), hsz, 4 * nh, cudaMemcpyDeviceToHost, st));
+    int32_t *big = ar.get<int32_t>(F.nnodes);
+    {
+        int32_t *arrived = ar.get<int32_t>(F.nnodes);
+        RSG_CUDA(cudaMemsetAsync(arrived, 0, sizeof(int32_t) * F.nnodes, st));
+        launch(k_bh_climb, nblk(F.nnodes, T), T, 0, st, F.nodes, F.nnodes, PO, mp, B, arrived);
+        const int db = nblk((int64_t)F.nnodes * 32, T);
+        if (exact)
+            launch(k_bh_dmin<1>, db, T, 0, st, F.nodes, F.nnodes, PO, B);
+        else
+            launch(k_bh_dmin<0>, db, T, 0, st, F.nodes, F.nnodes, PO, B);
+        // the nodes above a warp's size: a block each, or, in the batched
+        // form above bh_huge points, a block per chunk
+        launch(k_bh_big_flags, nblk(F.nnodes, T), T, 0, st, F.nodes, F.nnodes, arrived);
+        const int32_t nbig = select_idx(ar, arrived, big, F.nnodes, st);
+        if (nbig && exact) {
+            launch(k_bh_dmin_big, nbig, 256, 0, st, F.nodes, (const int32_t *)big, PO, B, 1);
+        } else if (nbig) {
+            const int huge = tuning().bh_huge, chunk = tuning().bh_chunk;
+            int32_t *bsz = ar.get<int32_t>(nbig);
+            launch(k_bh_big_sizes, nblk(nbig, T), T, 0, st, F.nodes, (const int32_t *)big, nbig,
+                   bsz);
+            std::vector<int32_t> id(nbig), sz(nbig), mid, hnode, hfirst(1, 0);
+            std::vector<int2> hitem;
+            RSG_CUDA(cudaMemcpyAsync(id.data(), big, 4 * nbig, cudaMemcpyDeviceToHost, st));
+            RSG_CUDA(cudaMemcpyAsync(sz.data(), bsz, 4 * nbig, cudaMemcpyDeviceToHost, st));
             RSG_CUDA(cudaStreamSynchronize(st));
-            for (int32_t j = 0; j < nh; j++) {
-                int nc = (sz[j] + chunk - 1) / chunk;
-                for (int c = 0; c < nc; c++) hitem.push_back(make_int2(hn_node[j], c));
-                hn_first.push_back((int32_t)hitem.size());
+            for (int32_t j = 0; j < nbig; j++) {
+                if (sz[j] <= huge) {
+                    mid.push_back(id[j]);
+                    continue;
+                }
+                const int nc = (sz[j] + chunk - 1) / chunk;
+                for (int c = 0; c < nc; c++) hitem.push_back(make_int2(id[j], c));
+                hnode.push_back(id[j]);
+                hfirst.push_back((int32_t)hitem.size());
             }
-            d_item = ar.get<int2>(hitem.size());
-            d_part = ar.get<double2>(hitem.size());
-            d_hnode = ar.get<int32_t>(nh);
-            d_hfirst = ar.get<int32_t>(nh + 1);
-            RSG_CUDA(cudaMemcpyAsync(d_item, hitem.data(), sizeof(int2) * hitem.size(),
-                                     cudaMemcpyHostToDevice, st));
-            RSG_CUDA(cudaMemcpyAsync(d_hnode, hn_node.data(), 4 * nh, cudaMemcpyHostToDevice, st));
-            RSG_CUDA(cudaMemcpyAsync(d_hfirst, hn_first.data(), 4 * (nh + 1),
-                                     cudaMemcpyHostToDevice, st));
-        }
-    }
-    size_t hj = hn_node.size();  // huge nodes not yet done (taken from the back: deepest first)
-    for (int l = F.nlv - 2; l >= 0; l--) {
-        int32_t a = F.lv_first[l], b = F.lv_first[l + 1];
-        if (b > a) {
-            if (exact)
-                launch(k_bh_internal, nblk(b - a, 64), 64, 0, st, F.nodes, a, b - a, PO, B);
-            else
-                launch(k_bh_internal_warp, nblk((int64_t)(b - a) * 32, 256), 256, 0, st, F.nodes, a,
-                       b - a, PO, B);
-            launch(k_bh_internal_big, b - a, 256, 0, st, F.nodes, a, b - a, PO, B, exact, huge);
-            size_t j1 = hj;
-            while (hj > 0 && hn_node[hj - 1] >= a) hj--;
-            if (j1 > hj) {
-                int32_t i0 = hn_first[hj], i1 = hn_first[j1];
-                launch(k_bh_huge_part, i1 - i0, 256, 0, st, F.nodes, (const int2 *)d_item + i0,
-                       chunk, PO, (const BHNode *)B, d_part + i0);
-                launch(k_bh_huge_fin, nblk((int)(j1 - hj), 64), 64, 0, st, F.nodes,
-                       (const int32_t *)d_hnode + hj, (const int32_t *)d_hfirst + hj,
-                       (int32_t)(j1 - hj), (const double2 *)d_part, B);
+            if (!mid.empty()) {
+                RSG_CUDA(cudaMemcpyAsync(big, mid.data(), 4 * mid.size(), cudaMemcpyHostToDevice,
+                                         st));
+                launch(k_bh_dmin_big, (unsigned)mid.size(), 256, 0, st, F.nodes,
+                       (const int32_t *)big, PO, B, 0);
+            }
+            if (!hnode.empty()) {
+                const int32_t nh = (int32_t)hnode.size();
+                int2 *d_item = ar.get<int2>(hitem.size());
+                double2 *d_part = ar.get<double2>(hitem.size());
+                int32_t *d_hnode = ar.get<int32_t>(nh), *d_hfirst = ar.get<int32_t>(nh + 1);
+                RSG_CUDA(cudaMemcpyAsync(d_item, hitem.data(), sizeof(int2) * hitem.size(),
+                                         cudaMemcpyHostToDevice, st));
+                RSG_CUDA(cudaMemcpyAsync(d_hnode, hnode.data(), 4 * nh, cudaMemcpyHostToDevice,
+                                         st));
+                RSG_CUDA(cudaMemcpyAsync(d_hfirst, hfirst.data(), 4 * (nh + 1),
+                                         cudaMemcpyHostToDevice, st));
+                launch(k_bh_huge_part, (unsigned)hitem.size(), 256, 0, st, F.nodes,
+                       (const int2 *)d_item, chunk, PO, (const BHNode *)B, d_part);
+                launch(k_bh_huge_fin, nblk(nh, 64), 64, 0, st, F.nodes, (const int32_t *)d_hnode,
+                       (const int32_t *)d_hfirst, nh, (const double2 *)d_part, B);
             }
         }
+        RSG_CHECK_LAUNCH();
     }
     phase_mark(st, "p.bh_mass");
     int32_t *lf = ar.get<int32_t>(F.nnodes), *leaves = ar.get<int32_t>(F.nnodes);
