@@ -69,27 +69,31 @@ __global__ void k_iota_i32(int32_t *a, int32_t n) {
 }
 // After k_children: the level's new nodes become [base, base + nnew), and
 // those that split again are the next level's active nodes.
-__global__ void k_level_advance(LevelState *ls, const int64_t *off, int32_t *lvl_end,
-                                int32_t level) {
+__global__ void k_level_advance(LevelState *ls, const int64_t *off) {
     if (threadIdx.x || blockIdx.x) return;
     const int64_t t = off[ls->nact];
     ls->base = ls->nnodes;
     ls->nnew = ls->err ? 0 : 2 * (int32_t)(t >> 32);
     ls->nnodes += ls->nnew;
     ls->nact = ls->err ? 0 : (int32_t)(t & 0xffffffffu);
-    lvl_end[level] = ls->nnodes;
 }
 
-__global__ void k_root_owner(const int32_t *rstart, const int32_t *rn, int32_t ntrees, int leaf,
+__global__ void k_root_owner(const int32_t *rstart, const int32_t *rn, int32_t ntrees, int sub,
                              int32_t *owner, int32_t *box_owner) {
     int t = blockIdx.x;  // tree; blockIdx.y strides through its elements
     if (t >= ntrees) return;
     int s = rstart[t], n = rn[t];
-    int o = n > leaf ? t : -1;
+    if (n <= sub) return;  // the whole tree is one block's (k_sub_build)
     for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < n; i += gridDim.y * blockDim.x) {
         box_owner[s + i] = t;
-        owner[s + i] = o;
+        owner[s + i] = t;
     }
+}
+// Whole trees of at most `sub` records go to the block-built subtrees.
+__global__ void k_root_subs(const int32_t *rn, int32_t ntrees, int sub, int sub0, SubRoot *subs,
+                            int32_t nsubs, LevelState *ls) {
+    int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < ntrees && rn[t] <= sub) list_sub(subs, nsubs, ls, sub0, t, rn[t], 0);
 }
 
 // ---- phase timers ----------------------------------------------------------

@@ -61,7 +61,7 @@ struct PosOf<MetricRec, D> {
     __device__ static float get(const MetricRec &r, int d) { return r.pos[d]; }
 };
 
-#define RSG_FOREST_LEVELS 4096  // deepest build accepted (checked by build_forest)
+#define RSG_FOREST_LEVELS 4096  // deepest build accepted
 
 // Device-side state of a forest build: the level's active count and the
 // node bookkeeping, so that levels run back to back without a host round
@@ -71,8 +71,13 @@ struct LevelState {
     int32_t nnodes;  // nodes created so far
     int32_t base;    // first node created by the last level
     int32_t nnew;    // nodes created by the last level
-    int32_t err;     // node capacity exceeded
-    int32_t pad[3];
+    int32_t err;     // 1: node capacity exceeded, 2: too many levels
+    int32_t nsub[2]; // subtrees listed for each size class of k_sub_build
+    int32_t pad;
+};
+// A subtree that one block builds (k_sub_build): its root and the root's level.
+struct SubRoot {
+    int32_t node, level;
 };
 
 template <int D>
@@ -80,11 +85,6 @@ struct Forest {
     KNode<D> *nodes = nullptr;  // nodes[t] is the root of tree t
     int32_t nnodes = 0;
     int32_t ntrees = 0;
-    // nodes created by level l of the build are [lv_first[l], lv_first[l+1]),
-    // l < nlv - 1; a fixed table so a build touches no host heap
-    int32_t lv_first[RSG_FOREST_LEVELS + 2];
-    int32_t nlv = 0;
-    void level_end(int32_t first) { lv_first[nlv++] = first; }
 };
 
 // ---- kernels ------------------------------------------------------------
@@ -214,16 +214,27 @@ __global__ void k_scatter(const KNode<D> *nodes, const RecT *src, RecT *dst, int
 }
 
 
+// Lists a subtree of n records for k_sub_build: class 0 (n <= sub0) from the
+// front of `subs`, class 1 from its back.
+__device__ __forceinline__ void list_sub(SubRoot *subs, int32_t nsubs, LevelState *ls, int sub0,
+                                         int32_t node, int32_t n, int32_t level) {
+    const int c = n > sub0;
+    const int at = atomicAdd(&ls->nsub[c], 1);
+    subs[c ? nsubs - 1 - at : at] = SubRoot{node, level};
+}
+
 // Split bookkeeping (src/fast3tree.c:798-846): create children for nodes
 // with 0 < m < n, turn the rest into leaves.  off[k] packs, over the active
-// nodes before k, the splits (high 32 bits) and the children that split
-// again (low 32 bits): node k's children go to nodes[ls->nnodes + 2 * splits]
-// and those holding more than `leaf` records to next[children], which is the
-// order a selection over the new nodes gives.  A level that would pass `cap`
-// nodes sets ls->err and changes nothing.
+// nodes before k, the splits (high 32 bits) and the children that this loop
+// splits again (low 32 bits): node k's children go to nodes[ls->nnodes + 2 *
+// splits], those of more than `sub` records to next[children] (the order a
+// selection over the new nodes gives), the others of more than `leaf` to the
+// list of block-built subtrees.  A level that would pass `cap` nodes sets
+// ls->err and changes nothing.
 template <int D>
 __global__ void k_children(KNode<D> *nodes, const int32_t *act, LevelState *ls,
                            const int32_t *m_arr, const int64_t *off, int32_t cap, int leaf,
+                           int sub, int sub0, int32_t level, SubRoot *subs, int32_t nsubs,
                            int32_t *next, unsigned *bmin, unsigned *bmax) {
     int k = blockIdx.x * blockDim.x + threadIdx.x;
     const int nact = ls->nact, base = ls->nnodes;
@@ -243,8 +254,10 @@ __global__ void k_children(KNode<D> *nodes, const int32_t *act, LevelState *ls,
     int l = base + 2 * (int)(off[k] >> 32);
     int na = (int)(off[k] & 0xffffffffu);
     nd.left = l;
-    if (m > leaf) next[na++] = l;
-    if (nd.n - m > leaf) next[na] = l + 1;
+    if (m > sub) next[na++] = l;
+    else if (m > leaf) list_sub(subs, nsubs, ls, sub0, l, m, level);
+    if (nd.n - m > sub) next[na] = l + 1;
+    else if (nd.n - m > leaf) list_sub(subs, nsubs, ls, sub0, l + 1, nd.n - m, level);
     for (int c = 0; c < 2; c++) {
         KNode<D> &ch = nodes[l + c];
         ch.start = nd.start + (c ? m : 0);
@@ -261,12 +274,13 @@ __global__ void k_children(KNode<D> *nodes, const int32_t *act, LevelState *ls,
 }
 
 // Element owner update: elements of split nodes move to their child.  The
-// levels scatter between two buffers; an element whose node stops splitting
-// is final now, and is copied from the buffer the level wrote (cur) to the
-// output array (out) when they differ -- once per element, not once per level.
+// levels scatter between two buffers; an element whose node these levels do
+// not split again (a leaf, or a subtree of at most `sub` records left to
+// k_sub_build) is copied from the buffer the level wrote (cur) to the output
+// array (out) when they differ -- once per element, not once per level.
 template <int D, class RecT>
 __global__ void k_owner_update(const KNode<D> *nodes, int64_t nrec, int32_t *owner,
-                               int32_t *box_owner, int leaf, const RecT *cur, RecT *out) {
+                               int32_t *box_owner, int sub, const RecT *cur, RecT *out) {
     int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= nrec) return;
     int a = owner[i];
@@ -284,17 +298,17 @@ __global__ void k_owner_update(const KNode<D> *nodes, int64_t nrec, int32_t *own
     int l = nd.left;
     int c = (i - nd.start) < nodes[l].n ? l : l + 1;
     box_owner[i] = c;
-    bool fin = nodes[c].n <= leaf;
+    bool fin = nodes[c].n <= sub;
     owner[i] = fin ? -1 : c;
     if (fin && cur != out) out[i] = cur[i];
 }
 
 // sflag[0 .. ub]: per active node, split (high 32 bits) and children that
-// split again (low 32 bits); 0 beyond the level's active count (ub bounds it
-// from above).
+// the level loop splits again (low 32 bits); 0 beyond the level's active count
+// (ub bounds it from above).
 template <int D>
 __global__ void k_split_flags(const int32_t *m_arr, const KNode<D> *nodes, const int32_t *act,
-                              const LevelState *ls, int32_t ub, int leaf, int64_t *sflag) {
+                              const LevelState *ls, int32_t ub, int sub, int64_t *sflag) {
     int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k > ub) return;
     if (k >= ls->nact) {
@@ -303,13 +317,12 @@ __global__ void k_split_flags(const int32_t *m_arr, const KNode<D> *nodes, const
     }
     int m = m_arr[k], n = nodes[act[k]].n;
     int64_t v = 0;
-    if (m > 0 && m < n) v = ((int64_t)1 << 32) | (int64_t)((m > leaf) + (n - m > leaf));
+    if (m > 0 && m < n) v = ((int64_t)1 << 32) | (int64_t)((m > sub) + (n - m > sub));
     sflag[k] = v;
 }
 
 __global__ void k_slot_set(const int32_t *act, const LevelState *ls, int32_t *slot);
-__global__ void k_level_advance(LevelState *ls, const int64_t *off, int32_t *lvl_end,
-                                int32_t level);
+__global__ void k_level_advance(LevelState *ls, const int64_t *off);
 
 // Builds a kd-forest over recs[0..nrec) whose trees are the segments
 // (rstart[t], rn[t]) (device arrays).  Elements outside every segment are
