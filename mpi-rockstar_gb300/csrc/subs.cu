@@ -141,75 +141,72 @@ __global__ void k_norm_seq(Rec *W, HierNodes N, int32_t base, int32_t count, int
     norm_sigmas(c, level0, ims, sig + 2 * k);
 }
 
-// Batched form, nodes up to RSG_SMALL particles: 32 nodes per warp.  For
-// each node in turn the lanes stride over its particles: the means and the
-// centred coordinates float((double)x - mean) in FP64, as the reference
-// forms them (a double-float mean or centring moved coordinates by an ulp
-// measurably more often), and the 21 second moments of the float products as
-// float pairs on the FP32 pipe (hi + lo, Knuth's two-sum: about 48 bits,
-// enough for RSG_SMALL terms); the lanes' sums are combined by shuffles
-// (deterministic).  Then the 32 nodes' sigmas (two 3x3 eigenvalue
-// problems each, in FP64) run side by side, one node per lane, instead of on
-// lane 0 of a warp per node.
-#define RSG_NORM_WARPS 4
-__global__ void __launch_bounds__(RSG_NORM_WARPS * 32)
-    k_norm_warp(Rec *W, HierNodes N, int32_t base, int32_t count, int level0, double ims,
-                double *sig) {
-    __shared__ double cs[RSG_NORM_WARPS][32][21];
+// Batched form, nodes up to RSG_SMALL particles, moments: one warp per node,
+// its lanes striding over the particles: the means and the centred
+// coordinates float((double)x - mean) in FP64, as the reference forms them (a
+// double-float mean or centring moved coordinates by an ulp measurably more
+// often), and the 21 second moments of the float products as float pairs on
+// the FP32 pipe (hi + lo, Knuth's two-sum: about 48 bits, enough for
+// RSG_SMALL terms); the lanes' sums are combined by shuffles (deterministic).
+// The sigmas (two 3x3 eigenvalue problems per node, a long FP64 chain) follow
+// one node per thread in k_norm_sig, so that neither part waits on the
+// other's shape: with 32 nodes in turn on one warp and their sigmas side by
+// side behind them, a level of a 64^3 snapshot took 0.68 ms, two thirds of
+// the chip's SMs without a warp; now 0.1 ms.
+__global__ void __launch_bounds__(128) k_norm_mom(Rec *W, HierNodes N, int32_t base,
+                                                  int32_t count, double *mom) {
     const unsigned FULL = 0xffffffffu;
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int32_t k0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32;
-    if (k0 >= count) return;
-    for (int q = 0; q < 32; q++) {
-        const int32_t k = k0 + q;
-        if (k >= count) break;
-        const int node = base + k;
-        const int s = N.start[node], n = N.n[node];
-        if (n <= 0 || n > RSG_SMALL) continue;
-        double acc[6] = {0, 0, 0, 0, 0, 0};
-        for (int i = lane; i < n; i += 32)
+    const int lane = threadIdx.x & 31;
+    const int32_t k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (k >= count) return;
+    const int s = N.start[base + k], n = N.n[base + k];
+    if (n <= 0 || n > RSG_SMALL) return;
+    double acc[6] = {0, 0, 0, 0, 0, 0};
+    for (int i = lane; i < n; i += 32)
 #pragma unroll
-            for (int d = 0; d < 6; d++) acc[d] += (double)W[s + i].pos[d];
-        double mean[6];
+        for (int d = 0; d < 6; d++) acc[d] += (double)W[s + i].pos[d];
+    double mean[6];
+#pragma unroll
+    for (int d = 0; d < 6; d++) {
+        for (int o = 16; o; o >>= 1) acc[d] += __shfl_xor_sync(FULL, acc[d], o);
+        mean[d] = acc[d] / (double)n;
+    }
+    float ch[21], cl[21];
+#pragma unroll
+    for (int jj = 0; jj < 21; jj++) ch[jj] = cl[jj] = 0.f;
+    for (int i = lane; i < n; i += 32) {
+        float qv[6];
 #pragma unroll
         for (int d = 0; d < 6; d++) {
-            for (int o = 16; o; o >>= 1) acc[d] += __shfl_xor_sync(FULL, acc[d], o);
-            mean[d] = acc[d] / (double)n;
+            qv[d] = __double2float_rn((double)W[s + i].pos[d] - mean[d]);
+            W[s + i].pos[d] = qv[d];
         }
-        float ch[21], cl[21];
-        for (int jj = 0; jj < 21; jj++) ch[jj] = cl[jj] = 0.f;
-        for (int i = lane; i < n; i += 32) {
-            float qv[6];
+        int jj = 0;
 #pragma unroll
-            for (int d = 0; d < 6; d++) {
-                qv[d] = __double2float_rn((double)W[s + i].pos[d] - mean[d]);
-                W[s + i].pos[d] = qv[d];
-            }
-            int jj = 0;
-            for (int x = 0; x < 6; x++)
-                for (int y = x; y < 6; y++, jj++) two_sum_acc(ch[jj], cl[jj], fmul(qv[x], qv[y]));
-        }
-        for (int jj = 0; jj < 21; jj++) {
-            for (int o = 16; o; o >>= 1) {
-                float h2 = __shfl_xor_sync(FULL, ch[jj], o);
-                float l2 = __shfl_xor_sync(FULL, cl[jj], o);
-                two_sum_acc(ch[jj], cl[jj], h2);
-                cl[jj] = fadd(cl[jj], l2);
-            }
-        }
-        if (lane < 21) {
-            double v = 0;
-            for (int jj = 0; jj < 21; jj++)
-                if (jj == lane) v = ((double)ch[jj] + (double)cl[jj]) / (double)n;
-            cs[w][q][lane] = v;
-        }
+        for (int x = 0; x < 6; x++)
+#pragma unroll
+            for (int y = x; y < 6; y++, jj++) two_sum_acc(ch[jj], cl[jj], fmul(qv[x], qv[y]));
     }
-    __syncwarp();
-    const int32_t k = k0 + lane;
-    if (k < count) {
-        const int n = N.n[base + k];
-        if (n > 0 && n <= RSG_SMALL) norm_sigmas(cs[w][lane], level0, ims, sig + 2 * k);
+#pragma unroll
+    for (int jj = 0; jj < 21; jj++) {
+        for (int o = 16; o; o >>= 1) {
+            float h2 = __shfl_xor_sync(FULL, ch[jj], o);
+            float l2 = __shfl_xor_sync(FULL, cl[jj], o);
+            two_sum_acc(ch[jj], cl[jj], h2);
+            cl[jj] = fadd(cl[jj], l2);
+        }
+        if (lane == jj) mom[(int64_t)jj * count + k] = ((double)ch[jj] + (double)cl[jj]) / (double)n;
     }
+}
+__global__ void k_norm_sig(HierNodes N, int32_t base, int32_t count, const double *mom,
+                           int level0, double ims, double *sig) {
+    const int32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= count) return;
+    const int n = N.n[base + k];
+    if (n <= 0 || n > RSG_SMALL) return;
+    double c[21];
+    for (int j = 0; j < 21; j++) c[j] = mom[(int64_t)j * count + k];
+    norm_sigmas(c, level0, ims, sig + 2 * k);
 }
 
 // Mid-size nodes: the block stages particles in shared memory and computes
@@ -2498,12 +2495,17 @@ SubsOut find_subs_device(Arena &ar, rsg_particle *d_p, int64_t num_p, const int6
         launch(k_fill_eln, cnt, T, 0, st, N, base, eln);
         {
             double *sig = ar.get<double>(2 * (int64_t)cnt);
-            if (exact)
+            if (exact) {
                 launch(k_norm_seq, nblk(cnt, 32), 32, 0, st, W, N, base, cnt, L == 0,
                        cfg.initial_metric_scaling, sig);
-            else
-                launch(k_norm_warp, nblk(cnt, RSG_NORM_WARPS * 32), RSG_NORM_WARPS * 32, 0, st, W,
-                       N, base, cnt, L == 0, cfg.initial_metric_scaling, sig);
+            } else {
+                size_t m0 = ar.used;
+                double *mom = ar.get<double>(21 * (int64_t)cnt);
+                launch(k_norm_mom, nblk((int64_t)cnt * 32, 128), 128, 0, st, W, N, base, cnt, mom);
+                launch(k_norm_sig, nblk(cnt, 32), 32, 0, st, N, base, cnt, (const double *)mom,
+                       L == 0, cfg.initial_metric_scaling, sig);
+                ar.used = m0;
+            }
             launch(k_norm_blk, cnt, 256, 0, st, W, N, base, L == 0, cfg.initial_metric_scaling, sig,
                    seq_lo, RSG_SEQ_MAX);
             if (exact) {
