@@ -533,12 +533,15 @@ Forest<D> build_forest(Arena &ar, RecT *recs, int64_t nrec, const int32_t *rstar
     // counts on the device; the host reads the state every RSG_FOREST_BATCH
     // levels.  Grids are sized by an upper bound of the active count (ub): at
     // most twice the previous level's, and at most one per sub + 1 records.
+    // A level past the last costs passes over nrec records, so large calls
+    // read after every level.
+    const int batch = nrec > (1 << 22) ? 1 : RSG_FOREST_BATCH;
     int64_t ub = hs.nact;
     int level = 0;
     RecT *buf[2] = {recs, tmp};  // levels scatter back and forth between these
     int cur = 0;
     while (hs.nact > 0) {
-        for (int b = 0; b < RSG_FOREST_BATCH && ub > 0; b++) {
+        for (int b = 0; b < batch && ub > 0; b++) {
             if (++level > RSG_FOREST_LEVELS) {
                 set_error(RSG_ERR_LIMIT, "kd-forest build exceeded %d levels", RSG_FOREST_LEVELS);
                 throw Failure();
