@@ -41,9 +41,9 @@ struct __align__(16) Rec {
 static_assert(sizeof(Rec) == 32, "Rec must be 32 bytes");
 
 // Node of a median-of-extent kd-tree (layout of src/fast3tree.c:184-193,
-// indices instead of pointers).
+// indices instead of pointers), aligned so that a copy takes 16-byte loads.
 template <int D>
-struct KNode {
+struct __align__(16) KNode {
     float mn[D], mx[D];
     int32_t start, n;
     int32_t div;     // split dimension, -1 for a leaf

@@ -22,6 +22,8 @@
 // included.
 #include <limits.h>
 
+#include <algorithm>
+
 #include <cooperative_groups.h>
 #include <cub/cub.cuh>
 #include <thrust/binary_search.h>
@@ -128,25 +130,9 @@ __device__ bool sphere3(const KNode<3> *nodes, int root, const Rec *recs, const 
 // returning false ends that lane's walk; nodes holding no index after the
 // lane's `after` are dropped for that lane (the points it finds after
 // `after` are unchanged).
-// on_leaf(j, hit), when given (LEAF = true), replaces on_point for leaf
-// points: every lane calls it for every point of a leaf any lane tests, in
-// converged code, with hit telling whether the point is in this lane's
-// sphere (warp-level ballots inside it are safe).  It cannot end a walk.
-struct NoLeaf {
-    __device__ void operator()(int, bool) const {}
-};
-// on_coop(m2, start, n), when given (COOP = true), replaces on_range: every
-// lane calls it, in converged code, for a node that the lanes of mask m2 take
-// whole (all of them meet the same node in a shared walk), so the warp can
-// work through the node's points together.  It cannot end a walk.
-struct NoCoop {
-    __device__ void operator()(unsigned, int, int) const {}
-};
-template <class FR, class FP, bool LEAF = false, class FL = NoLeaf, bool COOP = false,
-          class FC = NoCoop>
+template <class FR, class FP>
 __device__ void sphere3_warp(const KNode<3> *nodes, const Rec *recs, const float *c, bool active,
-                             float r, int after, int *errflag, FR on_range, FP on_point,
-                             FL on_leaf = FL(), FC on_coop = FC()) {
+                             float r, int after, int *errflag, FR on_range, FP on_point) {
     const unsigned FULL = 0xffffffffu;
     const unsigned bit = 1u << (threadIdx.x & 31);
     const float r2 = fmul(r, r);
@@ -170,20 +156,12 @@ __device__ void sphere3_warp(const KNode<3> *nodes, const Rec *recs, const float
                 kind = box_inside3(nd, c, r, r2) ? 2 : (nd.div < 0 ? 3 : 4);
         }
         bool stop = false;
-        if (COOP) {
-            const unsigned m2 = __ballot_sync(FULL, kind == 2);
-            if (m2) on_coop(m2, nd.start, nd.n);
-        } else if (kind == 2) {
-            stop = !on_range(nd.start, nd.n);
-        }
+        if (kind == 2) stop = !on_range(nd.start, nd.n);
         if (__any_sync(FULL, kind == 3)) {
             const unsigned long long cxy = f2_pack(c[0], c[1]);
             for (int k = 0; k < nd.n; k++) {
                 int j = nd.start + k;
-                bool hit = false;
-                if (kind == 3 && !stop) hit = dist3_p(cxy, c[2], recs[j]) < r2;
-                if (LEAF) on_leaf(j, hit);
-                else if (hit) stop = !on_point(j);
+                if (kind == 3 && !stop && dist3_p(cxy, c[2], recs[j]) < r2) stop = !on_point(j);
             }
         }
         live &= ~__ballot_sync(FULL, stop);
@@ -377,79 +355,305 @@ __global__ void __launch_bounds__(128) k_count_w(const KNode<3> *nodes, const Re
         [&](int j) { k++; return k <= 16; });
     if (act) cnt[i] = (uint8_t)(k > 17 ? 17 : k);
 }
-// Later dense neighbours of every dense particle k (j > k, j in S_r(k)),
-// counted then listed; skipcnt[j] counts the dense k that can skip j.
-// With llist, k's entries go to llist[loff[k] - lbase ...] (lbase: the
-// offset of the first particle of the chunk being listed).
-// The counting pass takes whole nodes together (the lanes meeting a node
-// share it): each lane counts its later dense points from the prefix count
-// dpfx (dense particles before an index), and the lanes stride over the
-// node's points, each dense point j getting one atomic that adds the number
-// of queries below j (the queries ascend with the lane, so those lanes are a
-// prefix of the warp).
-template <bool FILL>
-__global__ void __launch_bounds__(128) k_llist_w(const KNode<3> *nodes, const Rec *recs,
-                                                 const int *dense, int nd, float r,
-                                                 const uint8_t *cnt, const int *dpfx,
-                                                 const int64_t *loff, int64_t lbase, int *lcnt,
-                                                 int *llist, int *skipcnt, int *err) {
-    if (warp_idle(nd)) return;
-    int k;
-    bool act = warp_query(dense, nd, &k);
-    float c[3] = {0, 0, 0};
-    if (act) { c[0] = recs[k].pos[0]; c[1] = recs[k].pos[1]; c[2] = recs[k].pos[2]; }
-    int m = 0;
-    int64_t base = (loff && act) ? loff[k] - lbase : 0;
-    auto add = [&](int j) {
-        if (j > k && cnt[j] > 16) {
-            if (llist) llist[base + m] = j;
-            else atomicAdd(&skipcnt[j], 1);
-            m++;
-        }
-    };
-    // leaf points: the warp's lanes that count the same point j add their
-    // counts to skipcnt[j] with one atomic
-    const unsigned lane = threadIdx.x & 31;
-    auto leaf = [&](int j, bool hit) {
-        bool inc = hit && j > k && cnt[j] > 16;
-        if (llist) {
-            if (inc) llist[base + m] = j;
-        } else {
-            unsigned b = __ballot_sync(0xffffffffu, inc);
-            if (b && lane == (unsigned)(__ffs(b) - 1)) atomicAdd(&skipcnt[j], __popc(b));
-        }
-        m += inc;
-    };
-    auto range = [&](int s, int q) {
-        for (int j = s; j < s + q; j++) add(j);
-        return true;
-    };
-    auto point = [&](int j) {
-        add(j);
-        return true;
-    };
-    const int kq = act ? k : INT_MAX;
-    auto coop = [&](unsigned m2, int s, int q) {
-        if ((m2 >> lane) & 1u) {
-            const int a = max(s, k + 1);
-            if (a < s + q) m += dpfx[s + q] - dpfx[a];
-        }
-        const int k31 = __shfl_sync(0xffffffffu, kq, 31);
-        for (int b = 0; b < q; b += 32) {
-            const int j = s + b + lane;
-            int p = 0;  // lanes whose query is below j
+// ---- later dense neighbours, by group -------------------------------------
+// Dense particles are named here by their place in the tree-ordered list of
+// the dense ones.  The list is cut into groups of 32; bit l of a mask stands
+// for place 32 g + l.  Group g's list says which dense places j > k lie in
+// S_r(k) of its places k: (j, mask) for one j and the places k whose sphere
+// holds it, or (first, count) for a range of j beyond the group that every
+// place of the run (below) holds.  skip[j] counts the k.
+// The group's particles are neighbours in the tree, so in a halo a node or
+// point mostly lies inside or outside the spheres of all of them: 32 nodes,
+// then 32 points, are tested against the particles' box by one lane each,
+// nodes inside become ranges, and only the points between the two bounds are
+// tested by every lane.  Consecutive dense particles can lie far apart (a
+// jump between clusters, or across a high split of the tree), so a group is
+// worked in runs: the particles within RSG_REACH linking lengths of the first
+// one left, along every axis.  (At a quarter of the 512^3 volume the walks
+// take 59, 39, 30 and 28 ms for 0.25, 0.5, 1 and 2.)
+// A list of single pairs, one thread per particle in a shared walk, took two
+// walks (counts, then entries) and 4 B a pair: 121 ms for the 7.9e9 pairs of
+// that volume.
+// The bounds are exact in the reference's own float arithmetic: a box's or a
+// point's nearest and farthest offsets bound every lane's offsets, and
+// rounding is monotone, so the sums of their squares in the same order bound
+// the lane's sums.  A point is in S_r(k) when its distance is below r^2, or
+// equal to it when the walk takes one of the point's nodes whole
+// (glist_whole); the bounds used are strict, so equality is always tested.
+#define RSG_REACH 2.0f
+#define RSG_GE 128           // entries per chunk of a group's list
+#define RSG_GSTK 512
+#define RSG_RANGE 0x80000000u
+struct __align__(16) GChunk {
+    uint2 e[RSG_GE];         // (j, mask) or (RSG_RANGE | first, count)
+    int n;                   // entries
+    unsigned mask;           // the places of the run it belongs to
+    int group, ord;          // the chunk is its group's ord-th
+};
+struct GLists {
+    GChunk *pool;
+    int cap;                 // chunks of the pool
+    int *cursor;             // chunks asked for (more than cap: lists are cut)
+    int *nch;                // chunks per group
+};
+// Whether the reference's walk takes a node holding leaf x whole for the
+// query c: the topmost node that is out or inside decides.
+__device__ __noinline__ bool glist_whole(const KNode<3> *nodes, int x, const float *c, float r,
+                                         float r2) {
+    bool res = false;
+    for (; x >= 0; x = nodes[x].parent) {
+        if (box_out3(nodes[x], c, r2)) res = false;
+        else if (box_inside3(nodes[x], c, r, r2)) res = true;
+    }
+    return res;
+}
+// Least and greatest squared distance between the group's box [lo, hi] and
+// the box [mn, mx].
+__device__ __forceinline__ void group_bounds(const float *lo, const float *hi, const float *mn,
+                                             const float *mx, float &near, float &far) {
+    near = far = 0.f;
 #pragma unroll
-            for (int step = 16; step >= 1; step >>= 1)
-                if (__shfl_sync(0xffffffffu, kq, p + step - 1) < j) p += step;
-            if (p == 31 && k31 < j) p = 32;
-            const int c2 = __popc(m2 & (p >= 32 ? 0xffffffffu : ((1u << p) - 1u)));
-            if (j < s + q && c2 && cnt[j] > 16) atomicAdd(&skipcnt[j], c2);
+    for (int d = 0; d < 3; d++) {
+        const float a = fsub(mx[d], lo[d]), b = fsub(hi[d], mn[d]);
+        const float e = fmaxf(fmaxf(-a, -b), 0.f), f = fmaxf(fabsf(a), fabsf(b));
+        near = fadd(near, fmul(e, e));
+        far = fadd(far, fmul(f, f));
+    }
+}
+// Lists of the groups [g0, g1); dpfx holds the dense particles before every
+// index.  COUNT adds the points to skip[], the ranges to its differences
+// diff[], and all pairs to *pairs.
+template <bool COUNT>
+__global__ void __launch_bounds__(128) k_glist(const KNode<3> *nodes, const Rec *recs,
+                                               const int *dense, int nd, int g0, int g1, float r,
+                                               const uint8_t *cnt, const int *dpfx, GLists G,
+                                               int *skip, int *diff, unsigned long long *pairs,
+                                               int *err) {
+    __shared__ int stk[4][RSG_GSTK];
+    __shared__ uint2 stage[4][64];
+    const unsigned FULL = 0xffffffffu;
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int g = g0 + ((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    if (g >= g1) return;
+    const unsigned below = (1u << lane) - 1u;
+    const float r2 = fmul(r, r), reach = RSG_REACH * r;
+    int *S = stk[w];
+    uint2 *buf = stage[w];
+    const bool act = 32 * g + lane < nd;
+    const int k = act ? dense[32 * g + lane] : INT_MAX;
+    const int k31 = __shfl_sync(FULL, k, 31);
+    float c[3];
+#pragma unroll
+    for (int d = 0; d < 3; d++) c[d] = act ? recs[k].pos[d] : 0.f;
+    const unsigned long long cxy = f2_pack(c[0], c[1]);
+    int nch = 0;  // chunks asked for
+    unsigned long long np = 0;
+    bool lost = false;
+    for (unsigned pending = __ballot_sync(FULL, act); pending;) {
+        const int lead = __ffs(pending) - 1;
+        bool mine = (pending >> lane) & 1u;
+        float lo[3], hi[3];
+#pragma unroll
+        for (int d = 0; d < 3; d++)
+            mine &= fabsf(fsub(c[d], __shfl_sync(FULL, c[d], lead))) <= reach;
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+            lo[d] = ord2f(__reduce_min_sync(FULL, mine ? f2ord(c[d]) : 0xffffffffu));
+            hi[d] = ord2f(__reduce_max_sync(FULL, mine ? f2ord(c[d]) : 0u));
         }
-    };
-    sphere3_warp<decltype(range), decltype(point), true, decltype(leaf), !FILL,
-                 decltype(coop)>(nodes, recs, c, act, r, act ? k : INT_MAX - 1, err, range,
-                                 point, leaf, coop);
-    if (act && !llist) lcnt[k] = m;
+        const unsigned run = __ballot_sync(FULL, mine);
+        pending &= ~run;
+        const int kmin = __shfl_sync(FULL, k, lead);
+        const int kmax = __shfl_sync(FULL, k, 31 - __clz(run));
+        int ne = 0, ns = 0, chunk = -1;  // entries in the chunk, staged; the chunk
+        auto flush = [&](int m) {        // the first m <= 32 staged entries
+            if (ne == RSG_GE || ne == 0) {
+                int nc = 0;
+                if (lane == 0) nc = atomicAdd(G.cursor, 1);
+                nc = __shfl_sync(FULL, nc, 0);
+                lost |= nc >= G.cap;
+                if (lane == 0 && !lost) {
+                    if (ne == RSG_GE) G.pool[chunk].n = RSG_GE;
+                    G.pool[nc].mask = run;
+                    G.pool[nc].group = g;
+                    G.pool[nc].ord = nch;
+                }
+                nch++;
+                chunk = nc;
+                ne = 0;
+            }
+            if (!lost && lane < m) G.pool[chunk].e[ne + lane] = buf[lane];
+            ne += m;
+        };
+        auto append = [&](bool v, uint2 e) {  // one entry per lane with v
+            const unsigned em = __ballot_sync(FULL, v);
+            if (v) buf[ns + __popc(em & below)] = e;
+            ns += __popc(em);
+            __syncwarp();
+            if (ns >= 32) {
+                flush(32);
+                ns -= 32;
+                const uint2 rest = buf[32 + lane];
+                __syncwarp();
+                buf[lane] = rest;
+                __syncwarp();
+            }
+        };
+        // down the tree while only one child can hold points of the lists
+        int x = 0;
+        for (int depth = 0; depth < RSG_STACK; depth++) {
+            const int left = nodes[x].left;
+            if (nodes[x].div < 0) break;
+            const KNode<3> ch = nodes[left + (lane & 1)];
+            float near, far;
+            group_bounds(lo, hi, ch.mn, ch.mx, near, far);
+            const unsigned in =
+                __ballot_sync(FULL, ch.start + ch.n > kmin + 1 && near < r2) & 3u;
+            if (in == 3u) break;
+            if (in == 0u) {
+                x = -1;
+                break;
+            }
+            x = left + (in >> 1);
+        }
+        if (lane == 0) S[0] = x;
+        int sp = x >= 0;
+        __syncwarp();
+        while (sp > 0) {
+            const int take = (sp + 64 <= RSG_GSTK - RSG_STACK) ? min(sp, 32) : 1;
+            const int xi = lane < take ? S[sp - 1 - lane] : -1;
+            sp -= take;
+            __syncwarp();
+            int kind = 0, s0 = 0, m0 = 0, left = 0;  // 1 whole node, 2 leaf points, 3 descend
+            if (xi >= 0) {
+                const KNode<3> nd3 = nodes[xi];
+                float near, far;
+                group_bounds(lo, hi, nd3.mn, nd3.mx, near, far);
+                if (nd3.start + nd3.n > kmin + 1 && near < r2) {
+                    kind = far < r2 ? 1 : (nd3.div < 0 ? 2 : 3);
+                    s0 = nd3.start;
+                    m0 = nd3.n;
+                    left = nd3.left;
+                }
+            }
+            const unsigned dm = __ballot_sync(FULL, kind == 3);
+            if (__popc(dm) > ((RSG_GSTK - sp) >> 1)) {  // reported by the call: no list
+                if (lane == 0) {
+                    atomicExch(err, 1);
+                    G.nch[g] = nch;
+                    if (ne > 0 && !lost) G.pool[chunk].n = ne;
+                }
+                return;
+            }
+            if (kind == 3) {
+                const int at = sp + 2 * __popc(dm & below);
+                S[at] = left + 1;
+                S[at + 1] = left;
+            }
+            sp += 2 * __popc(dm);
+            // whole nodes beyond the run's own places: ranges
+            bool rg = kind == 1 && s0 > kmax;
+            if (__any_sync(FULL, rg)) {
+                int first = 0, many = 0;
+                if (rg) {
+                    first = dpfx[s0];
+                    many = dpfx[s0 + m0] - first;
+                    kind = 0;
+                    if (COUNT && many) {
+                        atomicAdd(&diff[first], __popc(run));
+                        atomicSub(&diff[first + many], __popc(run));
+                        np += (unsigned long long)many * __popc(run);
+                    }
+                }
+                append(many > 0, make_uint2(RSG_RANGE | (unsigned)first, (unsigned)many));
+            }
+            // the points after kmin of the round's other whole nodes and leaves
+            const int a0 = max(s0, kmin + 1);
+            const int pn = kind == 1 || kind == 2 ? max(0, s0 + m0 - a0) : 0;
+            int incl = pn;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(FULL, incl, o);
+                if (lane >= o) incl += v;
+            }
+            const int total = __shfl_sync(FULL, incl, 31);
+            for (int base = 0; base < total; base += 32) {
+                const int flat = base + lane;
+                int o = 0;
+#pragma unroll
+                for (int step = 16; step >= 1; step >>= 1) {
+                    const int v = __shfl_sync(FULL, incl, o + step - 1);
+                    if (v <= flat) o += step;
+                }
+                const int oi = __shfl_sync(FULL, incl, o), on = __shfl_sync(FULL, pn, o);
+                const int oa = __shfl_sync(FULL, a0, o), ok = __shfl_sync(FULL, kind, o);
+                const int ox = __shfl_sync(FULL, xi, o);
+                int j = -1;
+                bool all = false, some = false;
+                if (flat < total) {
+                    j = oa + (flat - (oi - on));
+                    if (cnt[j] > 16) {
+                        all = ok == 1;
+                        if (!all) {
+                            const float4 q = *reinterpret_cast<const float4 *>(recs + j);
+                            const float p[3] = {q.x, q.y, q.z};
+                            float near, far;
+                            group_bounds(lo, hi, p, p, near, far);
+                            all = far < r2;
+                            some = !all && near <= r2;
+                        }
+                    }
+                }
+                unsigned mask = all ? run : 0u;
+                if (__any_sync(FULL, all && j <= kmax)) {  // among the run's own places
+                    int p = 0;                             // particles of the group below j
+#pragma unroll
+                    for (int step = 16; step >= 1; step >>= 1)
+                        if (__shfl_sync(FULL, k, p + step - 1) < j) p += step;
+                    if (p == 31 && k31 < j) p = 32;
+                    if (all && p < 32) mask &= (1u << p) - 1u;
+                }
+                for (unsigned todo = __ballot_sync(FULL, some); todo; todo &= todo - 1) {
+                    const int b = __ffs(todo) - 1;
+                    const int jb = __shfl_sync(FULL, j, b), xb = __shfl_sync(FULL, ox, b);
+                    bool hit = false;
+                    if (mine && k < jb) {
+                        const float d = dist3_p(cxy, c[2], recs[jb]);
+                        hit = d < r2 || (d == r2 && glist_whole(nodes, xb, c, r, r2));
+                    }
+                    const unsigned hm = __ballot_sync(FULL, hit);
+                    if (lane == b) mask = hm;
+                }
+                const int dj = mask ? dpfx[j] : 0;
+                if (COUNT && mask) {
+                    atomicAdd(&skip[dj], __popc(mask));
+                    np += __popc(mask);
+                }
+                append(mask != 0u, make_uint2((unsigned)dj, mask));
+            }
+            __syncwarp();
+        }
+        if (ns > 0) flush(ns);
+        if (lane == 0 && ne > 0 && !lost) G.pool[chunk].n = ne;
+        __syncwarp();
+    }
+    if (lane == 0) G.nch[g] = nch;
+    if (COUNT) {
+        for (int o = 16; o; o >>= 1) np += __shfl_xor_sync(FULL, np, o);
+        if (lane == 0 && np) atomicAdd(pairs, np);
+    }
+}
+__global__ void k_gchunks(const int *gch, int ng, int64_t *nch) {
+    int g = blockIdx.x * blockDim.x + threadIdx.x;
+    if (g <= ng) nch[g] = g < ng ? gch[g] : 0;
+}
+// The chunks of every group side by side: (chunk, run's places) of group g at
+// table[off[g] - off0 ...].
+__global__ void k_gtable(const GChunk *pool, int n, const int64_t *off, int64_t off0,
+                         uint2 *table) {
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c < n)
+        table[off[pool[c].group] - off0 + pool[c].ord] = make_uint2((unsigned)c, pool[c].mask);
 }
 // The seeds' searches run one warp per seed (warp_sphere3): a seed's
 // spheres hold hundreds to thousands of points, and its neighbours in tree
@@ -685,109 +889,376 @@ __global__ void k_cand3(const KNode<3> *nodes, const Rec *recs, int n, float r,
 }
 
 // The ordered independent set of the dense particles (the seeds), decided
-// frontier by frontier.  Every dense particle enters the queue once, when it
-// is decided (or, for a particle decided beyond the chunk being walked, when
-// its own chunk starts); a frontier is queue[head, tail).  One warp walks the
-// later list of each frontier particle k: a seed marks its later neighbours
-// as skipped, and every decided particle releases one pending earlier
-// neighbour of each.  A particle with none pending that was not skipped is a
-// seed (all its earlier potential skippers are decided and none of them is
-// a seed).  When the lists are built one chunk of particles [c0, cend) at a
-// time (lbase = loff[c0]), a particle decided beyond cend has no list yet:
-// it keeps its state and enters the first frontier of its own chunk.
+// frontier by frontier.  skip[j] holds the earlier potential skippers of dense
+// place j still undecided, and in its high bits j's own fate; und is a bitmap
+// of the undecided places.  A place decided in one step is worked off in the
+// next: its bit is set in its group's mask of that step's parity (fresh), and
+// the groups with a bit are the frontier.  A group's list is walked once for
+// all the places decided (D), one warp per chunk: an undecided j held by a
+// seed among them is skipped, any other is released from as many skippers as
+// hold it, and a j with none left that was not skipped is a seed (all its
+// earlier potential skippers are decided and none of them is a seed).  Most
+// j are decided already -- a seed skips its whole sphere at once -- and cost
+// a bit, a range's a word for 32.  A step lasts as long as its longest chain
+// of dependent accesses, so the frontier is queued by chunks (a group in a
+// halo's core has hundreds; a warp per group took 0.3 ms a step), four places
+// a lane go through one atomic at a time, nothing waits for the queue
+// (k_kahn_next collects it from fresh), and the undecided stretches of long
+// ranges are left to the warps of k_kahn_wide.  A warp per particle over its
+// list of pairs, an atomic each, took 107 ms for 7.9e9 pairs.  When the
+// lists are built one chunk of groups [gbeg, gend) at a time, a place decided
+// beyond has no list yet: it keeps its fate and its group is queued when its
+// own chunk starts.
+#define RSG_SEED 0x40000000
+#define RSG_SKIPPED 0x20000000
+#define RSG_FATE (RSG_SEED | RSG_SKIPPED)
 struct KahnCtl {
-    int head, tail, next, iters, hit, overflow, cend, pad;
-    int64_t lbase;
+    int now, next;  // list chunks queued for this step; collected for the next
+    int par;        // parity of the step
+    int iters, hit, decided, gbeg, gend;
+    int done, nitems;
+    int going, had;  // places decided for the next step; this step had some
+    int more, pad;   // the loop goes on
+};
+struct KahnItem {  // a stretch of places for k_kahn_wide
+    int first, count;
+    int skip;      // 1: held by a seed
+    int many;      // places it is released by
 };
 struct KahnList {
-    const int64_t *loff;
-    const int *llist;
-    int *queue, qcap;
+    GLists G;
+    int nd, ng;
+    uint2 *table, *queue;  // (chunk, run's places) by group; (chunk, group) of the step
+    const int64_t *off;    // the groups' first entries of the table
+    unsigned *fresh[2];
     KahnCtl *ctl;
-    int *state, *skipcnt;
+    int *skip;
+    unsigned *und;
+    KahnItem *items;
+    int icap;
 };
-__device__ __forceinline__ void kahn_push(int *queue, int qcap, KahnCtl *ctl, int j) {
-    cg::coalesced_group g = cg::coalesced_threads();
-    int base = 0;
-    if (g.thread_rank() == 0) base = atomicAdd(&ctl->next, (int)g.size());
-    const int at = g.shfl(base, 0) + (int)g.thread_rank();
-    if (at < qcap) queue[at] = j;
-    else ctl->overflow = 1;
+// An undecided place j met in this step: `skip` as read by kahn_meet.
+__device__ __forceinline__ int kahn_meet(const KahnList &L, int j, bool seed, int many) {
+    return seed ? atomicOr(&L.skip[j], RSG_SKIPPED) : atomicSub(&L.skip[j], many);
 }
-__global__ void k_kahn(KahnList L) {
+__device__ __forceinline__ void kahn_decide(const KahnList &L, unsigned *fresh, int gend, int j,
+                                            bool seed, int many, int old) {
+    if (seed ? (old & RSG_FATE) != 0 : old != many) return;
+    if (!seed) atomicOr(&L.skip[j], RSG_SEED);
+    const int g = j >> 5;
+    const unsigned bit = 1u << (j & 31);
+    atomicAnd(&L.und[g], ~bit);
+    if (g < gend) atomicOr(&fresh[g], bit);
+}
+// The bits of word w that belong to places [a, a + c).
+__device__ __forceinline__ unsigned range_bits(int w, int a, int c) {
+    const int lo = max(a - 32 * w, 0), hi = min(a + c - 32 * w, 32);
+    return (hi >= 32 ? 0xffffffffu : (1u << hi) - 1u) & ~((1u << lo) - 1u);
+}
+__global__ void __launch_bounds__(256) k_kahn(KahnList L) {
+    const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const int w0 = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nw = (gridDim.x * blockDim.x) >> 5;
     const KahnCtl &C = *L.ctl;
-    const int head = C.head, tail = C.tail, cend = C.cend;
-    const int64_t lbase = C.lbase;
-    for (int f = head + w0; f < tail; f += nw) {
-        const int k = L.queue[f];
-        const int sk = L.state[k];
-        const int64_t e1 = L.loff[k + 1] - lbase;
-        for (int64_t e = L.loff[k] - lbase + lane; e < e1; e += 32) {
-            const int j = L.llist[e];
-            if (sk == 1 && atomicCAS(&L.state[j], 0, 2) == 0 && j < cend)
-                kahn_push(L.queue, L.qcap, L.ctl, j);
-            if (atomicSub(&L.skipcnt[j], 1) == 1 && atomicCAS(&L.state[j], 0, 1) == 0 && j < cend)
-                kahn_push(L.queue, L.qcap, L.ctl, j);
+    const int now = C.now, par = C.par, gend = C.gend;
+    const unsigned *cf = par ? L.fresh[1] : L.fresh[0];
+    unsigned *nf = par ? L.fresh[0] : L.fresh[1];
+    for (int f = w0; f < now; f += nw) {
+        const uint2 item = L.queue[f];
+        const GChunk &K = L.G.pool[item.x];
+        const int g = (int)item.y;
+        const unsigned D = cf[g];
+        const int me = 32 * g + lane;
+        const unsigned mask = K.mask;
+        const int m = K.n;
+        const unsigned Dr = mask & D;
+        const unsigned Sr = __ballot_sync(FULL, me < L.nd && (L.skip[me] & RSG_SEED)) & Dr;
+        uint2 ev[RSG_GE / 32];
+#pragma unroll
+        for (int u = 0; u < RSG_GE / 32; u++) {
+            ev[u] = make_uint2(0u, 0u);
+            if (32 * u + lane < m) ev[u] = __ldcs(&K.e[32 * u + lane]);
+        }
+#pragma unroll
+        for (int u = 0; u < RSG_GE / 32; u++) {
+            if (32 * u >= m) break;
+            const bool rg = ev[u].x & RSG_RANGE;
+            const int a = (int)(ev[u].x & ~RSG_RANGE);
+            const int c = rg ? (int)ev[u].y : 1;
+            const unsigned by = rg ? Dr : ev[u].y & Dr;
+            const int wa = a >> 5, wb = (a + c - 1) >> 5;
+            const bool wide = rg && wb - wa > 3;
+            bool hit = false;
+            if (by && !wide)
+                for (int w = wa; w <= wb; w++)
+                    hit |= (L.und[w] & range_bits(w, a, c)) != 0u;
+            // the places of the entries with an undecided one, flattened
+            if (__any_sync(FULL, hit)) {
+                const int pn = hit ? c : 0;
+                int incl = pn;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int v = __shfl_up_sync(FULL, incl, o);
+                    if (lane >= o) incl += v;
+                }
+                const int total = __shfl_sync(FULL, incl, 31);
+                for (int base = 0; base < total; base += 128) {
+                    int j[4], old[4], many[4];
+                    bool on[4], sd[4];
+#pragma unroll
+                    for (int q = 0; q < 4; q++) {
+                        on[q] = false;
+                        if (base + 32 * q >= total) continue;  // uniform
+                        const int flat = base + 32 * q + lane;
+                        int o = 0;
+#pragma unroll
+                        for (int step = 16; step >= 1; step >>= 1) {
+                            const int v = __shfl_sync(FULL, incl, o + step - 1);
+                            if (v <= flat) o += step;
+                        }
+                        const int oi = __shfl_sync(FULL, incl, o);
+                        const int on0 = __shfl_sync(FULL, pn, o);
+                        const int oa = __shfl_sync(FULL, a, o);
+                        const unsigned ob = __shfl_sync(FULL, by, o);
+                        j[q] = oa + (flat - (oi - on0));
+                        sd[q] = (ob & Sr) != 0u;
+                        many[q] = __popc(ob);
+                        on[q] = flat < total && ((L.und[j[q] >> 5] >> (j[q] & 31)) & 1u);
+                    }
+#pragma unroll
+                    for (int q = 0; q < 4; q++)
+                        if (on[q]) old[q] = kahn_meet(L, j[q], sd[q], many[q]);
+#pragma unroll
+                    for (int q = 0; q < 4; q++)
+                        if (on[q]) kahn_decide(L, nf, gend, j[q], sd[q], many[q], old[q]);
+                }
+            }
+            for (unsigned todo = __ballot_sync(FULL, wide); todo; todo &= todo - 1) {
+                const int b = __ffs(todo) - 1;
+                const int ba = __shfl_sync(FULL, a, b), bc = __shfl_sync(FULL, c, b);
+                const int be = (ba + bc - 1) >> 5;
+                for (int v0 = ba >> 5; v0 <= be; v0 += 32) {
+                    const int w = v0 + lane;
+                    const unsigned word = w <= be ? L.und[w] & range_bits(w, ba, bc) : 0u;
+                    const unsigned nz = __ballot_sync(FULL, word != 0u);
+                    if (!nz) continue;
+                    // eight words with an undecided place: an item
+                    const bool lead = (lane & 7) == 0 && ((nz >> lane) & 0xffu);
+                    const unsigned lm = __ballot_sync(FULL, lead);
+                    int at = 0;
+                    if (lane == 0) at = atomicAdd(&L.ctl->nitems, __popc(lm));
+                    at = __shfl_sync(FULL, at, 0) + __popc(lm & ((1u << lane) - 1u));
+                    const bool fits = at < L.icap;
+                    if (lead && fits) {
+                        const int f0 = max(32 * w, ba);
+                        L.items[at] = KahnItem{f0, min(32 * w + 256, ba + bc) - f0,
+                                               Sr != 0u, __popc(Dr)};
+                    }
+                    // no room: here and now
+                    for (unsigned rest = __ballot_sync(FULL, lead && !fits); rest;
+                         rest &= rest - 1) {
+                        const int l0 = __ffs(rest) - 1;
+                        for (int q = l0; q < l0 + 8; q++) {
+                            const unsigned bits = __shfl_sync(FULL, word, q);
+                            if (!((bits >> lane) & 1u)) continue;
+                            const int j = 32 * (v0 + q) + lane;
+                            kahn_decide(L, nf, gend, j, Sr != 0u, __popc(Dr),
+                                        kahn_meet(L, j, Sr != 0u, __popc(Dr)));
+                        }
+                    }
+                }
+            }
         }
     }
 }
-// Next frontier: the particles queued by the step just run.  False when
-// there are none or a limit was reached.
-__device__ __forceinline__ bool kahn_advance(KahnCtl *ctl, int qcap, int limit) {
-    const int old = ctl->tail;
-    const int nt = min(ctl->next, qcap);
-    ctl->head = old;
-    ctl->tail = nt;
-    const int it = ++ctl->iters;
-    bool more = nt > old && !ctl->overflow;
-    if (more && it >= limit) {
+// The stretches k_kahn left, a warp each: at most 256 places of eight words.
+__global__ void __launch_bounds__(256) k_kahn_wide(KahnList L) {
+    const int lane = threadIdx.x & 31;
+    const int w0 = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int nw = (gridDim.x * blockDim.x) >> 5;
+    const KahnCtl &C = *L.ctl;
+    const int n = min(C.nitems, L.icap), gend = C.gend;
+    unsigned *nf = C.par ? L.fresh[0] : L.fresh[1];
+    for (int f = w0; f < n; f += nw) {
+        const KahnItem it = L.items[f];
+        int old[8];
+        bool on[8];
+#pragma unroll
+        for (int q = 0; q < 8; q++) {
+            const int j = it.first + 32 * q + lane;
+            on[q] = j < it.first + it.count && ((L.und[j >> 5] >> (j & 31)) & 1u);
+        }
+#pragma unroll
+        for (int q = 0; q < 8; q++)
+            if (on[q]) old[q] = kahn_meet(L, it.first + 32 * q + lane, it.skip != 0, it.many);
+#pragma unroll
+        for (int q = 0; q < 8; q++)
+            if (on[q])
+                kahn_decide(L, nf, gend, it.first + 32 * q + lane, it.skip != 0, it.many, old[q]);
+    }
+}
+// Queues the chunks of the groups with decided places whose run holds one.
+// All lanes of a warp call it with their group's mask (0: none); a lane goes
+// through its group's chunks itself, or the warp does for it when they are
+// many.
+#define RSG_KLANE 16
+__device__ __forceinline__ void kahn_queue(const KahnList &L, int *count, int g, unsigned D,
+                                           bool step) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const uint2 *tab = L.table - L.off[L.ctl->gbeg];
+    int64_t o = 0;
+    int n = 0;
+    if (D) {
+        o = L.off[g];
+        n = (int)(L.off[g + 1] - o);
+    }
+    const bool own = n <= RSG_KLANE;
+    int c = 0;
+    if (own)
+        for (int t = 0; t < n; t++) c += (tab[o + t].y & D) != 0u;
+    int incl = c;
+#pragma unroll
+    for (int q = 1; q < 32; q <<= 1) {
+        const int v = __shfl_up_sync(FULL, incl, q);
+        if (lane >= q) incl += v;
+    }
+    const int total = __shfl_sync(FULL, incl, 31);
+    if (total) {
+        int at = 0;
+        if (lane == 0) at = atomicAdd(count, total);
+        at = __shfl_sync(FULL, at, 0) + incl - c;
+        if (own)
+            for (int t = 0; t < n; t++) {
+                const uint2 e = tab[o + t];
+                if (e.y & D) L.queue[at++] = make_uint2(e.x, (unsigned)g);
+            }
+    }
+    for (unsigned todo = __ballot_sync(FULL, !own); todo; todo &= todo - 1) {
+        const int b = __ffs(todo) - 1;
+        const int bg = __shfl_sync(FULL, g, b), bn = __shfl_sync(FULL, n, b);
+        const unsigned bd = __shfl_sync(FULL, D, b);
+        const int64_t bo = __shfl_sync(FULL, o, b);
+        for (int t0 = 0; t0 < bn; t0 += 32) {
+            uint2 e = make_uint2(0u, 0u);
+            if (t0 + lane < bn) e = tab[bo + t0 + lane];
+            const bool on = (e.y & bd) != 0u;
+            const unsigned m = __ballot_sync(FULL, on);
+            if (!m) continue;
+            int at = 0;
+            if (lane == 0) at = atomicAdd(count, __popc(m));
+            at = __shfl_sync(FULL, at, 0) + __popc(m & ((1u << lane) - 1u));
+            if (on) L.queue[at] = make_uint2(e.x, (unsigned)bg);
+        }
+    }
+    const int dec = __reduce_add_sync(FULL, __popc(D));
+    if (lane == 0 && dec) {
+        atomicAdd(&L.ctl->decided, dec);
+        if (step) L.ctl->going = 1;
+    }
+}
+// Collects the next frontier from the groups' masks and clears those of the
+// step just run; the last block to finish advances the step.  False when no
+// place was decided or a limit was reached.  A step without decided places
+// (the host loop may run some past the last) does not count.
+__device__ __forceinline__ bool kahn_collect(const KahnList &L, int limit, bool counts,
+                                             bool *last) {
+    KahnCtl *ctl = L.ctl;
+    unsigned *cf = ctl->par ? L.fresh[1] : L.fresh[0];
+    const unsigned *nf = ctl->par ? L.fresh[0] : L.fresh[1];
+    const int gb = ctl->gbeg, ge = ctl->gend;
+    bool any = false;
+    const int nt = gridDim.x * blockDim.x, t = blockIdx.x * blockDim.x + threadIdx.x;
+    for (int g = gb + t; g < ge; g += nt)
+        if (cf[g]) {
+            cf[g] = 0u;
+            any = true;
+        }
+    // neighbouring groups (a halo's are decided together) to different warps,
+    // by the 32 bytes a read takes
+    const int64_t nw = nt >> 5;
+    for (int64_t s0 = t >> 5; gb + 8 * s0 < ge; s0 += 4 * nw) {
+        const int64_t gl = gb + 8 * (s0 + ((t & 31) >> 3) * nw) + (t & 7);
+        const int g = gl < ge ? (int)gl : ge;
+        const unsigned D = g < ge ? nf[g] : 0u;
+        if (__any_sync(0xffffffffu, D != 0u)) kahn_queue(L, &ctl->next, g, D, true);
+    }
+    any = __syncthreads_or(any);
+    __threadfence();
+    *last = false;
+    if (threadIdx.x == 0) {
+        if (any) atomicOr(&ctl->had, 1);
+        __threadfence();
+        *last = atomicAdd(&ctl->done, 1) == (int)gridDim.x - 1;
+    }
+    if (!*last) return false;
+    if (counts | atomicExch(&ctl->had, 0)) ctl->iters++;
+    bool more = atomicExch(&ctl->going, 0) != 0;
+    ctl->now = atomicExch(&ctl->next, 0);
+    ctl->done = 0;
+    ctl->nitems = 0;
+    ctl->par ^= 1;
+    if (more && ctl->iters >= limit) {
         ctl->hit = 1;
         more = false;
     }
+    ctl->more = more;
     return more;
 }
-__global__ void k_kahn_next(KahnCtl *ctl, int qcap, int limit) { kahn_advance(ctl, qcap, limit); }
-__global__ void k_kahn_next_g(KahnCtl *ctl, int qcap, int limit, cudaGraphConditionalHandle h) {
-    cudaGraphSetConditional(h, kahn_advance(ctl, qcap, limit) ? 1u : 0u);
+__global__ void k_kahn_next(KahnList L, int limit, int counts) {
+    bool last;
+    kahn_collect(L, limit, counts != 0, &last);
 }
-// Dense particles with no earlier potential skipper are seeds; those before
-// the first chunk's end start the first frontier.
-__global__ void k_kahn_init(const int *dense, int nd, const int *skipcnt, int cend, int *state,
-                            int *queue, int qcap, KahnCtl *ctl) {
-    int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= nd) return;
-    const int i = dense[t];
-    if (skipcnt[i] == 0) {
-        state[i] = 1;
-        if (i < cend) kahn_push(queue, qcap, ctl, i);
+__global__ void k_kahn_next_g(KahnList L, int limit, cudaGraphConditionalHandle h) {
+    bool last;
+    const bool more = kahn_collect(L, limit, true, &last);
+    if (last) cudaGraphSetConditional(h, more ? 1u : 0u);
+}
+// skip[] from the points' counts and the ranges' (pre: their differences
+// summed); places with no earlier potential skipper are seeds, the others
+// undecided.
+__global__ void k_kahn_init(int nd, const int *pre, int *skip, unsigned *und) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    bool open = false;
+    if (t < nd) {
+        const int v = skip[t] + pre[t];
+        open = v != 0;
+        skip[t] = open ? v : RSG_SEED;
+    }
+    const unsigned b = __ballot_sync(0xffffffffu, open);
+    if ((t & 31) == 0 && t < nd) und[t >> 5] = b;
+}
+// A chunk's first frontier: its groups' places decided so far.  One thread
+// per group, reading its 32 fates; k_kahn_start names the chunk before.
+__global__ void k_kahn_chunk(KahnList L) {
+    const KahnCtl &C = *L.ctl;
+    const int gend = C.gend;
+    unsigned *cf = C.par ? L.fresh[1] : L.fresh[0];
+    for (int g0 = C.gbeg + blockIdx.x * blockDim.x; g0 < gend; g0 += gridDim.x * blockDim.x) {
+        const int g = g0 + threadIdx.x;
+        unsigned D = 0u;
+        if (g < gend) {
+            for (int l = 0; l < 32 && 32 * g + l < L.nd; l++)
+                if (L.skip[32 * g + l] & RSG_FATE) D |= 1u << l;
+            cf[g] = D;
+        }
+        if (__any_sync(0xffffffffu, D != 0u)) kahn_queue(L, &L.ctl->now, g, D, false);
     }
 }
-// First frontier of a later chunk: its dense particles already decided
-// while earlier chunks were walked.
-__global__ void k_kahn_chunk(const int *dense, int nd, const int *state, int *queue, int qcap,
-                             KahnCtl *ctl) {
-    int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= nd) return;
-    const int i = dense[t];
-    if (state[i] != 0) kahn_push(queue, qcap, ctl, i);
-}
-// A chunk's walk begins: its list range and the frontier queued for it.
-__global__ void k_kahn_start(KahnCtl *ctl, int qcap, int cend, int64_t lbase) {
-    ctl->cend = cend;
-    ctl->lbase = lbase;
-    ctl->head = ctl->tail;
-    ctl->tail = min(ctl->next, qcap);
+__global__ void k_kahn_start(KahnCtl *ctl, int gbeg, int gend) {
+    ctl->gbeg = gbeg;
+    ctl->gend = gend;
+    ctl->now = ctl->next = ctl->nitems = ctl->going = ctl->had = ctl->done = 0;
 }
 struct ChunkTarget {
     int64_t step;
     __host__ __device__ int64_t operator()(int64_t t) const { return (t + 1) * step; }
 };
-__global__ void k_state8(const int *s32, int n, uint8_t *s8) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) s8[i] = (uint8_t)s32[i];
+// State of the dense particles: 1 a seed, 2 skipped by one (others: 0).
+__global__ void k_state8(const int *dense, int nd, const int *skip, uint8_t *s8) {
+    int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < nd) s8[dense[t]] = (skip[t] & RSG_SEED) ? 1 : 2;
 }
 
 // Label of every particle: the smallfof of the set it joined (root null),
@@ -822,10 +1293,6 @@ __global__ void k_runs3(const int *hpos, const int *nh, int n, int64_t minsz, in
     keep[g] = (e - s) >= minsz;
 }
 
-__global__ void k_mark_undecided(const int *dense, int nd, uint8_t *state) {
-    int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < nd) state[dense[t]] = 0;
-}
 __global__ void k_take2(const int32_t *idx, int m, const int32_t *a, const int32_t *b,
                         int32_t *a2, int32_t *b2) {
     int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -856,12 +1323,12 @@ static int sm_count() {
     return v > 0 ? v : 1;
 }
 // The seed frontiers of one chunk as one graph: a while node whose body runs
-// a step (k_kahn) and advances the frontier (k_kahn_next_g sets the loop
-// condition), so no step waits for the host.
+// a step (k_kahn, k_kahn_wide) and advances the frontier (k_kahn_next_g sets
+// the loop condition), so no step waits for the host.
 struct KahnGraph {
     cudaGraph_t g = nullptr;
     cudaGraphExec_t e = nullptr;
-    void build(int GK, int TK, KahnList L, int limit) {
+    void build(int GK, int GN, int TK, KahnList L, int limit) {
         RSG_CUDA(cudaGraphCreate(&g, 0));
         cudaGraphConditionalHandle h;
         RSG_CUDA(cudaGraphConditionalHandleCreate(&h, g, 1, cudaGraphCondAssignDefault));
@@ -870,7 +1337,7 @@ struct KahnGraph {
         cp.conditional.handle = h;
         cp.conditional.type = cudaGraphCondTypeWhile;
         cp.conditional.size = 1;
-        cudaGraphNode_t cn, wn, nn;
+        cudaGraphNode_t cn, wn, xn, nn;
         RSG_CUDA(cudaGraphAddNode(&cn, g, nullptr, nullptr, 0, &cp));
         cudaGraph_t body = cp.conditional.phGraph_out[0];
         void *wargs[] = {(void *)&L};
@@ -880,14 +1347,13 @@ struct KahnGraph {
         kp.blockDim = dim3(TK);
         kp.kernelParams = wargs;
         RSG_CUDA(cudaGraphAddKernelNode(&wn, body, nullptr, 0, &kp));
-        KahnCtl *ctl = L.ctl;
-        int qcap = L.qcap;
-        void *nargs[] = {(void *)&ctl, (void *)&qcap, (void *)&limit, (void *)&h};
+        kp.func = (void *)k_kahn_wide;
+        RSG_CUDA(cudaGraphAddKernelNode(&xn, body, &wn, 1, &kp));
+        void *nargs[] = {(void *)&L, (void *)&limit, (void *)&h};
         kp.func = (void *)k_kahn_next_g;
-        kp.gridDim = dim3(1);
-        kp.blockDim = dim3(1);
+        kp.gridDim = dim3(GN);
         kp.kernelParams = nargs;
-        RSG_CUDA(cudaGraphAddKernelNode(&nn, body, &wn, 1, &kp));
+        RSG_CUDA(cudaGraphAddKernelNode(&nn, body, &xn, 1, &kp));
         RSG_CUDA(cudaGraphInstantiate(&e, g, 0));
     }
     cudaStream_t ran = nullptr;
@@ -988,13 +1454,12 @@ FofOut fof3d_device(Arena &ar, const rsg_particle *d_in, int64_t n64, const rsg_
     // dense particles (more than 16 neighbours), in tree order
     int *dense = ar.get<int>(n);
     int nd = select_where(ar, n, DFlag{cnt}, dense, st);
-    // later-dense-neighbour lists and pending-skipper counts
-    // (64-bit offsets: the lists can hold more than 2^31 entries)
-    int *lcnt = ar.get<int>(n + 1), *skipcnt = ar.get<int>(n);
-    int64_t *loff = ar.get<int64_t>(n + 1);
-    RSG_CUDA(cudaMemsetAsync(lcnt, 0, sizeof(int) * (n + 1), st));
-    RSG_CUDA(cudaMemsetAsync(skipcnt, 0, sizeof(int) * n, st));
-    // dense particles before every index (the counting pass's whole nodes)
+    // groups of 32 dense particles, their lists of later dense neighbours and
+    // every particle's pending skippers
+    const int ng = (nd + 31) / 32;
+    int *skip = ar.get<int>(nd + 1);
+    RSG_CUDA(cudaMemsetAsync(skip, 0, sizeof(int) * (nd + 1), st));
+    // dense particles before every index
     int *dpfx = ar.get<int>(n + 1);
     {
         thrust::transform_iterator<DenseI, const uint8_t *, int> dit((const uint8_t *)cnt, DenseI{});
@@ -1005,44 +1470,96 @@ FofOut fof3d_device(Arena &ar, const rsg_particle *d_in, int64_t n64, const rsg_
         cub::DeviceScan::ExclusiveSum(pt, pb, dit, dpfx, n + 1, st);
         ar.used = m0;
     }
-    launch(k_llist_w<false>, nblk(nd, TW), TW, 0, st, F.nodes, recs, (const int *)dense, nd, r,
-           (const uint8_t *)cnt, (const int *)dpfx, (const int64_t *)nullptr, (int64_t)0, lcnt,
-           (int *)nullptr, skipcnt, err);
-    size_t cb = 0;
-    thrust::transform_iterator<ToI64, const int32_t *, int64_t> lc64((const int32_t *)lcnt, ToI64{});
-    cub::DeviceScan::ExclusiveSum(nullptr, cb, lc64, loff, n + 1, st);
-    void *ct = ar.take(cb + 256);
-    cub::DeviceScan::ExclusiveSum(ct, cb, lc64, loff, n + 1, st);
-    int64_t ne = 0;
-    RSG_CUDA(cudaMemcpyAsync(&ne, loff + n, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
-    RSG_CUDA(cudaStreamSynchronize(st));
-    // The list lives in the arena when it fits beside what the rest of the FOF
-    // takes from it (< 256 B per particle: the label derivation and the
-    // partition sort).  A larger one (hundreds of entries
-    // per particle in very dense snapshots) gets an allocation of its own for
-    // this call, as large as free device memory allows (less 1 GiB, or
-    // RSG_FOF_LIST_ENTRIES entries when that is set); when the whole list
-    // does not fit, it is built and walked one chunk of particles at a time,
-    // chunks in particle order.  A fixed arena holds the list whole or fails.
-    // That allocation stays with the host thread for its later calls, as the
-    // arena does: allocating and freeing a hundred gigabytes costs tens of
-    // milliseconds each, and the free waits for the device.
-    int *llist;
-    int64_t lcap = ne > 0 ? ne : 1;  // entries the list buffer holds
-    size_t lat = (ar.used + 255) & ~(size_t)255;
+    KahnList KL;
+    KL.nd = nd;
+    KL.skip = skip;
+    KL.und = ar.get<unsigned>(ng + 1);
+    int *diff = ar.get<int>(nd + 1);
+    RSG_CUDA(cudaMemsetAsync(diff, 0, sizeof(int) * (nd + 1), st));
+    size_t dsb = 0;
+    cub::DeviceScan::InclusiveSum(nullptr, dsb, diff, diff, nd + 1, st);
+    void *dst_tmp = ar.take(dsb + 256);
+    KL.ng = ng;
+    KL.icap = ng < (1 << 20) ? ng + 256 : 1 << 20;
+    KL.items = ar.get<KahnItem>(KL.icap);
+    for (int b = 0; b < 2; b++) {
+        KL.fresh[b] = ar.get<unsigned>(ng + 1);
+        RSG_CUDA(cudaMemsetAsync(KL.fresh[b], 0, sizeof(unsigned) * (ng + 1), st));
+    }
+    KL.ctl = ar.get<KahnCtl>(1);
+    RSG_CUDA(cudaMemsetAsync(KL.ctl, 0, sizeof(KahnCtl), st));
+    KL.G.nch = ar.get<int>(ng + 1);
+    int64_t *gn = ar.get<int64_t>(ng + 1), *go = ar.get<int64_t>(ng + 1), *gm = ar.get<int64_t>(1);
+    KL.off = go;
+    size_t sb = 0, mb = 0;
+    cub::DeviceScan::ExclusiveSum(nullptr, sb, gn, go, ng + 1, st);
+    cub::DeviceReduce::Max(nullptr, mb, gn, gm, ng + 1, st);
+    const size_t gtb = (sb > mb ? sb : mb) + 256;
+    void *gtmp = ar.take(gtb);
+    // {chunks asked for, pairs}
+    unsigned long long *tot = ar.get<unsigned long long>(2);
+    RSG_CUDA(cudaMemsetAsync(tot, 0, 2 * sizeof(*tot), st));
+    KL.G.cursor = (int *)tot;
+    // The lists go to the arena beside what the rest of the FOF takes from it
+    // (< 256 B per particle: the label derivation and the partition sort).
+    // Lists that do not fit (very dense snapshots) get an allocation of
+    // their own, as large as free device memory allows (less 1 GiB, or room
+    // for RSG_FOF_LIST_ENTRIES entries when that is set); when not all fit,
+    // they are built and walked one chunk of groups at a time, chunks in
+    // order.  A fixed arena holds the lists whole or fails.  That allocation
+    // stays with the host thread for its later calls, as the arena does:
+    // allocating and freeing tens of gigabytes costs tens of milliseconds,
+    // and the free waits for the device.
     const char *lenv = getenv("RSG_FOF_LIST_ENTRIES");
-    int64_t lforce = lenv ? atoll(lenv) : 0;
-    if (ar.fixed || (!lforce && lat + sizeof(int) * (size_t)lcap + (size_t)256 * n + (64u << 20) <= ar.cap)) {
-        llist = ar.get<int>(lcap);
+    const int64_t lforce = lenv ? atoll(lenv) : 0;
+    const size_t lat = (ar.used + 255) & ~(size_t)255;
+    const size_t rest = ar.fixed ? 0 : (size_t)256 * n + (64u << 20);
+    // a chunk, its place in the groups' table and in a step's queue
+    const size_t each = sizeof(GChunk) + 2 * sizeof(uint2);
+    int64_t fit = lat + rest + 1024 < ar.cap ? (int64_t)((ar.cap - lat - rest - 1024) / each) : 0;
+    if (lforce > 0 && !ar.fixed) fit = 0;
+    KL.G.cap = (int)std::min<int64_t>(fit, INT_MAX / 2);
+    KL.G.pool = ar.get<GChunk>(KL.G.cap);
+    const int TG = 128;
+    auto gblk = [&](int groups) { return nblk((int64_t)groups * 32, TG); };
+    launch(k_glist<true>, gblk(ng), TG, 0, st, F.nodes, recs, (const int *)dense, nd, 0, ng, r,
+           (const uint8_t *)cnt, (const int *)dpfx, KL.G, skip, diff, tot + 1, err);
+    if (nd > 0) cub::DeviceScan::InclusiveSum(dst_tmp, dsb, diff, diff, nd + 1, st);
+    launch(k_kahn_init, nblk(nd, T), T, 0, st, nd, (const int *)diff, skip, KL.und);
+    unsigned long long htot[2] = {0, 0};
+    RSG_CUDA(cudaMemcpyAsync(htot, tot, sizeof(htot), cudaMemcpyDeviceToHost, st));
+    RSG_CUDA(cudaStreamSynchronize(st));
+    const int64_t nch = (int64_t)(uint32_t)htot[0];  // chunks the lists take
+    const int64_t ne = (int64_t)htot[1];
+    launch(k_gchunks, nblk(ng + 1, T), T, 0, st, (const int *)KL.G.nch, ng, gn);
+    sb = mb = gtb;
+    cub::DeviceScan::ExclusiveSum(gtmp, sb, gn, go, ng + 1, st);
+    // chunk boundaries: groups c[t] .. c[t+1], the chunks of their lists
+    std::vector<int> cb_h(2, 0);
+    std::vector<int64_t> lb_h(2, 0);
+    cb_h[1] = ng;
+    lb_h[1] = nch;
+    const bool built = nch <= KL.G.cap;
+    ar.used = lat;
+    if (built) {
+        ar.get<GChunk>(nch);
+        KL.table = ar.get<uint2>(nch);
+        KL.queue = ar.get<uint2>(nch);
     } else {
+        if (ar.fixed) {
+            set_error(RSG_ERR_LIMIT, "device arena exhausted (%lld neighbour list chunks, room "
+                      "for %d)", (long long)nch, KL.G.cap);
+            throw Failure();
+        }
         ListCache &lc = g_list_cache;
         size_t fb = 0, tb = 0;
         RSG_CUDA(cudaMemGetInfo(&fb, &tb));
         fb += lc.bytes;  // the kept buffer is this call's to use
-        int64_t avail = fb > ((size_t)1 << 30) ? (int64_t)((fb - ((size_t)1 << 30)) / sizeof(int)) : 0;
-        if (lforce > 0) avail = lforce;
-        if (avail < lcap) lcap = avail;
-        const size_t need = sizeof(int) * (size_t)(lcap > 0 ? lcap : 1);
+        int64_t avail = fb > ((size_t)1 << 30) ? (int64_t)((fb - ((size_t)1 << 30)) / each) : 0;
+        if (lforce > 0) avail = lforce / RSG_GE;
+        avail = std::min<int64_t>(avail, INT_MAX / 2);
+        const int64_t lcap = std::min(avail, nch);
+        const size_t need = each * (size_t)(lcap > 0 ? lcap : 1);
         if (lc.bytes < need) {
             if (lc.p) RSG_CUDA(cudaFree(lc.p));
             lc.p = nullptr;
@@ -1050,112 +1567,104 @@ FofOut fof3d_device(Arena &ar, const rsg_particle *d_in, int64_t n64, const rsg_
             RSG_CUDA(cudaMalloc(&lc.p, need));
             lc.bytes = need;
         }
-        llist = (int *)lc.p;
-    }
-    // chunk boundaries: particles c[t] .. c[t+1], dense entries d[t] .. d[t+1]
-    std::vector<int> cb_h(2, 0), db_h(2, 0);
-    std::vector<int64_t> lb_h(1, 0);
-    cb_h[1] = n;
-    db_h[1] = nd;
-    if (lcap < ne) {
-        int maxl = 0;
-        {
-            int *dmax = ar.get<int>(1);
-            size_t mb = 0;
-            cub::DeviceReduce::Max(nullptr, mb, lcnt, dmax, n, st);
-            size_t m0 = ar.used;
-            void *mt = ar.take(mb + 256);
-            cub::DeviceReduce::Max(mt, mb, lcnt, dmax, n, st);
-            ar.used = m0;
-            RSG_CUDA(cudaMemcpyAsync(&maxl, dmax, sizeof(int), cudaMemcpyDeviceToHost, st));
+        KL.G.pool = (GChunk *)lc.p;
+        KL.G.cap = (int)lcap;
+        KL.table = (uint2 *)(KL.G.pool + lcap);
+        KL.queue = KL.table + lcap;
+        if (lcap < nch) {
+            int64_t maxl = 0;
+            cub::DeviceReduce::Max(gtmp, mb, gn, gm, ng + 1, st);
+            RSG_CUDA(cudaMemcpyAsync(&maxl, gm, sizeof(maxl), cudaMemcpyDeviceToHost, st));
             RSG_CUDA(cudaStreamSynchronize(st));
-        }
-        int64_t step = lcap - maxl;
-        if (step < (int64_t)maxl || step < (1 << 16)) {
-            set_error(RSG_ERR_LIMIT, "later-dense lists need more device memory than is free");
-            throw Failure();
-        }
-        int64_t m = (ne + step - 1) / step;  // chunks
-        int *cbd = ar.get<int>(m + 1), *dbd = ar.get<int>(m + 1);
-        thrust::transform_iterator<ChunkTarget, thrust::counting_iterator<int64_t>, int64_t> tgt(
-            thrust::counting_iterator<int64_t>(0), ChunkTarget{step});
-        thrust::lower_bound(thrust::cuda::par_nosync.on(st), loff, loff + n + 1, tgt, tgt + (m - 1), cbd);
-        thrust::lower_bound(thrust::cuda::par_nosync.on(st), dense, dense + nd, cbd, cbd + (m - 1), dbd);
-        cb_h.assign(m + 1, 0);
-        db_h.assign(m + 1, 0);
-        RSG_CUDA(cudaMemcpyAsync(cb_h.data() + 1, cbd, sizeof(int) * (m - 1), cudaMemcpyDeviceToHost, st));
-        RSG_CUDA(cudaMemcpyAsync(db_h.data() + 1, dbd, sizeof(int) * (m - 1), cudaMemcpyDeviceToHost, st));
-        RSG_CUDA(cudaStreamSynchronize(st));
-        cb_h[m] = n;
-        db_h[m] = nd;
-        lb_h.assign(m + 1, 0);
-        for (int64_t t = 0; t <= m; t++)
-            RSG_CUDA(cudaMemcpyAsync(&lb_h[t], loff + cb_h[t], sizeof(int64_t), cudaMemcpyDeviceToHost, st));
-        RSG_CUDA(cudaStreamSynchronize(st));
-        for (int64_t t = 0; t < m; t++)
-            if (lb_h[t + 1] - lb_h[t] > lcap) {
-                set_error(RSG_ERR_LIMIT, "later-dense list chunk exceeds its buffer");
+            const int64_t step = lcap - maxl;
+            if (step < maxl || step * RSG_GE < (1 << 12)) {
+                set_error(RSG_ERR_LIMIT, "later-dense lists need more device memory than is free");
                 throw Failure();
             }
+            const int64_t m = (nch + step - 1) / step;  // chunks
+            int *cbd = ar.get<int>(m + 1);
+            thrust::transform_iterator<ChunkTarget, thrust::counting_iterator<int64_t>, int64_t> tgt(
+                thrust::counting_iterator<int64_t>(0), ChunkTarget{step});
+            thrust::lower_bound(thrust::cuda::par_nosync.on(st), (const int64_t *)go, (const int64_t *)go + ng + 1, tgt,
+                                tgt + (m - 1), cbd);
+            cb_h.assign(m + 1, 0);
+            lb_h.assign(m + 1, 0);
+            RSG_CUDA(cudaMemcpyAsync(cb_h.data() + 1, cbd, sizeof(int) * (m - 1),
+                                     cudaMemcpyDeviceToHost, st));
+            RSG_CUDA(cudaStreamSynchronize(st));
+            cb_h[m] = ng;
+            for (int64_t t = 0; t <= m; t++)
+                RSG_CUDA(cudaMemcpyAsync(&lb_h[t], go + cb_h[t], sizeof(int64_t),
+                                         cudaMemcpyDeviceToHost, st));
+            RSG_CUDA(cudaStreamSynchronize(st));
+            for (int64_t t = 0; t < m; t++)
+                if (lb_h[t + 1] - lb_h[t] > lcap) {
+                    set_error(RSG_ERR_LIMIT, "later-dense list chunk exceeds its buffer");
+                    throw Failure();
+                }
+        }
     }
     const int nchunks = (int)cb_h.size() - 1;
-    int *state32 = ar.get<int>(n);
-    RSG_CUDA(cudaMemsetAsync(state32, 0, sizeof(int) * n, st));
-    int *queue = ar.get<int>(nd + 1);
-    const int qcap = nd + 1;
-    KahnCtl *ctl = (KahnCtl *)ar.get<int64_t>(8);
-    RSG_CUDA(cudaMemsetAsync(ctl, 0, sizeof(KahnCtl), st));
-    launch(k_kahn_init, nblk(nd, T), T, 0, st, (const int *)dense, nd, (const int *)skipcnt,
-           cb_h[1], state32, queue, qcap, ctl);
-    const KahnList KL{(const int64_t *)loff, (const int *)llist, queue, qcap, ctl, state32, skipcnt};
     // every step but a chunk's last decides a particle
     const int limit = nd + nchunks + 2;
     int kres = 0;
     RSG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&kres, k_kahn, 256, 0));
-    const int TK = 256, GK = (kres > 0 ? kres : 1) * sm_count();
+    const int TK = 256;
+    const int GK = (int)std::min<int64_t>((int64_t)(kres > 0 ? kres : 1) * sm_count(),
+                                          nch * 32 / TK + 1);
+    const int GN = std::min<int>(4 * sm_count(), nblk(ng, TK));
     // the frontier steps run as a device-side graph loop; with per-launch
     // event timing, and in fixed storage (instantiating a graph may take
-    // device memory), the host drives the same steps
+    // device memory), the host drives the same steps, in fixed storage a few
+    // between reads of the state
     const bool host_loop = launch_stats().selecting || ar.fixed;
+    const int burst = launch_stats().selecting ? 1 : 8;
     KahnGraph G;
-    if (!host_loop && nd > 0) G.build(GK, TK, KL, limit);
+    if (!host_loop && nd > 0) G.build(GK, GN, TK, KL, limit);
     for (int t = 0; t < nchunks; t++) {
-        int d0 = db_h[t], d1 = db_h[t + 1];
-        if (d1 <= d0) continue;
-        int64_t lbase = lb_h.size() > 1 ? lb_h[t] : 0;
-        launch(k_llist_w<true>, nblk(d1 - d0, TW), TW, 0, st, F.nodes, recs,
-               (const int *)dense + d0, d1 - d0, r, (const uint8_t *)cnt, (const int *)dpfx,
-               (const int64_t *)loff, lbase, lcnt, llist, skipcnt, err);
-        if (t > 0)
-            launch(k_kahn_chunk, nblk(d1 - d0, T), T, 0, st, (const int *)dense + d0, d1 - d0,
-                   (const int *)state32, queue, qcap, ctl);
-        launch(k_kahn_start, 1, 1, 0, st, ctl, qcap, cb_h[t + 1], lbase);
+        const int c0 = cb_h[t], c1 = cb_h[t + 1];
+        if (c1 <= c0) continue;
+        if (!built) {
+            RSG_CUDA(cudaMemsetAsync(KL.G.cursor, 0, sizeof(int), st));
+            launch(k_glist<false>, gblk(c1 - c0), TG, 0, st, F.nodes, recs, (const int *)dense, nd,
+                   c0, c1, r, (const uint8_t *)cnt, (const int *)dpfx, KL.G, skip, diff, tot + 1,
+                   err);
+        }
+        const int lc = (int)(lb_h[t + 1] - lb_h[t]);
+        launch(k_gtable, nblk(lc, T), T, 0, st, (const GChunk *)KL.G.pool, lc, KL.off, lb_h[t],
+               KL.table);
+        launch(k_kahn_start, 1, 1, 0, st, KL.ctl, c0, c1);
+        launch(k_kahn_chunk, GN, TK, 0, st, KL);
         if (!host_loop) {
             G.run(st);
             continue;
         }
         for (;;) {
-            launch(k_kahn, GK, TK, 0, st, KL);
-            launch(k_kahn_next, 1, 1, 0, st, ctl, qcap, limit);
+            for (int b = 0; b < burst; b++) {
+                launch(k_kahn, GK, TK, 0, st, KL);
+                launch(k_kahn_wide, GK, TK, 0, st, KL);
+                launch(k_kahn_next, GN, TK, 0, st, KL, limit, (int)(burst == 1));
+            }
             KahnCtl hc;
-            RSG_CUDA(cudaMemcpyAsync(&hc, ctl, sizeof(hc), cudaMemcpyDeviceToHost, st));
+            RSG_CUDA(cudaMemcpyAsync(&hc, KL.ctl, sizeof(hc), cudaMemcpyDeviceToHost, st));
             RSG_CUDA(cudaStreamSynchronize(st));
-            if (hc.tail <= hc.head || hc.hit || hc.overflow) break;
+            if (!hc.more || hc.hit) break;
         }
     }
     KahnCtl kc;
-    RSG_CUDA(cudaMemcpyAsync(&kc, ctl, sizeof(kc), cudaMemcpyDeviceToHost, st));
+    RSG_CUDA(cudaMemcpyAsync(&kc, KL.ctl, sizeof(kc), cudaMemcpyDeviceToHost, st));
     RSG_CUDA(cudaStreamSynchronize(st));
-    if (kc.hit || kc.overflow || kc.next != nd) {
-        set_error(RSG_ERR_LIMIT, "3D FOF seed selection left %lld of %d dense particles undecided",
-                  (long long)nd - kc.next, nd);
+    if (kc.hit || kc.decided != nd) {
+        set_error(RSG_ERR_LIMIT, "3D FOF seed selection left %d of %d dense particles undecided",
+                  nd - kc.decided, nd);
         throw Failure();
     }
-    if (G.e) launch_stats().launches += 2 * (int64_t)kc.iters;
+    if (G.e) launch_stats().launches += 3 * (int64_t)kc.iters;
     phase_mark(st, "fof.elist");
     // non-dense particles: state 0 (never seeds)
     uint8_t *state = ar.get<uint8_t>(n);
-    launch(k_state8, nblk(n, T), T, 0, st, state32, n, state);
+    RSG_CUDA(cudaMemsetAsync(state, 0, n, st));
+    launch(k_state8, nblk(nd, T), T, 0, st, (const int *)dense, nd, (const int *)skip, state);
     phase_mark(st, "fof.seeds");
     if (getenv("RSG_TIMING"))
         fprintf(stderr, "  [fof] dense %d, dense pairs %lld in %d chunk(s), frontier steps %d\n",
