@@ -95,8 +95,10 @@ __global__ void k_bv_best(const int32_t *cF, const int32_t *cW, int64_t nc, cons
     if (c >= nc) return;
     int a = compS[cF[c]], b = compS[cW[c]];
     if (a == b) return;
-    atomicMin(&best[a], (int32_t)c);
-    atomicMin(&best[b], (int32_t)c);
+    // candidates come in ascending order, so most meet a smaller one already
+    // there: a read spares the large sets' words an atomic per candidate
+    if (best[a] > (int32_t)c) atomicMin(&best[a], (int32_t)c);
+    if (best[b] > (int32_t)c) atomicMin(&best[b], (int32_t)c);
     *any = 1;
 }
 // Every root hooks onto the other side of its earliest outgoing merge; of
