@@ -493,16 +493,45 @@ __device__ __forceinline__ bool box_out6(const KNode<6> &nd, const float *c, flo
     return false;
 }
 
-// fast3tree_find_next_closest_distance (src/fast3tree.c:956-1030), with the
-// recursion unrolled onto an explicit stack; the running radius threads
-// through the visits in the reference's order.
+// The first 48 bytes of a node, its box, as three 16-byte loads.
+__device__ __forceinline__ float box_near6(const KNode<6> *nd, const float *c) {
+    const float4 *v = reinterpret_cast<const float4 *>(nd);
+    const float4 a = v[0], b = v[1], e = v[2];
+    const float mn[6] = {a.x, a.y, a.z, a.w, b.x, b.y};
+    const float mx[6] = {b.z, b.w, e.x, e.y, e.z, e.w};
+    float d = 0.f;
+#pragma unroll
+    for (int i = 0; i < 6; i++) {
+        const float g = fmaxf(fmaxf(fsub(mn[i], c[i]), fsub(c[i], mx[i])), 0.f);
+        d = fadd(d, fmul(g, g));
+    }
+    return d;
+}
+// fast3tree_find_next_closest_distance (src/fast3tree.c:956-1030).  The
+// reference first takes the least distance other than 0 in the query's own
+// leaf (or the node above it while the parent's split is degenerate), then
+// visits the rest of the tree depth first, leaving out the nodes at or beyond
+// the running radius r = sqrt(d) and the points not below r * r.  Its
+// value does not depend on the order of the visits: sqrt(r * r) rounds to r
+// for any binary float r short of underflow (Boldo, "Stupid is as stupid
+// does: taking the square root of the square of a floating-point number",
+// 2015), so a point or node left out, its square at or above r * r, could not
+// have lowered r, and the result is the rounded root of the least square over
+// the own node (0 excepted) and every other point.
+// So the walk here climbs from the own node, where the near points are, and
+// takes each sibling on the way nearest child first, with both children
+// tested at their parent; the distance stays squared.  Each lane walks on to
+// its next leaf, then the lanes holding a leaf test their leaves together.
 __device__ float next_closest(const KNode<6> *nodes, int root, const Rec *W, const float *c,
                               bool valid, int *err) {
     const unsigned FULL = 0xffffffffu;
     int nd = root;
-    float r = 0.f;
+    float best = 0.f;
     int stack[RSG_STACK6];
+    float far[RSG_STACK6];
     int sp = 0;
+    const unsigned long long c2[3] = {f2_pack(c[0], c[1]), f2_pack(c[2], c[3]),
+                                      f2_pack(c[4], c[5])};
     if (valid) {
         while (nodes[nd].div >= 0) {
             const KNode<6> &x = nodes[nd];
@@ -514,65 +543,74 @@ __device__ float next_closest(const KNode<6> *nodes, int root, const Rec *W, con
             else break;
         }
         const KNode<6> &o = nodes[nd];
-        float md = 0.f;
         for (int j = 0; j < 6; j++) {
             float dx = fsub(o.mx[j], o.mn[j]);
-            md = fadd(md, fmul(dx, dx));
+            best = fadd(best, fmul(dx, dx));
         }
-        const unsigned long long c2[3] = {f2_pack(c[0], c[1]), f2_pack(c[2], c[3]),
-                                          f2_pack(c[4], c[5])};
         for (int i = 0; i < o.n; i++) {
             unsigned long long q2[3];
             rec_pairs(W + o.start + i, q2);
             float d = dist6_p(c2, q2);
-            if (d && d < md) md = d;
+            if (d && d < best) best = d;
         }
-        r = sqrt_fd(md);
-        stack[sp++] = root;
     }
-    // Each lane walks its own depth-first order (the reference's, with its
-    // own pruning radius) until it reaches its next leaf; then the lanes
-    // holding a leaf test their leaves together.  A lane's sequence of node
-    // tests and leaf updates is unchanged; only its interleaving with the
-    // other lanes is.
-    while (__any_sync(FULL, sp > 0)) {
+    bool go = valid;
+    while (__any_sync(FULL, go)) {
         int leaf = -1;
-        while (sp) {
-            const int ni = stack[--sp];
-            const KNode<6> &x = nodes[ni];
-            if (box_out6(x, c, r) || ni == nd) continue;
-            if (x.div < 0) {
-                leaf = ni;
-                break;
+        while (go && leaf < 0) {
+            int ni;
+            if (sp > 0) {
+                if (far[--sp] >= best) continue;
+                ni = stack[sp];
+            } else {  // climb: the next sibling on the way to the root
+                if (nd == root) {
+                    go = false;
+                    break;
+                }
+                const int p = nodes[nd].parent, l = nodes[p].left;
+                ni = l == nd ? l + 1 : l;
+                nd = p;
+                if (box_near6(nodes + ni, c) >= best) continue;
             }
-            int a = x.left, b = x.left + 1;
-            if (c[x.div] > fmul(0.5f, fadd(x.mn[x.div], x.mx[x.div]))) {
-                a = x.left + 1;
-                b = x.left;
+            for (;;) {
+                const int4 t = reinterpret_cast<const int4 *>(nodes + ni)[3];
+                if (t.z < 0) {  // div
+                    leaf = ni;
+                    break;
+                }
+                int a = t.w, b = t.w + 1;
+                float da = box_near6(nodes + a, c), db = box_near6(nodes + b, c);
+                if (db < da) {
+                    a = t.w + 1;
+                    b = t.w;
+                    const float w = da;
+                    da = db;
+                    db = w;
+                }
+                if (da >= best) break;
+                if (db < best) {
+                    if (sp >= RSG_STACK6) {
+                        atomicExch(err, 1);
+                        go = false;
+                        break;
+                    }
+                    stack[sp] = b;
+                    far[sp++] = db;
+                }
+                ni = a;
             }
-            if (sp + 2 > RSG_STACK6) {
-                atomicExch(err, 1);
-                sp = 0;
-                break;
-            }
-            stack[sp++] = b;
-            stack[sp++] = a;
         }
         if (leaf >= 0) {
-            const KNode<6> &x = nodes[leaf];
-            const unsigned long long c2[3] = {f2_pack(c[0], c[1]), f2_pack(c[2], c[3]),
-                                              f2_pack(c[4], c[5])};
-            float r2 = fmul(r, r);
-            for (int i = 0; i < x.n; i++) {
+            const int s = nodes[leaf].start, n = nodes[leaf].n;
+            for (int i = 0; i < n; i++) {
                 unsigned long long q2[3];
-                rec_pairs(W + x.start + i, q2);
-                float d = dist6_p(c2, q2);
-                if (d < r2) r2 = d;
+                rec_pairs(W + s + i, q2);
+                const float d = dist6_p(c2, q2);
+                if (d < best) best = d;
             }
-            r = sqrt_fd(r2);
         }
     }
-    return r;
+    return sqrt_fd(best);
 }
 
 // Sample queries in tree order: key (node, position in the node) of every
