@@ -1161,20 +1161,37 @@ __global__ void k_halo_scans(rsg_halo *H, const rsg_extra_halo_info *E, int32_t 
 namespace rsg {
 
 // ---- block-cooperative scans for large halos ------------------------------
-// Same arithmetic as corevel/kinetic/more_props/shape above.  The block
-// computes every per-particle operand in parallel (ellipsoidal radius,
-// weights, tensor products, densities, energies); sums that the reference
-// accumulates in array order are then accumulated by warp 0 with one lane
-// per accumulator, walking the staged operands in order, so each sum rounds
-// exactly as the reference's loop while all of them advance together.
-// Threshold decisions (density thresholds, Vmax) become block reductions.
+// Same arithmetic as corevel/kinetic/more_props/shape above, one block per
+// halo.  Sums that the reference accumulates in array order are chains of
+// dependent FP64 roundings, and a large halo's chains set the length of the
+// plain step, so a chain holds nothing but its own additions: most warps of
+// the block compute the operands of the next stretch of records (ellipsoidal
+// radius, weights, tensor products, reciprocals), left out the records that
+// the reference skips, while a warp per kind of chain, one lane per
+// accumulator, adds up the stretch before it from shared memory.  Running
+// means divide by the count; the count's reciprocal is an operand, which
+// leaves four steps of the division in the chain (run_div).  Thresholds,
+// counts and maxima are block reductions.  With every operand computed by
+// the lanes of the chain, FP64 divisions in it, the records read from global
+// memory and the bin and pseudo-evolution scans on one thread, the 38,305
+// records of the largest halo of a 524,288-particle snapshot took 228 ms (and those below
+// 1,024 records, a thread each, 52 ms); now 51 ms for all.
 #define RSG_SB 256
 
-struct BlkBuf {
-    double v[RSG_SB][9];
-    unsigned char skip[RSG_SB];
-    int32_t np[RSG_SB];
-};
+// RN(a / b) for an integer 0 < b < 2^31 from y = RN(1 / b), in three steps
+// (after Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", 1990).  q = RN(a y) is within 1.5 units in the last
+// place (ulp) of a / b.  b q and a are multiples of ulp(q), so the residual
+// r = a - b q, at most 1.5 b ulps, is exact.  q + r y differs from a / b by
+// less than 2^-52 ulp, while a / b, when it is not a double or the midpoint of
+// two, is at least 2^-32 ulp from any midpoint, and it never is a midpoint
+// (b times one has too many bits for a), so the last rounding is that of
+// a / b.  The operands here are differences of float-valued data, far from
+// underflow.
+__device__ __forceinline__ double run_div(double a, double b, double y) {
+    const double q = a * y;
+    return fma(fma(-q, b, a), y, q);
+}
 
 // inclusive count of non-skipped entries up to each thread of a chunk
 __device__ int chunk_prefix(int flag, int *warp_tot) {
@@ -1189,31 +1206,180 @@ __device__ int chunk_prefix(int flag, int *warp_tot) {
     return off + incl;
 }
 
-// deterministic block sum of one double (all threads call; result in all)
-__device__ double bsum(double v, double *sm) {
-    for (int o = 16; o; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = v;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double t = 0;
-        for (int i = 0; i < RSG_SB / 32; i++) t += sm[i];
-        sm[RSG_SB / 32] = t;
+#define RSG_CVC 64  // records per stretch of the core-velocity pipeline
+struct CoreBuf {    // the stretches in flight
+    double x[4][RSG_CVC][3], y[4][RSG_CVC], vel[8][RSG_CVC][3], pr[4][RSG_CVC][3];
+    double var[4][RSG_CVC][3], tv[4][RSG_CVC], tq[4][RSG_CVC];
+};
+// Stretches of a chain: the threads from FIRST on stage NP records each time.
+template <int FIRST, int W>
+struct RunBuf {
+    static constexpr int NP = RSG_SB - FIRST;
+    double v[2][NP][W];
+    int m[2];             // operands staged
+    int wtot[RSG_SB / 32];
+    int base;
+};
+typedef RunBuf<96, 13> MeanBuf;  // pass 2: three warps of chains
+typedef RunBuf<32, 7> ShapeBuf;
+typedef RunBuf<32, 4> EnergyBuf;
+union ScanBuf {
+    CoreBuf core;
+    MeanBuf mean;
+    ShapeBuf shape;
+    EnergyBuf energy;
+};
+__device__ __forceinline__ void stagers_sync(int n) {
+    asm volatile("bar.sync 1, %0;" ::"r"(n) : "memory");
+}
+// Stages one stretch: the stagers with `ok` get consecutive slots of buf
+// (their order is the records'); `put(slot, rank)` writes the operands, rank
+// counting the staged records from 1.  base: records staged before.
+template <class Buf, class Put>
+__device__ __forceinline__ void stage_run(Buf &B, int buf, bool ok, int &base, Put put) {
+    constexpr int FIRST = RSG_SB - Buf::NP;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const unsigned b = __ballot_sync(0xffffffffu, ok);
+    if (lane == 0) B.wtot[w] = __popc(b);
+    stagers_sync(Buf::NP);
+    int off = 0, tot = 0;
+    for (int i = FIRST / 32; i < RSG_SB / 32; i++) {
+        if (i < w) off += B.wtot[i];
+        tot += B.wtot[i];
     }
-    __syncthreads();
-    double r = sm[RSG_SB / 32];
-    __syncthreads();
-    return r;
+    const int at = off + __popc(b & ((1u << lane) - 1u));
+    if (ok) put(B.v[buf][at], base + at + 1);
+    if (threadIdx.x == FIRST) B.m[buf] = tot;
+    base += tot;
+    stagers_sync(Buf::NP);  // wtot may be written again
 }
 
+// calculate_corevel (src/properties.c:165-214): rmax / core_max by
+// reductions, then a pipeline of stretches, one step apart: (0) records and
+// reciprocals staged; (1) warp 0 runs the three means; (2) the products of the
+// variances; (3) warp 1 adds them; (4) the combined variance and its quotient;
+// (5) warp 2 takes the decisions against the running minimum.
+__device__ void corevel_blk(rsg_halo &h, const PotRec *q, int64_t tot, const DevCfg &C,
+                            CoreBuf &B) {
+    __shared__ unsigned long long rm[2];
+    double rt = C.rvir_dens * (4.0 * M_PI / 3.0);
+    if (threadIdx.x == 0) { rm[0] = 0; rm[1] = 0; }
+    __syncthreads();
+    // rmax = largest j with j*j > r2^3 * rt^2 (or -1)
+    long long best = -1;
+    for (int64_t j = threadIdx.x; j < tot; j += blockDim.x) {
+        float r2 = q[j].r2;
+        if ((double)(j * j) > (double)fmul(fmul(r2, r2), r2) * (rt * rt)) best = j;
+    }
+    atomicMax(&rm[0], (unsigned long long)(best + 1));
+    __syncthreads();
+    int64_t rmax = (int64_t)rm[0] - 1;
+    if (rmax < 1) return;
+    long long cb = -1;
+    for (int64_t j = threadIdx.x; j < tot; j += blockDim.x)
+        if ((double)q[j].r2 * 100.0 < (double)q[rmax].r2) cb = j;
+    atomicMax(&rm[1], (unsigned long long)(cb + 1));
+    __syncthreads();
+    int64_t cmax = (int64_t)rm[1] - 1;
+    if (cmax < 100) cmax = 100;
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t nc = (rmax + RSG_CVC - 1) / RSG_CVC;
+    double run = 0;  // warps 0 and 1: mean and variance (lanes 0-2); warp 2: minimum
+    double core_err = 0, core = 0, bulk = 0;
+    int64_t n_core = 0;
+    const int t = (int)threadIdx.x - 96;
+    for (int64_t c = 0; c < nc + 5; c++) {
+        // the stretch of this warp's step and its records
+        const int64_t cc = w == 0 ? c - 1 : w == 1 ? c - 3 : w == 2 ? c - 5
+                           : t < RSG_CVC ? c : c - 2;
+        const bool on = cc >= 0 && cc < nc;
+        const int b = (int)(cc & 3);
+        const int m = on ? (int)min((int64_t)RSG_CVC, rmax - cc * RSG_CVC) : 0;
+        if (w == 0) {
+            if (lane < 3) {
+                const double i0 = (double)(cc * RSG_CVC + 1);
+#pragma unroll 4
+                for (int u = 0; u < m; u++) {
+                    run += run_div(B.x[b][u][lane] - run, i0 + (double)u, B.y[b][u]);
+                    B.vel[cc & 7][u][lane] = run;
+                }
+            }
+        } else if (w == 1) {
+            if (lane < 3) {
+#pragma unroll 8
+                for (int u = 0; u < m; u++) {
+                    run += B.pr[b][u][lane];
+                    B.var[b][u][lane] = run;
+                }
+            }
+        } else if (w == 2) {
+            int last = -1, last_core = -1;
+            double err = core_err;
+            for (int u = 0; u < m; u++) {
+                const int64_t i = cc * RSG_CVC + u;
+                if ((i < 10) || (B.tv[b][u] < run * (i - 3) * i)) {
+                    run = i > 3 ? B.tq[b][u] : 0;
+                    if (i < cmax) {
+                        last_core = u;
+                        err = run;
+                    }
+                    last = u;
+                }
+            }
+            if (lane < 3) {
+                if (last >= 0) bulk = B.vel[cc & 7][last][lane];
+                if (last_core >= 0) {
+                    core = B.vel[cc & 7][last_core][lane];
+                    n_core = cc * RSG_CVC + last_core;
+                    core_err = err;
+                }
+            }
+        } else if (t < RSG_CVC) {
+            if (t < m) {
+                const int64_t i = cc * RSG_CVC + t;
+                for (int k = 0; k < 3; k++) B.x[b][t][k] = (double)q[i].pos[k + 3];
+                B.y[b][t] = 1.0 / (double)(i + 1);
+            }
+        } else if (t < 2 * RSG_CVC) {
+            const int u = t - RSG_CVC;
+            if (u < m)
+                for (int k = 0; k < 3; k++) {
+                    const double before = u ? B.vel[cc & 7][u - 1][k]
+                                            : (cc ? B.vel[(cc - 1) & 7][RSG_CVC - 1][k] : 0.0);
+                    const double x = B.x[b][u][k];
+                    B.pr[b][u][k] = (x - before) * (x - B.vel[cc & 7][u][k]);
+                }
+            const int64_t c4 = c - 4;
+            if (c4 >= 0 && c4 < nc && c4 * RSG_CVC + u < rmax) {
+                const int64_t i = c4 * RSG_CVC + u;
+                const double *v = B.var[c4 & 3][u];
+                const double tv = (v[0] + v[1]) + v[2];
+                B.tv[c4 & 3][u] = tv;
+                B.tq[c4 & 3][u] = tv / (double)((i - 3) * i);
+            }
+        }
+        __syncthreads();
+    }
+    if (w == 2 && lane < 3) {
+        h.corevel[lane] = (float)core;
+        h.bulkvel[lane] = (float)bulk;
+        h.pos[lane + 3] = (float)core;
+        if (lane == 0) {
+            h.n_core = n_core;
+            h.min_vel_err = (float)core_err;
+            h.min_bulkvel_err = (float)run;
+        }
+    }
+    __syncthreads();
+}
+
+// calc_shape (src/properties.c:216-326)
 __device__ void shape_blk(rsg_halo &h, const PotRec *po, int64_t tot, int bound,
-                          const DevCfg &C, BlkBuf &B, int exact) {
-    __shared__ double red_s[RSG_SB / 32 + 1];
+                          const DevCfg &C, ShapeBuf &B) {
     __shared__ double orth[3][3], eig[3], acc[7];
     __shared__ float minr_s;
     __shared__ int64_t it_s;
     __shared__ int done, an_s;
-    __shared__ int wt[RSG_SB / 32];
     // number of analysed particles (bound filter)
     int cntl = 0;
     for (int64_t j = threadIdx.x; j < tot; j += RSG_SB) cntl += !(bound && unbound(po[j]));
@@ -1242,62 +1408,53 @@ __device__ void shape_blk(rsg_halo &h, const PotRec *po, int64_t tot, int bound,
         minr_s = minr;
         it_s = it;
     }
-    (void)wt;
     __syncthreads();
     if (done) return;
     const float hp0 = h.pos[0], hp1 = h.pos[1], hp2 = h.pos[2];
+    constexpr int NP = ShapeBuf::NP, FIRST = RSG_SB - NP;
+    const int64_t nc = (tot + NP - 1) / NP;
     for (int64_t i = 0; i < it_s; i++) {
         double a = 0;  // lane k of warp 0 owns accumulator k (w, m00, m11, m22, m10, m20, m21)
-        double part[7] = {0, 0, 0, 0, 0, 0, 0};  // batched mode: per-thread partial sums
-        for (int64_t b0 = 0; b0 < tot; b0 += RSG_SB) {
-            int64_t j = b0 + threadIdx.x;
-            unsigned char sk = 1;
-            double vv[7];
-            if (j < tot && !(bound && unbound(po[j]))) {
-                const float *p = po[j].pos;
-                double dd[3] = {(double)fsub(p[0], hp0), (double)fsub(p[1], hp1),
-                                (double)fsub(p[2], hp2)};
-                double r = 0, dr;
-                for (int k = 0; k < 3; k++) {
-                    dr = 0;
-                    for (int l = 0; l < 3; l++) dr += orth[k][l] * dd[l];
-                    r += dr * dr / eig[k];
+        int base = 0;
+        for (int64_t c = 0; c <= nc; c++) {
+            if (threadIdx.x >= FIRST) {
+                if (c < nc) {
+                    const int64_t j = c * NP + threadIdx.x - FIRST;
+                    double dd[3], tw = 1.0;
+                    bool ok = j < tot && !(bound && unbound(po[j]));
+                    if (ok) {
+                        const float *p = po[j].pos;
+                        dd[0] = (double)fsub(p[0], hp0);
+                        dd[1] = (double)fsub(p[1], hp1);
+                        dd[2] = (double)fsub(p[2], hp2);
+                        double r = 0, dr;
+                        for (int k = 0; k < 3; k++) {
+                            dr = 0;
+                            for (int l = 0; l < 3; l++) dr += orth[k][l] * dd[l];
+                            r += dr * dr / eig[k];
+                        }
+                        if (r < (double)minr_s) r = minr_s;
+                        ok = r > 0 && r <= 1;
+                        if (ok && C.weighted_shapes) tw = 1.0 / r;
+                    }
+                    stage_run(B, (int)(c & 1), ok, base, [&](double *v, int) {
+                        v[0] = tw;
+                        v[1] = dd[0] * dd[0] * tw;
+                        v[2] = dd[1] * dd[1] * tw;
+                        v[3] = dd[2] * dd[2] * tw;
+                        v[4] = dd[0] * dd[1] * tw;
+                        v[5] = dd[0] * dd[2] * tw;
+                        v[6] = dd[1] * dd[2] * tw;
+                    });
                 }
-                if (r < (double)minr_s) r = minr_s;
-                if (r > 0 && r <= 1) {
-                    double tw = (C.weighted_shapes) ? 1.0 / r : 1.0;
-                    vv[0] = tw;
-                    vv[1] = dd[0] * dd[0] * tw;
-                    vv[2] = dd[1] * dd[1] * tw;
-                    vv[3] = dd[2] * dd[2] * tw;
-                    vv[4] = dd[0] * dd[1] * tw;
-                    vv[5] = dd[0] * dd[2] * tw;
-                    vv[6] = dd[1] * dd[2] * tw;
-                    sk = 0;
-                }
-            }
-            if (!exact) {
-                if (!sk)
-                    for (int c = 0; c < 7; c++) part[c] += vv[c];
-                continue;
-            }
-            if (!sk)
-                for (int c = 0; c < 7; c++) B.v[threadIdx.x][c] = vv[c];
-            B.skip[threadIdx.x] = sk;
-            __syncthreads();
-            if (threadIdx.x < 7) {
-                int m = (tot - b0) < RSG_SB ? (int)(tot - b0) : RSG_SB;
-                int c = threadIdx.x;
-                for (int t = 0; t < m; t++)
-                    if (!B.skip[t]) a += B.v[t][c];
+            } else if (c > 0 && threadIdx.x < 7) {
+                const int b = (int)((c - 1) & 1), m = B.m[b];
+                const double *v = &B.v[b][0][threadIdx.x];
+#pragma unroll 8
+                for (int t = 0; t < m; t++) a += v[7 * t];
             }
             __syncthreads();
         }
-        if (!exact)
-            for (int c = 0; c < 7; c++) {
-                double t = bsum(part[c], red_s);
-                if (threadIdx.x == c) a = t;
-            }
         if (threadIdx.x < 7) acc[threadIdx.x] = a;
         __syncthreads();
         if (threadIdx.x == 0) {
@@ -1374,15 +1531,101 @@ __device__ void blk_argmax(double &cv, int64_t &j, double *scv, int64_t *sj) {
     __syncthreads();
 }
 
+// Runs f(j, np) for every analysed record j < tot, np counting them from 1
+// (all threads of the block call it together).
+template <class F>
+__device__ void each_counted(const PotRec *po, int64_t tot, int bound, int *wt, int *last, F f) {
+    int64_t base = 0;
+    for (int64_t b0 = 0; b0 < tot; b0 += RSG_SB) {
+        const int64_t j = b0 + threadIdx.x;
+        const int ok = j < tot && !(bound && unbound(po[j]));
+        const int incl = chunk_prefix(ok, wt);
+        if (ok) f(j, base + incl);
+        if (threadIdx.x == RSG_SB - 1) *last = incl;
+        __syncthreads();
+        base += *last;
+        __syncthreads();
+    }
+}
+
+// calc_scale_radius (src/nfw.c:130-173) and _calc_pseudo_evolution_masses
+// (src/properties.c:351-382), the bins' edges, counts and maxima by the block
+__device__ void radii_blk(rsg_halo &h, float mvir, float scale, const PotRec *po, int64_t dtot,
+                          int64_t tot, int bound, const DevCfg &C, int *wt, int *last) {
+    __shared__ float br[51], w[50];
+    __shared__ long long an_s, npd_s;
+    __shared__ unsigned long long mx_s;
+    for (int i = threadIdx.x; i < 51; i += RSG_SB) br[i] = 0;
+    for (int i = threadIdx.x; i < 50; i += RSG_SB) w[i] = 0;
+    if (threadIdx.x == 0) {
+        an_s = npd_s = 0;
+        mx_s = 0;
+        h.rs = h.klypin_rs = klypin_rs(mvir, h.r, h.vmax, h.rvmax, scale);
+    }
+    __syncthreads();
+    long long an = 0;
+    for (int64_t i = threadIdx.x; i < dtot - 1; i += RSG_SB) an += !(bound && unbound(po[i]));
+    for (int o = 16; o; o >>= 1) an += __shfl_down_sync(0xffffffffu, an, o);
+    if ((threadIdx.x & 31) == 0 && an) atomicAdd((unsigned long long *)&an_s, (unsigned long long)an);
+    __syncthreads();
+    an = an_s;
+    if (an >= 100) {
+        int64_t pp = (int64_t)ceil(((double)an / (double)50));
+        if (pp < 15) pp = (an) / ((int64_t)(an / 15));
+        // every pp-th analysed record closes a bin
+        each_counted(po, dtot - 1, bound, wt, last, [&](int64_t i, int64_t c) {
+            const int64_t nb = c / pp;
+            if (nb * pp != c || nb > 50) return;
+            br[nb] = (float)(1e3 * 0.5 * (sqrt((double)po[i].r2) + sqrt((double)po[i + 1].r2)));
+            w[nb - 1] = 1;
+        });
+        if (threadIdx.x == 0) {
+            int64_t nb = an / pp;
+            if (nb > 50) nb = 50;
+            float b2[51], w2[50];
+            for (int i = 0; i < 51; i++) b2[i] = br[i];
+            for (int i = 0; i < 50; i++) w2[i] = w[i];
+            for (int i = 0; i < nb; i++)
+                if ((double)b2[i] * 1e-3 < 3 * C.force_res) w2[i] = 0.1f;
+            float chi2 = 0.0f;
+            h.rs = fit_bins(h.klypin_rs, b2, w2, nb, &chi2);
+            h.chi2 = chi2;
+        }
+    }
+    __syncthreads();
+    double rpd = (double)h.rs * 4.0;
+    if (rpd < (double)h.r / 5.0) rpd = (double)h.r / 5.0;
+    rpd *= 1e-3;
+    double mx = 0;
+    long long npd = 0;
+    each_counted(po, tot, bound, wt, last, [&](int64_t j, int64_t np_) {
+        const double r = sqrt((double)po[j].r2);
+        double r32 = sqrt(r);
+        r32 = r32 * r32 * r32;
+        const double v = (double)(np_ * np_) / r32;
+        if (v > mx) mx = v;
+        if (r < rpd) npd = np_;  // counts grow with j: the largest is the last
+    });
+    // not negative: the bits order them
+    atomicMax(&mx_s, (unsigned long long)__double_as_longlong(mx));
+    atomicMax((unsigned long long *)&npd_s, (unsigned long long)npd);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        mx = __longlong_as_double((long long)mx_s);
+        h.m_pe_d = (float)(npd_s * C.particle_mass);
+        h.m_pe_b = (float)(C.particle_mass * pow(mx, 2.0 / 3.0) /
+                           cbrt(4.0 * M_PI * C.rvir_dens_z0 / 3.0));
+    }
+    __syncthreads();
+}
+
 __device__ void more_props_blk(rsg_halo &h, const PotRec *po, int64_t tot, int bound,
-                               const DevCfg &C, BlkBuf &B, int exact) {
-    __shared__ double red_m[RSG_SB / 32 + 1];
+                               const DevCfg &C, ScanBuf &B) {
     __shared__ MPState S;
-    __shared__ int want;
-    __shared__ int wt[RSG_SB / 32];
+    __shared__ int wt[RSG_SB / 32], last;
     __shared__ double scv[RSG_SB / 32];
     __shared__ int64_t sj[RSG_SB / 32];
-    __shared__ unsigned long long red[8];
+    __shared__ unsigned long long red[8], nhs;
     float scale = (float)C.scale_now;
     const double f43 = 4.0 * M_PI / 3.0;
     const double dth = C.thresh_dens[0] * f43, d1 = C.thresh_dens[1] * f43;
@@ -1394,30 +1637,18 @@ __device__ void more_props_blk(rsg_halo &h, const PotRec *po, int64_t tot, int b
     if (threadIdx.x < 8) red[threadIdx.x] = 0;
     if (threadIdx.x == 0) { S.j0 = INT64_MAX; }
     __syncthreads();
-    int64_t base_np = 0;
     int64_t l_pmd = 0, l_dtot = 0, l_npa[4] = {0, 0, 0, 0}, l_npv = 0, l_j0 = INT64_MAX;
-    for (int64_t b0 = 0; b0 < tot; b0 += RSG_SB) {
-        int64_t j = b0 + threadIdx.x;
-        int ok = (j < tot) && !(bound && unbound(po[j]));
-        int incl = chunk_prefix(ok, wt);
-        int64_t np_ = base_np + incl;
-        if (ok) {
-            double r = sqrt((double)po[j].r2);
-            if (r < C.force_res) r = C.force_res;
-            double cd = ((double)np_ / (r * r * r));
-            if (cd > dth) { l_pmd = np_; l_dtot = j; if (j < l_j0) l_j0 = j; }
-            if (cd > d1) l_npa[0] = np_;
-            if (cd > d2) l_npa[1] = np_;
-            if (cd > d3) l_npa[2] = np_;
-            if (cd > d4) l_npa[3] = np_;
-            if (cd > rth) l_npv = np_;
-        }
-        __syncthreads();
-        if (threadIdx.x == RSG_SB - 1) B.np[0] = incl;
-        __syncthreads();
-        base_np += B.np[0];
-        __syncthreads();
-    }
+    each_counted(po, tot, bound, wt, &last, [&](int64_t j, int64_t np_) {
+        double r = sqrt((double)po[j].r2);
+        if (r < C.force_res) r = C.force_res;
+        double cd = ((double)np_ / (r * r * r));
+        if (cd > dth) { l_pmd = np_; l_dtot = j; if (j < l_j0) l_j0 = j; }
+        if (cd > d1) l_npa[0] = np_;
+        if (cd > d2) l_npa[1] = np_;
+        if (cd > d3) l_npa[2] = np_;
+        if (cd > d4) l_npa[3] = np_;
+        if (cd > rth) l_npv = np_;
+    });
     // counts grow with j, so the last qualifying value is the maximum
     atomicMax(&red[0], (unsigned long long)l_pmd);
     atomicMax(&red[1], (unsigned long long)l_dtot * (l_pmd > 0));
@@ -1425,34 +1656,33 @@ __device__ void more_props_blk(rsg_halo &h, const PotRec *po, int64_t tot, int b
     atomicMax(&red[6], (unsigned long long)l_npv);
     atomicMin((unsigned long long *)&S.j0, (unsigned long long)l_j0);
     __syncthreads();
-    // Vmax: first maximum of np/r over qualifying particles at or after j0
-    double bcv = -1;
-    int64_t bj = INT64_MAX;
-    base_np = 0;
-    for (int64_t b0 = 0; b0 < tot; b0 += RSG_SB) {
-        int64_t j = b0 + threadIdx.x;
-        int ok = (j < tot) && !(bound && unbound(po[j]));
-        int incl = chunk_prefix(ok, wt);
-        int64_t np_ = base_np + incl;
-        if (ok && j >= S.j0) {
-            double r = sqrt((double)po[j].r2);
-            if (r < C.force_res) r = C.force_res;
-            double cd = ((double)np_ / (r * r * r));
-            if (cd > rth) {
-                double cv = (double)np_ / r;
-                if (cv > bcv || (cv == bcv && j < bj)) { bcv = cv; bj = j; }
-            }
-        }
-        __syncthreads();
-        if (threadIdx.x == RSG_SB - 1) B.np[0] = incl;
-        __syncthreads();
-        base_np += B.np[0];
-        __syncthreads();
-    }
-    blk_argmax(bcv, bj, scv, sj);
+    // the pass that is not analysed leaves only its mass
+    const bool want = (!bound) == (!C.bound_props);
     if (threadIdx.x == 0) {
         S.pmd = (int64_t)red[0];
         S.dtot = (int64_t)red[1];
+        S.m = S.pmd * C.particle_mass;
+        if (!bound) h.m = (float)S.m;
+        else h.mgrav = (float)S.m;
+        nhs = (unsigned long long)INT64_MAX;
+    }
+    __syncthreads();
+    if (!want) return;
+    // Vmax: first maximum of np/r over qualifying particles at or after j0
+    double bcv = -1;
+    int64_t bj = INT64_MAX;
+    each_counted(po, tot, bound, wt, &last, [&](int64_t j, int64_t np_) {
+        if (j < S.j0) return;
+        double r = sqrt((double)po[j].r2);
+        if (r < C.force_res) r = C.force_res;
+        double cd = ((double)np_ / (r * r * r));
+        if (cd > rth) {
+            double cv = (double)np_ / r;
+            if (cv > bcv || (cv == bcv && j < bj)) { bcv = cv; bj = j; }
+        }
+    });
+    blk_argmax(bcv, bj, scv, sj);
+    if (threadIdx.x == 0) {
         for (int k = 0; k < 4; k++) S.npa[k] = (int64_t)red[2 + k];
         S.npv = (int64_t)red[6];
         S.vmax = 0;
@@ -1463,149 +1693,98 @@ __device__ void more_props_blk(rsg_halo &h, const PotRec *po, int64_t tot, int b
             if (r < C.force_res) r = C.force_res;
             S.rvmax = r;
         }
-        S.avg = 0;
-        S.nhalf = 0;
     }
     __syncthreads();
-    // pass 2 (src/properties.c:435-448): warp 0, lanes 0-2 own L[k], lanes
-    // 3-5 xavg[k], lanes 6-8 vavg[k] and vrms[k]
-    if (!exact) {
-        // batched mode: block sums; running means become plain means and the
-        // running second moments a two-pass sum about the mean
-        double lp[3] = {0, 0, 0}, xs[3] = {0, 0, 0}, vs[3] = {0, 0, 0};
-        int64_t cnt = 0, nh = INT64_MAX;
-        const float *c = h.pos;
-        int64_t base = 0;
-        for (int64_t b0 = 0; b0 < S.dtot; b0 += RSG_SB) {
-            int64_t j = b0 + threadIdx.x;
-            int ok = j < S.dtot && !(bound && unbound(po[j]));
-            int incl = chunk_prefix(ok, wt);
-            if (ok) {
-                const float *p = po[j].pos;
-                for (int k = 0; k < 3; k++) {
-                    int x = (k + 1) % 3, y = (k + 2) % 3;
-                    lp[k] += (double)fmul(fsub(p[x], c[x]), fsub(p[y + 3], c[y + 3]));
-                    lp[k] -= (double)fmul(fsub(p[y], c[y]), fsub(p[x + 3], c[x + 3]));
-                    xs[k] += (double)p[k];
-                    vs[k] += (double)p[k + 3];
-                }
-                cnt++;
-                int64_t run = base + incl;
-                if (j >= 1 && run * 2 >= S.pmd && j < nh) nh = j;
-            }
-            __syncthreads();
-            if (threadIdx.x == RSG_SB - 1) B.np[0] = incl;
-            __syncthreads();
-            base += B.np[0];
-            __syncthreads();
-        }
-        double tot_c = bsum((double)cnt, red_m);
-        for (int k = 0; k < 3; k++) {
-            double t = bsum(lp[k], red_m);
-            if (threadIdx.x == 0) S.L[k] = t;
-            t = bsum(xs[k], red_m);
-            if (threadIdx.x == 0) S.xa[k] = tot_c > 0 ? t / tot_c : 0;
-            t = bsum(vs[k], red_m);
-            if (threadIdx.x == 0) S.va[k] = tot_c > 0 ? t / tot_c : 0;
-        }
-        __syncthreads();
-        double v2[3] = {0, 0, 0};
-        for (int64_t j = threadIdx.x; j < S.dtot; j += RSG_SB) {
-            if (bound && unbound(po[j])) continue;
-            for (int k = 0; k < 3; k++) {
-                double d = (double)po[j].pos[k + 3] - S.va[k];
-                v2[k] += d * d;
-            }
-        }
-        for (int k = 0; k < 3; k++) {
-            double t = bsum(v2[k], red_m);
-            if (threadIdx.x == 0) S.vrms[k] = t;
-        }
-        __shared__ unsigned long long nhs;
-        if (threadIdx.x == 0) nhs = (unsigned long long)INT64_MAX;
-        __syncthreads();
-        atomicMin(&nhs, (unsigned long long)nh);
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            S.avg = (int64_t)tot_c;
-            S.nhalf = (nhs == (unsigned long long)INT64_MAX) ? 0 : (int64_t)nhs;
-        }
-        __syncthreads();
-    } else {
-        double acc_a = 0, acc_b = 0;
-        int64_t avg = 0, nhalf = 0;
-        const float *c = h.pos;
-        for (int64_t b0 = 0; b0 < S.dtot; b0 += RSG_SB) {
-            int64_t j = b0 + threadIdx.x;
-            unsigned char sk = 1;
-            if (j < S.dtot && !(bound && unbound(po[j]))) {
-                for (int d = 0; d < 6; d++) B.v[threadIdx.x][d] = (double)po[j].pos[d];
-                sk = 0;
-            }
-            B.skip[threadIdx.x] = sk;
-            __syncthreads();
-            if (threadIdx.x < 9) {
-                int lane = threadIdx.x;
-                int m = (S.dtot - b0) < RSG_SB ? (int)(S.dtot - b0) : RSG_SB;
-                for (int t = 0; t < m; t++) {
-                    if (B.skip[t]) continue;
-                    avg++;
-                    if (avg * 2 >= S.pmd && !nhalf) nhalf = b0 + t;
-                    const double *p = B.v[t];
-                    if (lane < 3) {
-                        int x = (lane + 1) % 3, y = (lane + 2) % 3;
+    // pass 2 (src/properties.c:435-448): warp 0 lane k owns L[k], warp 1
+    // xavg[k], warp 2 vavg[k] and vrms[k]
+    {
+        constexpr int NP = MeanBuf::NP, FIRST = RSG_SB - NP;
+        const int64_t nc = (S.dtot + NP - 1) / NP;
+        const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        double a = 0, a2 = 0;
+        int base = 0, seen = 0;
+        unsigned long long nh = (unsigned long long)INT64_MAX;
+        const float c0 = h.pos[0], c1 = h.pos[1], c2 = h.pos[2], c3 = h.pos[3], c4 = h.pos[4],
+                    c5 = h.pos[5];
+        for (int64_t c = 0; c <= nc; c++) {
+            if (threadIdx.x >= FIRST) {
+                if (c < nc) {
+                    const int64_t j = c * NP + threadIdx.x - FIRST;
+                    const bool ok = j < S.dtot && !(bound && unbound(po[j]));
+                    stage_run(B.mean, (int)(c & 1), ok, base, [&](double *v, int run) {
+                        const float *p = po[j].pos;
                         // L[0] += (p1-c1)(p5-c5) - ..., as add_ang_mom orders them
-                        float pa = fmul(fsub((float)p[x], c[x]), fsub((float)p[y + 3], c[y + 3]));
-                        float pb = fmul(fsub((float)p[y], c[y]), fsub((float)p[x + 3], c[x + 3]));
-                        acc_a += (double)pa;
-                        acc_a -= (double)pb;
-                    } else if (lane < 6) {
-                        int k = lane - 3;
-                        acc_a += (p[k] - acc_a) / ((double)avg);
-                    } else {
-                        int k = lane - 6;
-                        double md = p[k + 3] - acc_a;
-                        acc_a += md / (double)avg;
-                        acc_b += md * (p[k + 3] - acc_a);
+                        const float x0 = fsub(p[0], c0), x1 = fsub(p[1], c1), x2 = fsub(p[2], c2);
+                        const float v0 = fsub(p[3], c3), v1 = fsub(p[4], c4), v2 = fsub(p[5], c5);
+                        v[0] = (double)fmul(x1, v2);
+                        v[1] = (double)fmul(x2, v0);
+                        v[2] = (double)fmul(x0, v1);
+                        v[3] = (double)fmul(x2, v1);
+                        v[4] = (double)fmul(x0, v2);
+                        v[5] = (double)fmul(x1, v0);
+                        for (int k = 0; k < 6; k++) v[6 + k] = (double)p[k];
+                        v[12] = 1.0 / (double)run;
+                        if (j >= 1 && (int64_t)run * 2 >= S.pmd && (unsigned long long)j < nh)
+                            nh = (unsigned long long)j;
+                    });
+                }
+            } else if (c > 0 && lane < 3) {
+                const int b = (int)((c - 1) & 1), m = B.mean.m[b];
+                const double(*v)[13] = B.mean.v[b];
+                const double s0 = (double)(seen + 1);
+                if (w == 0) {
+#pragma unroll 4
+                    for (int t = 0; t < m; t++) {
+                        a += v[t][lane];
+                        a -= v[t][3 + lane];
+                    }
+                } else if (w == 1) {
+#pragma unroll 4
+                    for (int t = 0; t < m; t++)
+                        a += run_div(v[t][6 + lane] - a, s0 + (double)t, v[t][12]);
+                } else {
+#pragma unroll 4
+                    for (int t = 0; t < m; t++) {
+                        const double x = v[t][9 + lane], md = x - a;
+                        a += run_div(md, s0 + (double)t, v[t][12]);
+                        a2 += md * (x - a);
                     }
                 }
+                seen += m;
             }
             __syncthreads();
         }
-        if (threadIdx.x < 3) S.L[threadIdx.x] = acc_a;
-        else if (threadIdx.x < 6) S.xa[threadIdx.x - 3] = acc_a;
-        else if (threadIdx.x < 9) { S.va[threadIdx.x - 6] = acc_a; S.vrms[threadIdx.x - 6] = acc_b; }
-        if (threadIdx.x == 0) { S.avg = avg; S.nhalf = nhalf; }
+        if (threadIdx.x >= FIRST && nh != (unsigned long long)INT64_MAX) atomicMin(&nhs, nh);
+        if (lane < 3) {
+            if (w == 0) S.L[lane] = a;
+            if (w == 1) S.xa[lane] = a;
+            if (w == 2) { S.va[lane] = a; S.vrms[lane] = a2; }
+        }
+        if (threadIdx.x == 0) S.avg = seen;
         __syncthreads();
     }
     if (threadIdx.x == 0) {
-        S.m = S.pmd * C.particle_mass;
-        if (!bound) h.m = (float)S.m;
-        else h.mgrav = (float)S.m;
+        S.nhalf = nhs == (unsigned long long)INT64_MAX ? 0 : (int64_t)nhs;
         for (int k = 0; k < 3; k++) S.vrms[k] = (S.avg > 0) ? (S.vrms[k] / S.avg) : 0;
-        want = ((!bound) == (!C.bound_props));
-        if (want) {
-            double ds;
-            h.Xoff = h.Voff = 0;
-            for (int k = 0; k < 3; k++) {
-                ds = S.xa[k] - (double)h.pos[k];
-                h.Xoff = (float)((double)h.Xoff + ds * ds);
-                ds = S.va[k] - (double)h.pos[k + 3];
-                h.Voff = (float)((double)h.Voff + ds * ds);
-            }
-            for (int k = 0; k < 4; k++) h.alt_m[k] = (float)(S.npa[k] * C.particle_mass);
-            h.Xoff = (float)(sqrt((double)h.Xoff) * 1e3);
-            h.Voff = sqrt_fd(h.Voff);
-            h.vrms = (float)sqrt(S.vrms[0] + S.vrms[1] + S.vrms[2]);
-            h.vmax = (float)(RSG_VMAX_CONST * sqrt(S.vmax * (C.particle_mass / (double)scale)));
-            h.rvmax = (float)(S.rvmax * 1e3);
-            h.halfmass_radius = (float)(sqrt((double)po[S.nhalf].r2) * 1e3);
-            h.r = (float)(cbrt((3.0 / (4.0 * M_PI)) * S.npa[2] / C.thresh_dens[3]) * 1e3);
+        double ds;
+        h.Xoff = h.Voff = 0;
+        for (int k = 0; k < 3; k++) {
+            ds = S.xa[k] - (double)h.pos[k];
+            h.Xoff = (float)((double)h.Xoff + ds * ds);
+            ds = S.va[k] - (double)h.pos[k + 3];
+            h.Voff = (float)((double)h.Voff + ds * ds);
         }
+        for (int k = 0; k < 4; k++) h.alt_m[k] = (float)(S.npa[k] * C.particle_mass);
+        h.Xoff = (float)(sqrt((double)h.Xoff) * 1e3);
+        h.Voff = sqrt_fd(h.Voff);
+        h.vrms = (float)sqrt(S.vrms[0] + S.vrms[1] + S.vrms[2]);
+        h.vmax = (float)(RSG_VMAX_CONST * sqrt(S.vmax * (C.particle_mass / (double)scale)));
+        h.rvmax = (float)(S.rvmax * 1e3);
+        h.halfmass_radius = (float)(sqrt((double)po[S.nhalf].r2) * 1e3);
+        h.r = (float)(cbrt((3.0 / (4.0 * M_PI)) * S.npa[2] / C.thresh_dens[3]) * 1e3);
     }
     __syncthreads();
-    if (!want) return;
-    shape_blk(h, po, S.npa[2], bound, C, B, exact);
+    shape_blk(h, po, S.npa[2], bound, C, B.shape);
     __syncthreads();
     if (threadIdx.x == 0) {
         h.b_to_a2 = h.b_to_a;
@@ -1615,73 +1794,53 @@ __device__ void more_props_blk(rsg_halo &h, const PotRec *po, int64_t tot, int b
         h.r = (float)(cbrt((3.0 / (4.0 * M_PI)) * S.pmd / C.thresh_dens[0]) * 1e3);
     }
     __syncthreads();
-    shape_blk(h, po, S.dtot, bound, C, B, exact);
+    shape_blk(h, po, S.dtot, bound, C, B.shape);
     __syncthreads();
-    // estimate_total_energy over [0, dtot) in descending order: lane 0 sums
-    // ke, lane 1 the two coupled potential sums (src/properties.c:328-349)
-    __shared__ double en[3];
-    if (!exact) {
-        // tphi = sum a_i + sum b_i * (number of qualifying particles before i)
-        double kes = 0, ts = 0;
-        int64_t base = 0;
-        for (int64_t b0 = 0; b0 < S.dtot; b0 += RSG_SB) {
-            int64_t i = b0 + threadIdx.x;
-            int ok = i < S.dtot && po[i].pe > (double)po[i].ke;
-            int incl = chunk_prefix(ok, wt);
-            if (ok) {
-                double r = sqrt((double)po[i].r2);
-                if (r < C.force_res) r = C.force_res;
-                kes += (double)po[i].ke;
-                ts += C.particle_mass * i / r + (C.particle_mass / r) * (double)(base + incl - 1);
-            }
-            __syncthreads();
-            if (threadIdx.x == RSG_SB - 1) B.np[0] = incl;
-            __syncthreads();
-            base += B.np[0];
-            __syncthreads();
-        }
-        double t1 = bsum(kes, red_m), t2 = bsum(ts, red_m);
-        if (threadIdx.x == 0) { en[0] = t1; en[1] = t2; }
-        __syncthreads();
-    } else {
-        double acc_a = 0, acc_b = 0;
-        for (int64_t top = S.dtot - 1; top >= 0; top -= RSG_SB) {
-            int64_t i = top - threadIdx.x;
-            unsigned char sk = 1;
-            if (i >= 0 && po[i].pe > (double)po[i].ke) {
-                double r = sqrt((double)po[i].r2);
-                if (r < C.force_res) r = C.force_res;
-                B.v[threadIdx.x][0] = (double)po[i].ke;
-                B.v[threadIdx.x][1] = C.particle_mass * i / r;
-                B.v[threadIdx.x][2] = C.particle_mass / r;
-                sk = 0;
-            }
-            B.skip[threadIdx.x] = sk;
-            __syncthreads();
-            int m = (top + 1) < RSG_SB ? (int)(top + 1) : RSG_SB;
-            if (threadIdx.x == 0) {
-                for (int t = 0; t < m; t++)
-                    if (!B.skip[t]) acc_a += B.v[t][0];
-            } else if (threadIdx.x == 1) {
-                for (int t = 0; t < m; t++)
-                    if (!B.skip[t]) {
-                        acc_a += B.v[t][1] + acc_b;
-                        acc_b += B.v[t][2];
-                    }
+    // estimate_total_energy over [0, dtot) in descending order: lane 0 the two
+    // coupled potential sums, lane 1 the kinetic one in the same steps (its
+    // second operand is 0, and adding 0 changes nothing) (src/properties.c:
+    // 328-349)
+    __shared__ double en[2];
+    {
+        constexpr int NP = EnergyBuf::NP, FIRST = RSG_SB - NP;
+        const int64_t nc = (S.dtot + NP - 1) / NP;
+        double a = 0, run = 0;
+        int base = 0;
+        for (int64_t c = 0; c <= nc; c++) {
+            if (threadIdx.x >= FIRST) {
+                if (c < nc) {
+                    const int64_t i = S.dtot - 1 - (c * NP + threadIdx.x - FIRST);
+                    const bool ok = i >= 0 && po[i].pe > (double)po[i].ke;
+                    stage_run(B.energy, (int)(c & 1), ok, base, [&](double *v, int) {
+                        double r = sqrt((double)po[i].r2);
+                        if (r < C.force_res) r = C.force_res;
+                        v[0] = C.particle_mass * i / r;
+                        v[1] = (double)po[i].ke;
+                        v[2] = C.particle_mass / r;
+                        v[3] = 0;
+                    });
+                }
+            } else if (c > 0 && threadIdx.x < 2) {
+                const int b = (int)((c - 1) & 1), m = B.energy.m[b];
+                const double *v = &B.energy.v[b][0][threadIdx.x];
+#pragma unroll 4
+                for (int t = 0; t < m; t++) {
+                    a += v[4 * t] + run;
+                    run += v[4 * t + 2];
+                }
             }
             __syncthreads();
         }
-        if (threadIdx.x == 0) en[0] = acc_a;
-        if (threadIdx.x == 1) en[1] = acc_a;
+        if (threadIdx.x < 2) en[threadIdx.x] = a;
         __syncthreads();
     }
+    radii_blk(h, (float)S.m, scale, po, S.dtot, tot, bound, C, wt, &last);
     if (threadIdx.x == 0) {
         double rvir = cbrt((3.0 / (4.0 * M_PI)) * S.npv / C.rvir_dens) * 1e3;
         double mvir = S.npv * C.particle_mass, m = S.m;
-        scale_radius(h, (float)m, h.r, h.vmax, h.rvmax, scale, po, S.dtot, bound, C);
         for (int j = 0; j < 3; j++) h.J[j] = (float)(C.particle_mass * (double)scale * S.L[j]);
         {
-            double ke = en[0], tphi = en[1] / 2.0;
+            double ke = en[1], tphi = en[0] / 2.0;
             h.kin_to_pot = 0;
             if (tphi) h.kin_to_pot = (float)(ke / tphi);
             float sn = (float)C.scale_now;
@@ -1691,64 +1850,6 @@ __device__ void more_props_blk(rsg_halo &h, const PotRec *po, int64_t tot, int b
                     sqrt(S.L[0] * S.L[0] + S.L[1] * S.L[1] + S.L[2] * S.L[2]);
         h.spin = (float)((m > 0) ? (Jh * sqrt(fabs((double)h.energy)) / (RSG_GC * pow(m, 2.5))) : 0);
         h.bullock_spin = (float)((m > 0) ? (Jh / (mvir * sqrt(2.0 * RSG_GC * mvir * rvir * (double)scale / 1e3))) : 0);
-        pseudo_masses(h, po, tot, bound, C);
-    }
-    __syncthreads();
-}
-
-// calculate_corevel with the block: rmax / core_max by reductions, then the
-// three running means and variances on lanes 0-2 of warp 0 (the combined
-// variance, and so every decision, is shared through shuffles).
-__device__ void corevel_blk(rsg_halo &h, const PotRec *q, int64_t tot, const DevCfg &C) {
-    __shared__ unsigned long long rm[2];
-    double rt = C.rvir_dens * (4.0 * M_PI / 3.0);
-    if (threadIdx.x == 0) { rm[0] = 0; rm[1] = 0; }
-    __syncthreads();
-    // rmax = largest j with j*j > r2^3 * rt^2 (or -1)
-    long long best = -1;
-    for (int64_t j = threadIdx.x; j < tot; j += blockDim.x) {
-        float r2 = q[j].r2;
-        if ((double)(j * j) > (double)fmul(fmul(r2, r2), r2) * (rt * rt)) best = j;
-    }
-    atomicMax(&rm[0], (unsigned long long)(best + 1));
-    __syncthreads();
-    int64_t rmax = (int64_t)rm[0] - 1;
-    if (rmax < 1) return;
-    long long cb = -1;
-    for (int64_t j = threadIdx.x; j < tot; j += blockDim.x)
-        if ((double)q[j].r2 * 100.0 < (double)q[rmax].r2) cb = j;
-    atomicMax(&rm[1], (unsigned long long)(cb + 1));
-    __syncthreads();
-    int64_t cmax = (int64_t)rm[1] - 1;
-    if (cmax < 100) cmax = 100;
-    if (threadIdx.x < 3) {
-        const unsigned mask = 0x7u;
-        int k = threadIdx.x;
-        double vel = 0, var = 0, bv = 0;
-        for (int64_t i = 0; i < rmax; i++) {
-            double x = (double)q[i].pos[k + 3];
-            double dl = x - vel;
-            vel += dl / ((double)(i + 1));
-            var += dl * (x - vel);
-            double v0 = __shfl_sync(mask, var, 0), v1 = __shfl_sync(mask, var, 1),
-                   v2 = __shfl_sync(mask, var, 2);
-            double tv = (v0 + v1) + v2;
-            if ((i < 10) || (tv < bv * (i - 3) * i)) {
-                if (i > 3) bv = tv / (double)((i - 3) * i);
-                else bv = 0;
-                if (i < cmax) {
-                    if (k == 0) {
-                        h.n_core = i;
-                        h.min_vel_err = (float)bv;
-                    }
-                    h.corevel[k] = (float)vel;
-                }
-                h.bulkvel[k] = (float)vel;
-                if (k == 0) h.min_bulkvel_err = (float)bv;
-            }
-        }
-        __syncwarp(mask);
-        h.pos[k + 3] = h.corevel[k];
     }
     __syncthreads();
 }
@@ -1756,14 +1857,14 @@ __device__ void corevel_blk(rsg_halo &h, const PotRec *q, int64_t tot, const Dev
 __global__ void __launch_bounds__(RSG_SB) k_halo_scans_blk(rsg_halo *H, const rsg_extra_halo_info *E,
                                                            const int32_t *list, PotRec *PO,
                                                            const int32_t *toff, const int32_t *kept,
-                                                           const DevCfg *Cp, int exact) {
-    __shared__ BlkBuf B;
+                                                           const DevCfg *Cp) {
+    __shared__ ScanBuf B;
     int h = list[blockIdx.x];
     rsg_halo &hh = H[h];
     const DevCfg &C = *Cp;
     PotRec *q = PO + toff[h];
     int64_t tot = kept[h];
-    corevel_blk(hh, q, tot, C);
+    corevel_blk(hh, q, tot, C, B.core);
     __syncthreads();
     float sn = (float)C.scale_now;
     const float *vc = (E[h].sub_of > -1) ? hh.corevel : hh.bulkvel;
@@ -1783,20 +1884,23 @@ __global__ void __launch_bounds__(RSG_SB) k_halo_scans_blk(rsg_halo *H, const rs
         }
     }
     __syncthreads();
-    more_props_blk(hh, q, tot, 0, C, B, exact);
-    more_props_blk(hh, q, tot, 1, C, B, exact);
+    more_props_blk(hh, q, tot, 0, C, B);
+    more_props_blk(hh, q, tot, 1, C, B);
 }
 
-// halos split by size: small ones one thread each, large ones one block each
-__global__ void k_scan_split(const rsg_halo *H, int32_t NH, const int32_t *kept, int32_t big,
+// halos split by size: small ones one thread each, large ones one block each,
+// above RSG_PLAIN_BLK records (work: the counters' classes, split at 1024)
+#define RSG_PLAIN_BLK 64
+#define RSG_PLAIN_FEW 7000
+__global__ void k_scan_split(const rsg_halo *H, int32_t NH, const int32_t *kept,
                              int32_t *fsmall, int32_t *fbig, unsigned long long *work) {
     int h = blockIdx.x * blockDim.x + threadIdx.x;
     if (h >= NH) return;
     bool act = H[h].num_p >= 1;
-    fbig[h] = act && kept[h] > big;
-    fsmall[h] = act && kept[h] <= big;
+    fbig[h] = act && kept[h] > RSG_PLAIN_BLK;
+    fsmall[h] = act && kept[h] <= RSG_PLAIN_BLK;
     if (act) {
-        int b = kept[h] > big ? 0 : 1;
+        int b = kept[h] > 1024 ? 0 : 1;
         atomicAdd(&work[b], (unsigned long long)kept[h]);
         atomicAdd(&work[2 + b], 1ull);
     }
@@ -2169,13 +2273,19 @@ void additional_props(Arena &ar, const DevCfg &dc, const DevCfg *d_dc, const Rec
     {
         int32_t *fs = ar.get<int32_t>(NH), *fbg = ar.get<int32_t>(NH);
         int32_t *ls = ar.get<int32_t>(NH), *lb = ar.get<int32_t>(NH);
-        launch(k_scan_split, nblk(NH, T), T, 0, st, H, NH, kept, 1024, fs, fbg, work);
+        launch(k_scan_split, nblk(NH, T), T, 0, st, H, NH, kept, fs, fbg, work);
         if (exact) {
             int32_t nsm = select_idx(ar, fs, ls, NH, st);
             int32_t nbg = select_idx(ar, fbg, lb, NH, st);
-            launch(k_halo_scans_blk, nbg, RSG_SB, 0, st, H, E, lb, PO2, toff, kept, d_dc, exact);
-            launch(k_halo_scans_list, nblk(nsm, 32), 32, 0, st, H, E, ls, nsm, PO2, toff, kept,
-                   d_dc);
+            launch(k_halo_scans_blk, nbg, RSG_SB, 0, st, H, E, lb, PO2, toff, kept, d_dc);
+            // A thread takes 7.5 ms for a small halo whatever their number, up
+            // to where the FP64 pipe fills; a block 0.8 ms, six to an SM: the
+            // blocks are faster up to some eight waves of them.
+            if (nsm <= RSG_PLAIN_FEW)
+                launch(k_halo_scans_blk, nsm, RSG_SB, 0, st, H, E, ls, PO2, toff, kept, d_dc);
+            else
+                launch(k_halo_scans_list, nblk(nsm, 32), 32, 0, st, H, E, ls, nsm, PO2, toff,
+                       kept, d_dc);
         } else {
             seg_props(ar, dc, d_dc, PO2, npo, H, E, NH, toff, kept, st);
         }

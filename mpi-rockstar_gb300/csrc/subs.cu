@@ -112,15 +112,21 @@ __device__ void norm_sigmas(const double *corr, int level0, double ims, double *
     sig[1] = sv;
 }
 
-// Nodes up to RSG_SEQ_MAX particles: one thread, array order, so every FP64
-// sum rounds as the reference's loop does.
+// Plain form, nodes up to RSG_NORM_SEQ particles: one thread, array order, so
+// every FP64 sum rounds as the reference's loop does.  Its 27 sums share one
+// lane (430 cycles a particle: an FP64 instruction holds the narrow pipe for
+// 16), against 64 cycles for the same sums on a lane each in k_norm_blk, so
+// it keeps only the nodes too small to give a block work; with nodes up to
+// 2,048 on it the normalisations of a 524,288-particle snapshot took 26 ms, now
+// 12 ms.
+#define RSG_NORM_SEQ 64
 __global__ void k_norm_seq(Rec *W, HierNodes N, int32_t base, int32_t count, int level0,
                            double ims, double *sig) {
     int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= count) return;
     int node = base + k;
     int s = N.start[node], n = N.n[node];
-    if (n <= 0 || n > RSG_SMALL) return;
+    if (n <= 0 || n > RSG_NORM_SEQ) return;
     double mean[6] = {0, 0, 0, 0, 0, 0};
     for (int i = 0; i < n; i++)
         for (int d = 0; d < 6; d++) mean[d] += (double)W[s + i].pos[d];
@@ -2567,11 +2573,11 @@ SubsOut find_subs_device(Arena &ar, rsg_particle *d_p, int64_t num_p, const int6
     // reference's quickselect runs on, whose early exit on equal end values
     // (mutual nearest neighbours) returns a value that depends on that
     // array's order (src/groupies.c:768-786).
-    // norm_sd sums in array order (bit-exact) for nodes in (seq_lo,
+    // norm_sd sums in array order (bit-exact) by blocks for nodes in (seq_lo,
     // RSG_SEQ_MAX] in the plain form; the batched form sums in parallel
     // (rounding can move a normalised coordinate by one float ulp, rarely:
     // the near-threshold count bounds what that can change)
-    const int seq_lo = exact ? RSG_SMALL : RSG_SEQ_MAX;
+    const int seq_lo = exact ? RSG_NORM_SEQ : RSG_SEQ_MAX;
     const int seq_max = RSG_SEQ_MAX;
     const int T = 256;
     // groups with particles, their working offsets
