@@ -177,14 +177,28 @@ __global__ void k_gadget_assemble(const unsigned char *pos, const unsigned char 
     out[i] = q;
 }
 
-// smallest and largest id (ordered atomics on the signed values)
-__global__ void k_id_range(const rsg_particle *p, int64_t n, long long *mm) {
+// One pass over the records (they take 0.21 ms for 16.8M; a pass for the range,
+// one for the keys and the copy back after the gather took 0.36): a copy of
+// them, the gather's source, so that it writes in place; the ids, and the smallest and
+// largest id (ordered atomics on the signed values).  Two threads share a
+// record, 16 bytes each, or four, 8 bytes each, where the caller's records
+// are aligned to no more than that (V).
+template <class V>
+__global__ void k_id_scan(const rsg_particle *p, int64_t n, rsg_particle *copy, long long *id,
+                          long long *mm) {
+    constexpr int P = sizeof(rsg_particle) / sizeof(V);
+    const V *src = reinterpret_cast<const V *>(p);
+    V *dst = reinterpret_cast<V *>(copy);
     long long lo = LLONG_MAX, hi = LLONG_MIN;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const long long v = (long long)p[i].id;
-        lo = v < lo ? v : lo;
-        hi = v > hi ? v : hi;
+    const int64_t step = (int64_t)gridDim.x * blockDim.x;  // of P: a thread keeps its part
+    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < P * n; t += step) {
+        const V v = src[t];
+        dst[t] = v;
+        if (t & (P - 1)) continue;
+        const long long w = (long long)(((unsigned long long)v.y << 32) | v.x);
+        id[t / P] = w;
+        lo = w < lo ? w : lo;
+        hi = w > hi ? w : hi;
     }
     for (int o = 16; o; o >>= 1) {
         const long long a = __shfl_down_sync(0xffffffffu, lo, o), b = __shfl_down_sync(0xffffffffu, hi, o);
@@ -198,17 +212,27 @@ __global__ void k_id_range(const rsg_particle *p, int64_t n, long long *mm) {
 }
 // keys id - min as unsigned (order-preserving for signed ids), values the
 // record index
-__global__ void k_id_keys(const rsg_particle *p, int64_t n, const long long *mm,
-                          unsigned long long *key, int32_t *idx) {
+template <class K>
+__global__ void k_id_keys(int64_t n, const long long *mm, const unsigned long long *id, K *key,
+                          int32_t *idx) {
     int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
-    key[i] = (unsigned long long)p[i].id - (unsigned long long)mm[0];
+    key[i] = (K)(id[i] - (unsigned long long)mm[0]);
     idx[i] = (int32_t)i;
 }
+// dst[i] = src[idx[i]], records read and written as V
+template <class V>
 __global__ void k_gather_p(const rsg_particle *src, const int32_t *idx, int64_t n,
                            rsg_particle *dst) {
-    int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i < n) dst[i] = src[idx[i]];
+    constexpr int P = sizeof(rsg_particle) / sizeof(V);
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const V *s = reinterpret_cast<const V *>(src + idx[i]);
+    V v[P];
+#pragma unroll
+    for (int q = 0; q < P; q++) v[q] = s[q];
+#pragma unroll
+    for (int q = 0; q < P; q++) reinterpret_cast<V *>(dst + i)[q] = v[q];
 }
 __global__ void k_mm_init(long long *mm) {
     mm[0] = LLONG_MAX;
@@ -357,10 +381,11 @@ int read_core(const char *path, const struct rsg_gadget_opts *opt, struct rsg_co
 void sort_device(rsg_particle *d_p, int64_t n, Arena &ar, cudaStream_t st) {
     rsg_particle *d_q = ar.get<rsg_particle>(n);
     unsigned long long *k1 = ar.get<unsigned long long>(n), *k2 = ar.get<unsigned long long>(n);
-    int32_t *v1 = ar.get<int32_t>(n), *v2 = ar.get<int32_t>(n);
     long long *mm = ar.get<long long>(2);
     launch(k_mm_init, 1, 1, 0, st, mm);
-    launch(k_id_range, 152 * 8, 256, 0, st, (const rsg_particle *)d_p, n, mm);
+    const bool wide = ((uintptr_t)d_p & 15) == 0;
+    launch(wide ? k_id_scan<uint4> : k_id_scan<uint2>, 152 * 8, 256, 0, st,
+           (const rsg_particle *)d_p, n, d_q, (long long *)k1, mm);
     RSG_CHECK_LAUNCH();
     long long h_mm[2];
     RSG_CUDA(cudaMemcpyAsync(h_mm, mm, sizeof h_mm, cudaMemcpyDeviceToHost, st));
@@ -368,17 +393,23 @@ void sort_device(rsg_particle *d_p, int64_t n, Arena &ar, cudaStream_t st) {
     if (h_mm[0] == h_mm[1]) return;  // one id: the order stays
     const unsigned long long range = (unsigned long long)h_mm[1] - (unsigned long long)h_mm[0];
     const int end_bit = 64 - __builtin_clzll(range);
-    launch(k_id_keys, nblk(n, 256), 256, 0, st, (const rsg_particle *)d_p, n,
-           (const long long *)mm, k1, v1);
+    // Ranges below 2^32 sort 4-byte keys, 8 bytes a record in each pass instead
+    // of 12, in the same order.  (One 8-byte word with the index below the key:
+    // 0.70 ms for 16.8M records, against 0.63.)
+    int32_t *v1 = ar.get<int32_t>(n), *v2 = ar.get<int32_t>(n);
     size_t tb = 0;
-    RSG_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb, k1, k2, v1, v2, (int)n, 0, end_bit, st));
-    void *tmp = ar.take(tb + 256);
-    RSG_CUDA(cub::DeviceRadixSort::SortPairs(tmp, tb, k1, k2, v1, v2, (int)n, 0, end_bit, st));
-    launch(k_gather_p, nblk(n, 256), 256, 0, st, (const rsg_particle *)d_p, (const int32_t *)v2,
-           n, d_q);
+    auto sorted = [&](auto *a, auto *b) {
+        launch(k_id_keys<std::remove_pointer_t<decltype(a)>>, nblk(n, 256), 256, 0, st, n,
+               (const long long *)mm, (const unsigned long long *)k1, a, v1);
+        RSG_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb, a, b, v1, v2, (int)n, 0, end_bit, st));
+        void *tmp = ar.take(tb + 256);
+        RSG_CUDA(cub::DeviceRadixSort::SortPairs(tmp, tb, a, b, v1, v2, (int)n, 0, end_bit, st));
+    };
+    if (end_bit <= 32) sorted((uint32_t *)k2, (uint32_t *)k2 + n);
+    else sorted(k1, k2);
+    launch(wide ? k_gather_p<uint4> : k_gather_p<uint2>, nblk(n, 256), 256, 0, st,
+           (const rsg_particle *)d_q, (const int32_t *)v2, n, d_p);
     RSG_CHECK_LAUNCH();
-    RSG_CUDA(cudaMemcpyAsync(d_p, d_q, sizeof(rsg_particle) * (size_t)n, cudaMemcpyDeviceToDevice,
-                             st));
     RSG_CUDA(cudaStreamSynchronize(st));
 }
 
