@@ -744,14 +744,24 @@ __device__ float total_energy(const PotRec *po, int64_t tot, float *ratio, const
     return (float)((ke - tphi) * C.particle_mass * RSG_GC / (double)sn);
 }
 
-// calc_shape (src/properties.c:216-326) for 32 halos per warp, in the
-// reference's summation order.  Each iteration runs the record phase of
+// calc_shape (src/properties.c:216-326) for `per` halos per warp (at most
+// 32), in the reference's summation order.  Each iteration runs the record phase of
 // every halo still iterating in turn -- the lanes compute the terms of 32
 // records at a time (ellipsoid radius, weight, products) and lane c < 7 adds
-// accumulator c over them in record order -- and then the 32 halos'
-// decisions (Jacobi, the 1% rule) side by side, one per lane: left to one
-// lane, that FP64 work occupied the narrow FP64 pipe for a single lane's
-// result.  `B` is this warp's state in shared memory.
+// accumulator c over them in record order -- and then the halos' decisions
+// (Jacobi, the 1% rule) side by side, one per lane: left to one lane, that
+// FP64 work (19,000 cycles of the narrow FP64 pipe) is spent for a single
+// lane's result, which matters where the pipe is full and not where most SMs
+// have no warp: `per` grows with the halos (shape_per).  `B` is this warp's
+// state in shared memory.
+// Halos per warp: the fewest that leave at most eight warps an SM (162 halos:
+// 2.5 ms with 32 to a warp, 0.85 with one; 6,059: 5.6 with 32, 3.5 with 4, 3.3
+// with 8).
+static int shape_per(int32_t nh) {
+    int per = 1;
+    while (per < 32 && nh / per > 8 * 152) per *= 2;
+    return per;
+}
 struct ShapeBatch {
     double v[32][7];
     double acc[32][7];
@@ -761,9 +771,17 @@ struct ShapeBatch {
     int set[32];  // records of halo base + q, -1 for a halo this warp skips
 };
 __device__ void shape_batch(rsg_halo *H, const int32_t *toff, const PotRec *PO, int32_t base,
-                            int32_t NH, int bound, const DevCfg &C, ShapeBatch &B) {
+                            int per, int32_t NH, int bound, const DevCfg &C, ShapeBatch &B) {
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
+    int64_t an = 0;  // analysed records of halo base + lane
+    for (int q = 0; q < per; q++) {
+        const int tot = B.set[q];
+        int c = 0;
+        for (int j = lane; j < tot; j += 32) c += !(bound && unbound(PO[toff[base + q] + j]));
+        c = __reduce_add_sync(FULL, c);
+        if (lane == q) an = c;
+    }
     {
         // lane q sets up halo base + q (the loop's prologue, src/properties.c:222-250)
         const int32_t hq = base + lane;
@@ -771,10 +789,6 @@ __device__ void shape_batch(rsg_halo *H, const int32_t *toff, const PotRec *PO, 
         float minr = 0.f;
         if (hq < NH && B.set[lane] >= 0) {
             rsg_halo &h = H[hq];
-            const PotRec *po = PO + toff[hq];
-            const int64_t tot = B.set[lane];
-            int64_t an = 0;
-            for (int64_t j = 0; j < tot; j++) an += !(bound && unbound(po[j]));
             int64_t it = C.shape_iterations;
             minr = fmul((float)C.force_res, (float)C.force_res);
             h.b_to_a = h.c_to_a = 0;
@@ -802,9 +816,9 @@ __device__ void shape_batch(rsg_halo *H, const int32_t *toff, const PotRec *PO, 
     }
     __syncwarp();
     int maxit = 0;
-    for (int q = 0; q < 32; q++) maxit = max(maxit, B.done[q] ? 0 : B.it[q]);
+    for (int q = 0; q < per; q++) maxit = max(maxit, B.done[q] ? 0 : B.it[q]);
     for (int i = 0; i < maxit; i++) {
-        for (int q = 0; q < 32; q++) {
+        for (int q = 0; q < per; q++) {
             if (B.done[q] || i >= B.it[q]) continue;
             const int32_t hq = base + q;
             const PotRec *po = PO + toff[hq];
@@ -2179,8 +2193,9 @@ static void seg_props(Arena &ar, const DevCfg &dc, const DevCfg *d_dc, PotRec *P
         phase_mark(st, "p.passes");
         for (int which = 0; which < 2; which++) {
             launch(k_sh_init, HB, HT, 0, st, NH, H, cnt, toff, d_dc, which, S);
-            launch(k_sh_small, nblk(NH, 128), 128, 0, st, NH, H, toff,
-                   (const PotRec *)PO, d_dc, (const HS *)S, bound);
+            const int per = shape_per(NH);
+            launch(k_sh_small, nblk(nblk(NH, per), 4), 128, 0, st, NH, H, toff,
+                   (const PotRec *)PO, d_dc, (const HS *)S, bound, per);
             for (int64_t i = 0; i < dc.shape_iterations; i++) {
                 launch(k_sh_sum, nc, RSG_CT, 0, st, CH, PO, H, flag, S, d_dc, cp);
                 launch(k_sh_fin, HB, HT, 0, st, NH, H, c0, nch, cp, S);

@@ -95,21 +95,23 @@ __device__ __forceinline__ int rand_r_glibc(unsigned *seed) {
 // norm_sd (src/groupies.c:788-830) + calc_deviations (src/jacobi.c:156-172).
 // Moments go to mom[node * 27]: 6 means then the 21 upper-triangular
 // second moments of the centred coordinates; sig[node * 2] gets sig_x, sig_v.
-__device__ void norm_sigmas(const double *corr, int level0, double ims, double *sig) {
-    double full[6][6];
-    int k = 0;
-    for (int a = 0; a < 6; a++)
-        for (int b = a; b < 6; b++) full[a][b] = full[b][a] = corr[k++];
+// corr: the 21 moments; half 0 gives sig_x, half 1 sig_v
+__device__ double norm_sigma(const double *corr, int half, int level0, double ims) {
+    // rows of the upper triangle start at 0, 6, 11, 15, 18, 20
+    const double *c = half ? corr + 15 : corr;
     double in[3][3];
-    for (int a = 0; a < 3; a++)
-        for (int b = 0; b < 3; b++) in[a][b] = full[a][b];
-    double sx = min_eig_sqrt(in);
-    for (int a = 0; a < 3; a++)
-        for (int b = 0; b < 3; b++) in[a][b] = full[a + 3][b + 3];
-    double sv = min_eig_sqrt(in);
-    if (level0) sx *= ims;  // n == num_copies holds for the group itself only
-    sig[0] = sx;
-    sig[1] = sv;
+    int k = 0;
+    for (int a = 0; a < 3; a++) {
+        for (int b = a; b < 3; b++) in[a][b] = in[b][a] = c[k++];
+        if (!half) k += 3;  // the products with the other half
+    }
+    double s = min_eig_sqrt(in);
+    if (!half && level0) s *= ims;  // n == num_copies holds for the group itself only
+    return s;
+}
+__device__ void norm_sigmas(const double *corr, int level0, double ims, double *sig) {
+    sig[0] = norm_sigma(corr, 0, level0, ims);
+    sig[1] = norm_sigma(corr, 1, level0, ims);
 }
 
 // Plain form, nodes up to RSG_NORM_SEQ particles: one thread, array order, so
@@ -155,8 +157,8 @@ __global__ void k_norm_seq(Rec *W, HierNodes N, int32_t base, int32_t count, int
 // the FP32 pipe (hi + lo, Knuth's two-sum: about 48 bits, enough for
 // RSG_SMALL terms); the lanes' sums are combined by shuffles (deterministic).
 // The sigmas (two 3x3 eigenvalue problems per node, a long FP64 chain) follow
-// one node per thread in k_norm_sig, so that neither part waits on the
-// other's shape: with 32 nodes in turn on one warp and their sigmas side by
+// in k_norm_sig, a thread for each, so that neither part waits on the other's
+// shape: with 32 nodes in turn on one warp and their sigmas side by
 // side behind them, a level of a 64^3 snapshot took 0.68 ms, two thirds of
 // the chip's SMs without a warp; now 0.1 ms.
 __global__ void __launch_bounds__(128) k_norm_mom(Rec *W, HierNodes N, int32_t base,
@@ -204,15 +206,14 @@ __global__ void __launch_bounds__(128) k_norm_mom(Rec *W, HierNodes N, int32_t b
         if (lane == jj) mom[(int64_t)jj * count + k] = ((double)ch[jj] + (double)cl[jj]) / (double)n;
     }
 }
-__global__ void k_norm_sig(HierNodes N, int32_t base, int32_t count, const double *mom,
-                           int level0, double ims, double *sig) {
-    const int32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void k_norm_sig(int32_t count, const double *mom, int level0, double ims,
+                           double *sig) {
+    const int32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int32_t k = t >> 1;
     if (k >= count) return;
-    const int n = N.n[base + k];
-    if (n <= 0 || n > RSG_SMALL) return;
     double c[21];
     for (int j = 0; j < 21; j++) c[j] = mom[(int64_t)j * count + k];
-    norm_sigmas(c, level0, ims, sig + 2 * k);
+    sig[t] = norm_sigma(c, t & 1, level0, ims);
 }
 
 // Mid-size nodes: the block stages particles in shared memory and computes
@@ -340,17 +341,15 @@ __global__ void __launch_bounds__(256) k_nch_mom(Rec *W, const NChunk *C, const 
         if (threadIdx.x == 0) P[blockIdx.x].d[j] = t;
     }
 }
+// The moments of the chunked nodes, a warp each: lane j adds second moment j
+// over the chunks in order.
 __global__ void k_nch_fin(HierNodes N, int32_t base, int32_t cnt, const int32_t *nch,
-                          const int32_t *c0, const NPart *P, int level0, double ims,
-                          double *sig) {
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= cnt || nch[k] == 0) return;
-    double cc[21];
-    for (int j = 0; j < 21; j++) cc[j] = 0;
-    for (int c = c0[k]; c < c0[k] + nch[k]; c++)
-        for (int j = 0; j < 21; j++) cc[j] += P[c].d[j];
-    for (int j = 0; j < 21; j++) cc[j] /= (double)N.n[base + k];
-    norm_sigmas(cc, level0, ims, sig + 2 * k);
+                          const int32_t *c0, const NPart *P, double *mom) {
+    const int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, j = threadIdx.x & 31;
+    if (k >= cnt || nch[k] == 0 || j >= 21) return;
+    double cc = 0;
+    for (int c = c0[k]; c < c0[k] + nch[k]; c++) cc += P[c].d[j];
+    mom[(int64_t)j * cnt + k] = cc / (double)N.n[base + k];
 }
 
 // Larger nodes: one block, deterministic tree reductions.
@@ -2653,21 +2652,13 @@ SubsOut find_subs_device(Arena &ar, rsg_particle *d_p, int64_t num_p, const int6
         RSG_CUDA(cudaMemsetAsync(eln, 0xff, 4 * M, st));
         launch(k_fill_eln, cnt, T, 0, st, N, base, eln);
         {
+            const size_t m0 = ar.used;
             double *sig = ar.get<double>(2 * (int64_t)cnt);
             if (exact) {
                 launch(k_norm_seq, nblk(cnt, 32), 32, 0, st, W, N, base, cnt, L == 0,
                        cfg.initial_metric_scaling, sig);
-            } else {
-                size_t m0 = ar.used;
-                double *mom = ar.get<double>(21 * (int64_t)cnt);
-                launch(k_norm_mom, nblk((int64_t)cnt * 32, 128), 128, 0, st, W, N, base, cnt, mom);
-                launch(k_norm_sig, nblk(cnt, 32), 32, 0, st, N, base, cnt, (const double *)mom,
-                       L == 0, cfg.initial_metric_scaling, sig);
-                ar.used = m0;
-            }
-            launch(k_norm_blk, cnt, 256, 0, st, W, N, base, L == 0, cfg.initial_metric_scaling, sig,
-                   seq_lo, RSG_SEQ_MAX);
-            if (exact) {
+                launch(k_norm_blk, cnt, 256, 0, st, W, N, base, L == 0,
+                       cfg.initial_metric_scaling, sig, seq_lo, RSG_SEQ_MAX);
                 launch(k_norm_par, cnt, T, 0, st, W, N, base, L == 0, cfg.initial_metric_scaling,
                        sig, seq_max);
             } else {
@@ -2675,6 +2666,9 @@ SubsOut find_subs_device(Arena &ar, rsg_particle *d_p, int64_t num_p, const int6
                 launch(k_nch_count, nblk(cnt + 1, T), T, 0, st, N, base, cnt, tuning().norm_chunk,
                        seq_lo, RSG_SEQ_MAX, nch);
                 int32_t nc = excl_scan(ar, (const int32_t *)nch, c0, cnt + 1, st);
+                // the moments of every node, then their sigmas
+                double *mom = ar.get<double>(21 * (int64_t)cnt);
+                launch(k_norm_mom, nblk((int64_t)cnt * 32, 128), 128, 0, st, W, N, base, cnt, mom);
                 if (nc > 0) {
                     NChunk *C = ar.get<NChunk>(nc);
                     NPart *P = ar.get<NPart>(nc);
@@ -2685,14 +2679,16 @@ SubsOut find_subs_device(Arena &ar, rsg_particle *d_p, int64_t num_p, const int6
                     launch(k_nch_mean, nblk(cnt, T), T, 0, st, N, base, cnt, (const int32_t *)nch,
                            (const int32_t *)c0, (const NPart *)P, mean);
                     launch(k_nch_mom, nc, 256, 0, st, W, (const NChunk *)C, (const double *)mean, P);
-                    launch(k_nch_fin, nblk(cnt, T), T, 0, st, N, base, cnt, (const int32_t *)nch,
-                           (const int32_t *)c0, (const NPart *)P, L == 0,
-                           cfg.initial_metric_scaling, sig);
+                    launch(k_nch_fin, nblk((int64_t)cnt * 32, T), T, 0, st, N, base, cnt,
+                           (const int32_t *)nch, (const int32_t *)c0, (const NPart *)P, mom);
                 }
+                launch(k_norm_sig, nblk(2 * (int64_t)cnt, 32), 32, 0, st, cnt,
+                       (const double *)mom, L == 0, cfg.initial_metric_scaling, sig);
             }
             launch(k_norm_div_el, nblk(M, T), T, 0, st, W, M, (const int32_t *)eln,
                    (const double *)sig);
             RSG_CHECK_LAUNCH();
+            ar.used = m0;
         }
         phase_mark(st, "d.norm_sd");
         int32_t *rst = N.start + base, *rn = N.n + base;
