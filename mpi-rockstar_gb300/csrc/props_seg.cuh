@@ -135,14 +135,38 @@ __global__ void __launch_bounds__(RSG_CT) k_sg_cnt_chunk(const Chunk *CH, const 
     if (threadIdx.x == 0) cp[blockIdx.x].i[0] = s;
 }
 // exclusive prefix over each halo's chunks, in chunk order
+// The passes over a halo's chunks run one thread per halo; a halo of more
+// than RSG_FEW_CHUNKS (600 for the 1.3M records of a quarter of the 512^3
+// volume's largest) is its warp's together, an accumulator to a lane in chunk
+// order, so that its loads do not follow one another.
+#define RSG_FEW_CHUNKS 8
 __global__ void k_sg_cnt_off(int32_t NH, const int32_t *c0, const int32_t *nch, CP *cp) {
-    int h = blockIdx.x * blockDim.x + threadIdx.x;
-    if (h >= NH) return;
-    long long run = 0;
-    for (int c = c0[h]; c < c0[h] + nch[h]; c++) {
-        long long t = cp[c].i[0];
-        cp[c].i[0] = run;
-        run += t;
+    const unsigned FULL = 0xffffffffu;
+    const int h = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+    const int f = h < NH ? c0[h] : 0, n = h < NH ? nch[h] : 0;
+    if (n <= RSG_FEW_CHUNKS) {
+        long long run = 0;
+        for (int c = f; c < f + n; c++) {
+            long long t = cp[c].i[0];
+            cp[c].i[0] = run;
+            run += t;
+        }
+    }
+    for (unsigned todo = __ballot_sync(FULL, n > RSG_FEW_CHUNKS); todo; todo &= todo - 1) {
+        const int b = __ffs(todo) - 1;
+        const int bf = __shfl_sync(FULL, f, b), bn = __shfl_sync(FULL, n, b);
+        long long run = 0;
+        for (int b0 = 0; b0 < bn; b0 += 32) {
+            const bool on = b0 + lane < bn;
+            const long long t = on ? cp[bf + b0 + lane].i[0] : 0;
+            long long inc = t;
+            for (int o = 1; o < 32; o <<= 1) {
+                const long long v = __shfl_up_sync(FULL, inc, o);
+                if (lane >= o) inc += v;
+            }
+            if (on) cp[bf + b0 + lane].i[0] = run + inc - t;
+            run += __shfl_sync(FULL, inc, 31);
+        }
     }
 }
 __global__ void __launch_bounds__(RSG_CT) k_sg_cnt_scan(const Chunk *CH, const uint8_t *flag,
@@ -233,15 +257,36 @@ __global__ void __launch_bounds__(RSG_CT) k_cv_sums(const Chunk *CH, const PotRe
 }
 __global__ void k_cv_off(int32_t NH, const rsg_halo *H, const int32_t *c0, const int32_t *nch,
                          const HS *S, CP *cp) {
-    int h = blockIdx.x * blockDim.x + threadIdx.x;
-    if (h >= NH || H[h].num_p < 1 || S[h].rmax < 1) return;
-    double run[6] = {0, 0, 0, 0, 0, 0};
-    for (int c = c0[h]; c < c0[h] + nch[h]; c++)
-        for (int d = 0; d < 6; d++) {
-            double t = cp[c].d[d];
-            cp[c].d[d] = run[d];
-            run[d] += t;
+    const unsigned FULL = 0xffffffffu;
+    const int h = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+    const bool act = h < NH && H[h].num_p >= 1 && S[h].rmax >= 1;
+    const int f = act ? c0[h] : 0, n = act ? nch[h] : 0;
+    if (n <= RSG_FEW_CHUNKS) {
+        double run[6] = {0, 0, 0, 0, 0, 0};
+        for (int c = f; c < f + n; c++)
+            for (int d = 0; d < 6; d++) {
+                double t = cp[c].d[d];
+                cp[c].d[d] = run[d];
+                run[d] += t;
+            }
+    }
+    for (unsigned todo = __ballot_sync(FULL, n > RSG_FEW_CHUNKS); todo; todo &= todo - 1) {
+        const int b = __ffs(todo) - 1;
+        const int bf = __shfl_sync(FULL, f, b), bn = __shfl_sync(FULL, n, b);
+        if (lane >= 6) continue;
+        double run = 0;
+        for (int b0 = 0; b0 < bn; b0 += 8) {
+            double t[8];
+#pragma unroll
+            for (int u = 0; u < 8; u++) t[u] = b0 + u < bn ? cp[bf + b0 + u].d[lane] : 0.0;
+#pragma unroll
+            for (int u = 0; u < 8; u++)
+                if (b0 + u < bn) {
+                    cp[bf + b0 + u].d[lane] = run;
+                    run += t[u];
+                }
         }
+    }
 }
 // running mean and variance at every i < rmax from prefix sums, the test
 // value g_i = tv_i / ((i-3) i) (0 for i <= 3), and per chunk the first
@@ -738,14 +783,30 @@ __global__ void __launch_bounds__(RSG_CT) k_sh_sum(const Chunk *CH, const PotRec
 }
 __global__ void k_sh_fin(int32_t NH, rsg_halo *H, const int32_t *c0, const int32_t *nch,
                          const CP *cp, HS *S) {
-    int h = blockIdx.x * blockDim.x + threadIdx.x;
-    if (h >= NH || H[h].num_p < 1) return;
-    HS &s = S[h];
-    if (s.done) return;
-    rsg_halo &hh = H[h];
+    const unsigned FULL = 0xffffffffu;
+    const int h = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+    const bool act = h < NH && H[h].num_p >= 1 && !S[h].done;
+    const int f = act ? c0[h] : 0, n = act ? nch[h] : 0;
     double acc[7] = {0, 0, 0, 0, 0, 0, 0};
-    for (int c = c0[h]; c < c0[h] + nch[h]; c++)
-        for (int d = 0; d < 7; d++) acc[d] += cp[c].d[d];
+    if (n <= RSG_FEW_CHUNKS)
+        for (int c = f; c < f + n; c++)
+            for (int d = 0; d < 7; d++) acc[d] += cp[c].d[d];
+    for (unsigned todo = __ballot_sync(FULL, n > RSG_FEW_CHUNKS); todo; todo &= todo - 1) {
+        const int b = __ffs(todo) - 1;
+        const int bf = __shfl_sync(FULL, f, b), bn = __shfl_sync(FULL, n, b);
+        double a = 0;
+        if (lane < 7) {
+#pragma unroll 8
+            for (int c = 0; c < bn; c++) a += cp[bf + c].d[lane];
+        }
+        for (int d = 0; d < 7; d++) {
+            const double v = __shfl_sync(FULL, a, d);
+            if (lane == b) acc[d] = v;
+        }
+    }
+    if (!act) return;
+    HS &s = S[h];
+    rsg_halo &hh = H[h];
     double w = acc[0];
     if (!w) {
         s.done = 1;

@@ -170,14 +170,20 @@ __global__ void __launch_bounds__(RSG_UF_WARPS * 32)
     if (t >= nr) return;
     const int e0 = rs[t], e1 = (t + 1 < nr) ? rs[t + 1] : ne;
     if (e1 - e0 <= RSG_UF_WARP) return;
+    // the next batch's sets are read while this one's chain runs
+    int c = e0 + lane < e1 ? eid[e0 + lane] : -1;
+    int lw = c >= 0 ? cW[c] : -1, lf = c >= 0 ? cF[c] : -1;
+    c = e0 + 32 + lane < e1 ? eid[e0 + 32 + lane] : -1;
     for (int b = e0; b < e1; b += 32) {
         const int i = b + lane;
         int rl = -1, rc = -1;
         if (i < e1) {
-            const int c = eid[i];
-            rl = rt_find(R, cW[c]);
-            rc = rt_find(R, cF[c]);
+            rl = rt_find(R, lw);
+            rc = rt_find(R, lf);
         }
+        lw = c >= 0 ? cW[c] : -1;
+        lf = c >= 0 ? cF[c] : -1;
+        c = b + 64 + lane < e1 ? eid[b + 64 + lane] : -1;
         __syncwarp();
 #pragma unroll
         for (int q = 0; q < 31; q++) {
