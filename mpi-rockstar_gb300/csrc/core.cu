@@ -59,41 +59,44 @@ Arena::~Arena() {
     if (base) cudaFree(base);
 }
 
-__global__ void k_slot_set(const int32_t *act, const LevelState *ls, int32_t *slot) {
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < ls->nact) slot[act[k]] = k;
-}
-__global__ void k_iota_i32(int32_t *a, int32_t n) {
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < n) a[k] = k;
-}
-// After k_children: the level's new nodes become [base, base + nnew), and
-// those that split again are the next level's active nodes.
-__global__ void k_level_advance(LevelState *ls, const int64_t *off) {
-    if (threadIdx.x || blockIdx.x) return;
-    const int64_t t = off[ls->nact];
-    ls->base = ls->nnodes;
-    ls->nnew = ls->err ? 0 : 2 * (int32_t)(t >> 32);
-    ls->nnodes += ls->nnew;
-    ls->nact = ls->err ? 0 : (int32_t)(t & 0xffffffffu);
-}
-
-__global__ void k_root_owner(const int32_t *rstart, const int32_t *rn, int32_t ntrees, int sub,
-                             int32_t *owner, int32_t *box_owner) {
-    int t = blockIdx.x;  // tree; blockIdx.y strides through its elements
-    if (t >= ntrees) return;
-    int s = rstart[t], n = rn[t];
-    if (n <= sub) return;  // the whole tree is one block's (k_sub_build)
-    for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < n; i += gridDim.y * blockDim.x) {
-        box_owner[s + i] = t;
-        owner[s + i] = t;
+__global__ void k_rank_scan(int32_t *tpre, int32_t nt) {
+    __shared__ int32_t wsum[32];
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5, T = blockDim.x;
+    const int per = (nt + T - 1) / T;
+    const int a = min(t * per, nt), b = min(a + per, nt);
+    int sum = 0;
+    for (int i = a; i < b; i++) sum += tpre[i];
+    int incl = sum;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
     }
+    if (lane == 31) wsum[w] = incl;
+    __syncthreads();
+    if (w == 0) {
+        int v = lane < T / 32 ? wsum[lane] : 0;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, v, o);
+            if (lane >= o) v += u;
+        }
+        if (lane < T / 32) wsum[lane] = v;
+    }
+    __syncthreads();
+    int run = (w ? wsum[w - 1] : 0) + incl - sum;
+    for (int i = a; i < b; i++) {
+        const int v = tpre[i];
+        tpre[i] = run;
+        run += v;
+    }
+    if (t == T - 1) tpre[nt] = run;
 }
-// Whole trees of at most `sub` records go to the block-built subtrees.
-__global__ void k_root_subs(const int32_t *rn, int32_t ntrees, int sub, int sub0, SubRoot *subs,
-                            int32_t nsubs, LevelState *ls) {
-    int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < ntrees && rn[t] <= sub) list_sub(subs, nsubs, ls, sub0, t, rn[t], 0);
+__global__ void k_root_owner(const int32_t *rstart, const int32_t *rn, int32_t ntrees,
+                             const int32_t *slot, int32_t *owner) {
+    int t = blockIdx.x;  // tree; blockIdx.y strides through its elements
+    if (t >= ntrees || slot[t] < 0) return;
+    int s = rstart[t], n = rn[t], k = slot[t];
+    for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < n; i += gridDim.y * blockDim.x)
+        owner[s + i] = k;
 }
 
 // ---- phase timers ----------------------------------------------------------

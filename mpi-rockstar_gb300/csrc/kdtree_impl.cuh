@@ -31,98 +31,7 @@ inline void check_i32_total(Arena &ar, const int32_t *in, int64_t n, const char 
     }
 }
 
-// Box accumulation with per-thread runs: each thread walks ITEMS consecutive
-// elements, keeps a running min/max while the owner stays the same and
-// flushes with ordered atomics when it changes, so a node spanning millions
-// of elements receives one atomic per run rather than one per element.
-template <int D, class RecT, int ITEMS>
-__global__ void k_box_runs(const RecT *recs, int64_t nrec, const int32_t *owner,
-                           unsigned *bmin, unsigned *bmax) {
-    int64_t i0 = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) * ITEMS;
-    int cur = -1;
-    unsigned lo[D], hi[D];
-    for (int it = 0; it < ITEMS; it++) {
-        int64_t i = i0 + it;
-        if (i >= nrec) break;
-        int a = owner[i];
-        if (a != cur) {
-            if (cur >= 0)
-                for (int d = 0; d < D; d++) {
-                    atomicMin(&bmin[(int64_t)cur * D + d], lo[d]);
-                    atomicMax(&bmax[(int64_t)cur * D + d], hi[d]);
-                }
-            cur = a;
-            for (int d = 0; d < D; d++) {
-                lo[d] = 0xffffffffu;
-                hi[d] = 0u;
-            }
-        }
-        if (a < 0) continue;
-        const RecT r = recs[i];
-        for (int d = 0; d < D; d++) {
-            unsigned o = f2ord(PosOf<RecT, D>::get(r, d));
-            lo[d] = min(lo[d], o);
-            hi[d] = max(hi[d], o);
-        }
-    }
-    // last run: a warp whose lanes all hold the same node (the top levels of
-    // a build) combines it first and issues one atomic per dimension
-    const unsigned FULL = 0xffffffffu;
-    if (__match_any_sync(FULL, cur) == FULL) {
-        if (cur >= 0)
-            for (int d = 0; d < D; d++) {
-                unsigned a = __reduce_min_sync(FULL, lo[d]), b = __reduce_max_sync(FULL, hi[d]);
-                if ((threadIdx.x & 31) == 0) {
-                    atomicMin(&bmin[(int64_t)cur * D + d], a);
-                    atomicMax(&bmax[(int64_t)cur * D + d], b);
-                }
-            }
-    } else if (cur >= 0) {
-        for (int d = 0; d < D; d++) {
-            atomicMin(&bmin[(int64_t)cur * D + d], lo[d]);
-            atomicMax(&bmax[(int64_t)cur * D + d], hi[d]);
-        }
-    }
-}
-
-template <int D>
-__global__ void k_box_final_range(KNode<D> *nodes, int32_t first, int32_t count,
-                                  const unsigned *bmin, const unsigned *bmax) {
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= count) return;
-    int a = first + k;
-    for (int d = 0; d < D; d++) {
-        nodes[a].mn[d] = ord2f(bmin[(int64_t)a * D + d]);
-        nodes[a].mx[d] = ord2f(bmax[(int64_t)a * D + d]);
-    }
-}
-
-// The same for the last level's new nodes [ls->base, + ls->nnew), grid over ub.
-template <int D>
-__global__ void k_box_final_lvl(KNode<D> *nodes, const LevelState *ls, int32_t ub,
-                                const unsigned *bmin, const unsigned *bmax) {
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= ub || k >= ls->nnew) return;
-    int a = ls->base + k;
-    for (int d = 0; d < D; d++) {
-        nodes[a].mn[d] = ord2f(bmin[(int64_t)a * D + d]);
-        nodes[a].mx[d] = ord2f(bmax[(int64_t)a * D + d]);
-    }
-}
-__global__ void k_iota_i32(int32_t *a, int32_t n);
 #define RSG_FOREST_BATCH 4  // levels between reads of the build state
-
-__global__ void k_root_owner(const int32_t *rstart, const int32_t *rn, int32_t ntrees,
-                             int sub, int32_t *owner, int32_t *box_owner);
-__global__ void k_root_subs(const int32_t *rn, int32_t ntrees, int sub, int sub0, SubRoot *subs,
-                            int32_t nsubs, LevelState *ls);
-
-template <int D>
-__global__ void k_root_active(const KNode<D> *nodes, int32_t ntrees, int sub, int32_t *flag) {
-    int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= ntrees) return;
-    flag[t] = nodes[t].n > sub ? 1 : 0;
-}
 
 // One block's storage for a subtree of at most S records, of which at most
 // NA nodes split on one level (each holds more than `leaf` records).
@@ -193,13 +102,14 @@ __device__ __forceinline__ void sub_box(unsigned (*cbox)[2][2 * D], const float 
 // Children are numbered in the order the blocks allocate them: a node's two
 // children stay neighbours, and nothing depends on any other order.
 template <int D, class RecT, int S, int T, int NA>
-__global__ void __launch_bounds__(T) k_sub_build(RecT *recs, const SubRoot *roots,
-                                                 KNode<D> *nodes, LevelState *ls, int32_t cap,
-                                                 int leaf) {
+__global__ void __launch_bounds__(T) k_sub_build(RecT *out, const RecT *scratch,
+                                                 const SubRoot *roots, KNode<D> *nodes,
+                                                 LevelState *ls, int32_t cap, int leaf) {
     extern __shared__ __align__(16) unsigned char sub_sm[];
     SubShared<D, S, NA> &h = *reinterpret_cast<SubShared<D, S, NA> *>(sub_sm);
     const int t = threadIdx.x, lane = t & 31;
     const SubRoot root = roots[blockIdx.x];
+    const RecT *recs = root.src ? scratch : out;
     const int gs = nodes[root.node].start, n = nodes[root.node].n;
     const int tree = nodes[root.node].tree;
     const int nw = (n + 31) >> 5;
@@ -237,7 +147,6 @@ __global__ void __launch_bounds__(T) k_sub_build(RecT *recs, const SubRoot *root
         h.box[0][0][D + t] = hi;
     }
     int cur = 0, level = root.level;
-    if (n <= leaf) return;
     auto rank = [&](int x) {
         return h.wpre[x >> 5] + __popc(h.bits[x >> 5] & ((1u << (x & 31)) - 1u));
     };
@@ -432,35 +341,38 @@ __global__ void __launch_bounds__(T) k_sub_build(RecT *recs, const SubRoot *root
         }
         cur ^= 1;
     }
+    if (n <= leaf && !root.src) return;  // a leaf in its place
     // the records, 16 bytes of each at a time: read by every thread before any
-    // is written over
+    // is written over (the subtree may lie in `out` already)
     constexpr int V = sizeof(RecT) / 16, PER = S / T;
     static_assert(sizeof(RecT) % 16 == 0 && S % T == 0, "record vectors");
-    uint4 *rv = reinterpret_cast<uint4 *>(recs + gs);
+    const uint4 *sv = reinterpret_cast<const uint4 *>(recs + gs);
+    uint4 *dv = reinterpret_cast<uint4 *>(out + gs);
 #pragma unroll 1
     for (int v = 0; v < V; v++) {
         uint4 r[PER];
 #pragma unroll
         for (int u = 0; u < PER; u++) {
             const int i = t + u * T;
-            if (i < n) r[u] = rv[(int)h.idx[cur][i] * V + v];
+            if (i < n) r[u] = sv[(int)h.idx[cur][i] * V + v];
         }
         __syncthreads();
 #pragma unroll
         for (int u = 0; u < PER; u++) {
             const int i = t + u * T;
-            if (i < n) rv[i * V + v] = r[u];
+            if (i < n) dv[i * V + v] = r[u];
         }
     }
 }
 template <int D, class RecT, int S, int T, int NA>
-void launch_sub_build(int32_t count, RecT *recs, const SubRoot *roots, KNode<D> *nodes,
-                      LevelState *ls, int32_t cap, int leaf, cudaStream_t st) {
+void launch_sub_build(int32_t count, RecT *recs, const RecT *scratch, const SubRoot *roots,
+                      KNode<D> *nodes, LevelState *ls, int32_t cap, int leaf, cudaStream_t st) {
     if (count == 0) return;
     const size_t sm = sizeof(SubShared<D, S, NA>);
     RSG_CUDA(cudaFuncSetAttribute(k_sub_build<D, RecT, S, T, NA>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    launch(k_sub_build<D, RecT, S, T, NA>, count, T, sm, st, recs, roots, nodes, ls, cap, leaf);
+    launch(k_sub_build<D, RecT, S, T, NA>, count, T, sm, st, recs, scratch, roots, nodes, ls,
+           cap, leaf);
 }
 
 template <int D, class RecT>
@@ -479,119 +391,98 @@ Forest<D> build_forest(Arena &ar, RecT *recs, int64_t nrec, const int32_t *rstar
     const int sub0 = (int)std::min<int64_t>(S0, (int64_t)NA0 * (leaf + 1));
     const int sub = (int)std::min<int64_t>(S1, (int64_t)NA1 * (leaf + 1));
     const int64_t acap = n_in_trees / (sub + 1) + 1;  // nodes of more than `sub` records
-    const int32_t nsubs = (int32_t)(ntrees + n_in_trees / (leaf + 1) + 1);
+    const int32_t nsubs = (int32_t)cap;  // a node is listed once at most
     KNode<D> *nodes = ar.get<KNode<D>>(cap);
     const size_t mark = ar.used;  // everything below is released on return
     SubRoot *subs = ar.get<SubRoot>(nsubs);
     LevelState *ls = ar.get<LevelState>(1);
-    unsigned *bmin = ar.get<unsigned>(cap * D), *bmax = ar.get<unsigned>(cap * D);
-    int32_t *owner = ar.get<int32_t>(nrec), *box_owner = ar.get<int32_t>(nrec);
-    RecT *tmp = ar.get<RecT>(nrec);
-    int32_t *flag = ar.get<int32_t>(nrec + 1), *rank = ar.get<int32_t>(nrec + 1);
-    int32_t *fb = ar.get<int32_t>(nrec), *bs = ar.get<int32_t>(nrec);
-    int32_t *act = ar.get<int32_t>(acap), *act2 = ar.get<int32_t>(acap);
-    int32_t *slot = ar.get<int32_t>(cap);
-    float *lim = ar.get<float>(acap);
-    int32_t *m_arr = ar.get<int32_t>(acap), *q_arr = ar.get<int32_t>(acap);
-    int64_t *sflag = ar.get<int64_t>(acap + 1), *soff = ar.get<int64_t>(acap + 1);
-    int32_t *nflag = ar.get<int32_t>(ntrees), *ids = ar.get<int32_t>(ntrees);
-    size_t cub_bytes = 0, b2 = 0;
-    cub::DeviceScan::ExclusiveSum(nullptr, cub_bytes, flag, rank, (int)(nrec + 1), st);
-    cub::DeviceScan::ExclusiveSum(nullptr, b2, sflag, soff, (int)(acap + 1), st);
-    cub_bytes = cub_bytes > b2 ? cub_bytes : b2;
-    cub::DeviceSelect::Flagged(nullptr, b2, ids, nflag, act, &ls->nact, (int)ntrees, st);
-    cub_bytes = cub_bytes > b2 ? cub_bytes : b2;
-    void *cub_tmp = ar.take(cub_bytes + 256);
-
-    {
-        LevelState h0 = {};
-        h0.nnodes = ntrees;
-        RSG_CUDA(cudaMemcpyAsync(ls, &h0, sizeof(h0), cudaMemcpyHostToDevice, st));
+    int32_t *slot = ar.get<int32_t>(ntrees);
+    ActNode *act[2];
+    unsigned *cbox[2];
+    for (int b = 0; b < 2; b++) {
+        act[b] = ar.get<ActNode>(acap);
+        cbox[b] = ar.get<unsigned>(acap * 4 * D);
     }
-    launch(k_root_init<D, RecT>, nblk(ntrees, T), T, 0, st, rstart, rn, ntrees, nodes, bmin, bmax);
-    launch(k_root_active<D>, nblk(ntrees, T), T, 0, st, nodes, ntrees, sub, nflag);
-    launch(k_iota_i32, nblk(ntrees, T), T, 0, st, ids, ntrees);
-    cub::DeviceSelect::Flagged(cub_tmp, cub_bytes, ids, nflag, act, &ls->nact, ntrees, st);
-    launch(k_root_subs, nblk(ntrees, T), T, 0, st, rn, ntrees, sub, sub0, subs, nsubs, ls);
+    RSG_CUDA(cudaMemsetAsync(ls, 0, sizeof(LevelState), st));
+    RSG_CUDA(cudaMemcpyAsync(&ls->nnodes, &ntrees, sizeof(ntrees), cudaMemcpyHostToDevice, st));
+    launch(k_roots<D>, nblk(ntrees, T), T, 0, st, rstart, rn, ntrees, sub, sub0, nodes, act[0],
+           cbox[0], slot, subs, nsubs, ls);
     RSG_CHECK_LAUNCH();
-    LevelState hs;
+    struct Head {  // the fields of LevelState before nact[]
+        int32_t nnodes, err, nsub[2], ncopy, pad[3];
+    } hs;
+    static_assert(offsetof(LevelState, nact) == sizeof(Head), "LevelState layout");
+    int32_t nact = 0;
+    RSG_CUDA(cudaMemcpyAsync(&nact, &ls->nact[0], sizeof(nact), cudaMemcpyDeviceToHost, st));
     RSG_CUDA(cudaMemcpyAsync(&hs, ls, sizeof(hs), cudaMemcpyDeviceToHost, st));
     RSG_CUDA(cudaStreamSynchronize(st));
-    const int IT = 8;
-    if (hs.nact > 0) {
+    RecT *buf[2] = {recs, nullptr};  // levels scatter back and forth between these
+    if (nact > 0) {
+        buf[1] = ar.get<RecT>(nrec);
+        int32_t *owner = ar.get<int32_t>(nrec);
+        int32_t *fb = ar.get<int32_t>(nrec), *bs = ar.get<int32_t>(nrec);
+        int2 *copies = ar.get<int2>(acap);
+        const RankBits R = rank_alloc(ar, nrec, st);
+        const bool wide = sub >= RSG_STRETCH;
+        const int32_t nt = (int32_t)rank_tiles(nrec);
         RSG_CUDA(cudaMemsetAsync(owner, 0xff, sizeof(int32_t) * nrec, st));
-        RSG_CUDA(cudaMemsetAsync(box_owner, 0xff, sizeof(int32_t) * nrec, st));
         int64_t avg = n_in_trees / ntrees, y = avg / 2048;
         dim3 g((unsigned)ntrees, (unsigned)(y < 1 ? 1 : (y > 4096 ? 4096 : y)));
-        launch(k_root_owner, g, 256, 0, st, rstart, rn, ntrees, sub, owner, box_owner);
-        launch(k_box_runs<D, RecT, IT>, nblk((nrec + IT - 1) / IT, T), T, 0, st, recs, nrec,
-               box_owner, bmin, bmax);
-        launch(k_box_final_range<D>, nblk(ntrees, T), T, 0, st, nodes, 0, ntrees, bmin, bmax);
+        launch(k_root_owner, g, 256, 0, st, rstart, rn, ntrees, (const int32_t *)slot, owner);
+        launch(k_lv_flags<D, RecT>, nt, 256, 0, st, (const RecT *)recs, nrec,
+               (const int32_t *)owner, (const ActNode *)act[0], cbox[0], R, wide);
+        launch(k_root_split<D>, nblk(nact, T), T, 0, st, nodes, act[0], cbox[0],
+               (const LevelState *)ls);
         RSG_CHECK_LAUNCH();
-    }
-    // Levels of the nodes above `sub` records run back to back with their
-    // counts on the device; the host reads the state every RSG_FOREST_BATCH
-    // levels.  Grids are sized by an upper bound of the active count (ub): at
-    // most twice the previous level's, and at most one per sub + 1 records.
-    // A level past the last costs passes over nrec records, so large calls
-    // read after every level.
-    const int batch = nrec > (1 << 22) ? 1 : RSG_FOREST_BATCH;
-    int64_t ub = hs.nact;
-    int level = 0;
-    RecT *buf[2] = {recs, tmp};  // levels scatter back and forth between these
-    int cur = 0;
-    while (hs.nact > 0) {
-        for (int b = 0; b < batch && ub > 0; b++) {
-            if (++level > RSG_FOREST_LEVELS) {
-                set_error(RSG_ERR_LIMIT, "kd-forest build exceeded %d levels", RSG_FOREST_LEVELS);
-                throw Failure();
+        // Levels of the nodes above `sub` records run back to back with their
+        // counts on the device; the host reads them every RSG_FOREST_BATCH
+        // levels (every one in large calls: a level past the last costs passes
+        // over nrec records).  Grids are sized by an upper bound of the nodes
+        // (ub): at most twice the previous level's, and one per sub + 1 records.
+        const int batch = nrec > (1 << 22) ? 1 : RSG_FOREST_BATCH;
+        int64_t ub = nact;
+        int level = 0, cur = 0;
+        while (nact > 0) {
+            for (int b = 0; b < batch; b++) {
+                if (++level > RSG_FOREST_LEVELS) {
+                    set_error(RSG_ERR_LIMIT, "kd-forest build exceeded %d levels", RSG_FOREST_LEVELS);
+                    throw Failure();
+                }
+                const int x = (level - 1) & 1;
+                launch(k_lv_flags<D, RecT>, nt, 256, 0, st, (const RecT *)buf[cur], nrec,
+                       (const int32_t *)owner, (const ActNode *)act[x], cbox[x], R, wide);
+                launch(k_rank_scan, 1, 1024, 0, st, R.tpre, nt);
+                launch(k_lv_nodes<D>, nblk(ub, 64), 64, 0, st, nodes, act[x], act[1 - x],
+                       (const unsigned *)cbox[x], cbox[1 - x], ls, R, level, (int32_t)cap, leaf,
+                       sub, sub0, 1 - cur, subs, nsubs, copies);
+                launch(k_lv_tables, nt, 256, 0, st, nrec, (const int32_t *)owner,
+                       (const ActNode *)act[x], R, fb, bs, wide);
+                launch(k_lv_scatter<RecT>, nt, 256, 0, st, nrec, owner, (const ActNode *)act[x],
+                       R, (const int32_t *)fb, (const int32_t *)bs, (const RecT *)buf[cur],
+                       buf[1 - cur], wide);
+                RSG_CHECK_LAUNCH();
+                cur ^= 1;
+                ub = std::min<int64_t>(2 * ub, acap);
             }
-            const int32_t u = (int32_t)ub;
-            launch(k_slot_set, nblk(u, T), T, 0, st, (const int32_t *)act, (const LevelState *)ls,
-                   slot);
-            launch(k_prep<D>, nblk(u, T), T, 0, st, nodes, (const int32_t *)act,
-                   (const LevelState *)ls, lim);
-            launch(k_flags<D, RecT>, nblk(nrec + 1, T), T, 0, st, (const RecT *)buf[cur], nrec,
-                   owner, slot, nodes, lim, flag);
-            cub::DeviceScan::ExclusiveSum(cub_tmp, cub_bytes, flag, rank, (int)(nrec + 1), st);
-            launch(k_counts<D>, nblk(u, T), T, 0, st, nodes, (const int32_t *)act,
-                   (const LevelState *)ls, rank, m_arr, q_arr);
-            launch(k_tables<D>, nblk(nrec, T), T, 0, st, nodes, nrec, owner, slot, flag, rank,
-                   m_arr, fb, bs);
-            launch(k_scatter<D, RecT>, nblk(nrec, T), T, 0, st, nodes, (const RecT *)buf[cur],
-                   buf[1 - cur], nrec, owner, slot, flag, rank, m_arr, q_arr, fb, bs);
-            cur ^= 1;
-            launch(k_split_flags<D>, nblk(u + 1, T), T, 0, st, m_arr, nodes, (const int32_t *)act,
-                   (const LevelState *)ls, u, sub, sflag);
-            cub::DeviceScan::ExclusiveSum(cub_tmp, cub_bytes, sflag, soff, u + 1, st);
-            RSG_CHECK_LAUNCH();
-            launch(k_children<D>, nblk(u, T), T, 0, st, nodes, (const int32_t *)act, ls, m_arr,
-                   (const int64_t *)soff, (int32_t)cap, leaf, sub, sub0, level, subs, nsubs, act2,
-                   bmin, bmax);
-            launch(k_level_advance, 1, 32, 0, st, ls, (const int64_t *)soff);
-            std::swap(act, act2);  // the next level's active nodes
-            launch(k_owner_update<D, RecT>, nblk(nrec, T), T, 0, st, nodes, nrec, owner,
-                   box_owner, sub, (const RecT *)buf[cur], recs);
-            launch(k_box_runs<D, RecT, IT>, nblk((nrec + IT - 1) / IT, T), T, 0, st,
-                   (const RecT *)buf[cur], nrec, box_owner, bmin, bmax);
-            const int64_t u2 = std::min<int64_t>(2 * ub, cap);
-            launch(k_box_final_lvl<D>, nblk(u2, T), T, 0, st, nodes, (const LevelState *)ls,
-                   (int32_t)u2, bmin, bmax);
-            RSG_CHECK_LAUNCH();
-            ub = std::min<int64_t>(u2, acap);
+            RSG_CUDA(cudaMemcpyAsync(&nact, &ls->nact[level], sizeof(nact),
+                                     cudaMemcpyDeviceToHost, st));
+            RSG_CUDA(cudaMemcpyAsync(&hs, ls, sizeof(hs), cudaMemcpyDeviceToHost, st));
+            RSG_CUDA(cudaStreamSynchronize(st));
+            if (hs.err) break;
+            ub = nact;
         }
-        RSG_CUDA(cudaMemcpyAsync(&hs, ls, sizeof(hs), cudaMemcpyDeviceToHost, st));
-        RSG_CUDA(cudaStreamSynchronize(st));
-        if (hs.err) break;
-        ub = hs.nact;
+        if (hs.ncopy && !hs.err)
+            launch(k_copy_segs<RecT>, dim3(hs.ncopy, 64), 256, 0, st, (const int2 *)copies,
+                   (const RecT *)buf[1], recs);
     }
     if (!hs.err) {
         // the larger class first: its blocks are the long ones
-        launch_sub_build<D, RecT, S1, 512, NA1>(hs.nsub[1], recs,
+        launch_sub_build<D, RecT, S1, 512, NA1>(hs.nsub[1], recs, (const RecT *)buf[1],
                                                 (const SubRoot *)subs + (nsubs - hs.nsub[1]),
                                                 nodes, ls, (int32_t)cap, leaf, st);
-        launch_sub_build<D, RecT, S0, 128, NA0>(hs.nsub[0], recs, (const SubRoot *)subs, nodes,
-                                                ls, (int32_t)cap, leaf, st);
+        launch_sub_build<D, RecT, S0, 128, NA0>(hs.nsub[0], recs, (const RecT *)buf[1],
+                                                (const SubRoot *)subs, nodes, ls, (int32_t)cap,
+                                                leaf, st);
         RSG_CHECK_LAUNCH();
         RSG_CUDA(cudaMemcpyAsync(&hs, ls, sizeof(hs), cudaMemcpyDeviceToHost, st));
         RSG_CUDA(cudaStreamSynchronize(st));
