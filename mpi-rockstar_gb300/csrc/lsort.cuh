@@ -12,213 +12,218 @@ namespace rsg {
 #define RSG_LS_SUB0 256  // largest segment of the small blocks
 #define RSG_LS_SUB 2048  // largest segment one block finishes
 
-struct LSeg {
-    int32_t *start, *n;  // active segments
-    int32_t *mn, *mx;    // label range
-    int32_t *m, *q;
+// A segment that a round splits.
+struct LsNode {
+    int32_t start, n, pivot;
+    int32_t m, q;     // elements at or below the pivot; big ones among the first m
+    int32_t rs;       // big elements before start
+    int32_t next[2];  // the halves' places in the next round, -1: none
 };
-// Device-side state of a sort: the round's segment count and the segments
-// listed for the two classes of block.
+// A segment one block finishes, and the buffer that holds it.
+struct LsSub {
+    int32_t start, n, src, pad;
+};
+// Device-side state of a sort.
+#define RSG_LS_ROUNDS 200
 struct LsState {
-    int32_t ns;
-    int32_t nsub[2];
+    int32_t nsub[2];  // segments listed for the two classes of block
+    int32_t ncopy;    // finished segments to be copied to the output
     int32_t pad;
+    int32_t ns[RSG_LS_ROUNDS + 2];  // segments that round r splits
 };
 
-// owner[i]: the active segment holding element i (segments are disjoint and
-// listed by ascending start), -1 outside every segment.
-static __global__ void k_ls_owner(const int32_t *start, const int32_t *n, int32_t ns, int64_t M,
-                                  int32_t *owner) {
-    int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= M) return;
-    int lo = 0, hi = ns - 1, k = -1;
-    while (lo <= hi) {
-        int mid = (lo + hi) >> 1;
-        if (start[mid] <= i) {
-            k = mid;
-            lo = mid + 1;
-        } else {
-            hi = mid - 1;
-        }
-    }
-    owner[i] = (k >= 0 && i < (int64_t)start[k] + n[k]) ? k : -1;
+// pivot = min + (max - min) / 2 (src/fof.c:201)
+__device__ __forceinline__ int32_t ls_pivot(int64_t lo, int64_t hi) {
+    return (int32_t)(lo + (hi - lo) / 2);
 }
-static __global__ void k_ls_init(LSeg S, int32_t ns) {
+// Roots: segments above RSG_LS_SUB elements, in ascending order.  The first
+// pass only takes their label ranges (no label is above the pivot).
+static __global__ void k_ls_roots(const int2 *segs, int32_t ns, LsNode *act, int32_t *range) {
     int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= ns) return;
-    S.mn[k] = 0x7fffffff;
-    S.mx[k] = (int32_t)0x80000000;
-}
-// Label range of every segment.  A thread reads ITEMS consecutive elements;
-// threads whose elements all belong to one segment combine their ranges
-// with the other lanes of that segment before the atomics (a large segment
-// gets one atomic pair per warp instead of one per thread).
-template <int ITEMS>
-static __global__ void k_ls_minmax(const int32_t *lab, int64_t M, const int32_t *owner, LSeg S) {
-    const unsigned FULL = 0xffffffffu;
-    int64_t i0 = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) * ITEMS;
-    int first = -2;  // owner shared by all of this thread's elements, -1 mixed/none
-    int cur = -1, lo = 0x7fffffff, hi = (int)0x80000000;
-    for (int it = 0; it < ITEMS; it++) {
-        int64_t i = i0 + it;
-        int a = (i < M) ? owner[i] : -1;
-        if (first == -2) first = a;
-        else if (a != first) first = -1;
-        if (a != cur) {
-            if (cur >= 0 && first == -1) {  // mixed: this run goes out on its own
-                atomicMin(&S.mn[cur], lo);
-                atomicMax(&S.mx[cur], hi);
-            }
-            cur = a;
-            lo = 0x7fffffff;
-            hi = (int)0x80000000;
-        }
-        if (a < 0) continue;
-        int v = lab[i];
-        lo = min(lo, v);
-        hi = max(hi, v);
-    }
-    bool uni = first >= 0;  // every element in one segment: combine across the warp
-    unsigned grp = __match_any_sync(FULL, uni ? first : -1);
-    if (uni) {
-        int glo = __reduce_min_sync(grp, lo), ghi = __reduce_max_sync(grp, hi);
-        if ((threadIdx.x & 31) == __ffs(grp) - 1) {
-            atomicMin(&S.mn[first], glo);
-            atomicMax(&S.mx[first], ghi);
-        }
-    } else if (cur >= 0) {
-        atomicMin(&S.mn[cur], lo);
-        atomicMax(&S.mx[cur], hi);
+    LsNode a = {};
+    a.start = segs[k].x;
+    a.n = segs[k].y;
+    a.pivot = 0x7fffffff;
+    act[k] = a;
+    for (int h = 0; h < 2; h++) {
+        range[4 * k + 2 * h] = 0x7fffffff;
+        range[4 * k + 2 * h + 1] = (int32_t)0x80000000;
     }
 }
-// pivot = min + (max - min) / 2 (src/fof.c:201); a segment whose labels are
-// all equal is finished (no element is "big").
-__device__ __forceinline__ int32_t ls_pivot(int64_t lo, int64_t hi) {
-    return (lo == hi) ? 0x7fffffff : (int32_t)(lo + (hi - lo) / 2);
+static __global__ void k_ls_owner(const LsNode *act, int32_t *owner) {
+    const LsNode &a = act[blockIdx.x];
+    for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < a.n; i += gridDim.y * blockDim.x)
+        owner[a.start + i] = blockIdx.x;
 }
-static __global__ void k_ls_flags(const int32_t *lab, int64_t M, const int32_t *owner, LSeg S,
-                           int32_t *flag) {
-    int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i > M) return;
-    int f = 0;
-    if (i < M) {
-        int a = owner[i];
-        if (a >= 0) f = lab[i] > ls_pivot(S.mn[a], S.mx[a]);
-    }
-    flag[i] = f;
-}
-// m (= #small) and q (= #big before m) per segment, and which halves of
-// the segments that split go on: above RSG_LS_SUB elements to the next round
-// (hflag), from 2 to there to the block lists.  Grid over ub + 1, ub bounding
-// the round's segments.
-static __global__ void k_ls_counts(LSeg S, LsState *st, int32_t ub, const int32_t *rank,
-                                   int32_t *hflag, int2 *subs, int32_t nsubs) {
+// Pivots of the roots.  One whose labels are all equal splits off nothing:
+// its halves are itself and nothing, and go no further.
+static __global__ void k_ls_root_pivot(LsNode *act, int32_t ns, int32_t *range) {
     int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k > ub) return;
-    if (k >= st->ns) {
-        hflag[2 * k] = 0;
-        if (k < ub) hflag[2 * k + 1] = 0;
-        return;
-    }
-    int s = S.start[k], n = S.n[k];
-    int B = rank[s + n] - rank[s];
-    int m = n - B;
-    S.m[k] = m;
-    S.q[k] = rank[s + m] - rank[s];
-    const bool split = S.mn[k] != S.mx[k];
+    if (k >= ns) return;
+    const int32_t lo = range[4 * k], hi = range[4 * k + 1];
+    act[k].pivot = lo == hi ? 0x7fffffff : ls_pivot(lo, hi);
+    range[4 * k] = 0x7fffffff;
+    range[4 * k + 1] = (int32_t)0x80000000;
+}
+// One pass over the labels of a round: the "big" flags as rank bits and the
+// label ranges of both halves (as k_lv_flags takes its boxes).
+static __global__ void __launch_bounds__(256) k_ls_flags(const int32_t *lab, int64_t M,
+                                                         const int32_t *owner, const LsNode *act,
+                                                         int32_t *range, RankBits R) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int64_t first = blockIdx.x * (int64_t)RSG_TILE + w * RSG_STRETCH;
+    const int a0 = stretch_owner(owner, first, M, true);
+    __shared__ int part[8][4];
+    __shared__ int a_s;
+    if (threadIdx.x == 0) a_s = a0;
+    __syncthreads();
+    const bool whole = __syncthreads_and(a0 >= 0 && a0 == a_s);
+    uint32_t word = 0;
+    if (a0 >= 0) {
+        const int pivot = act[a0].pivot;
+        int lo[2] = {0x7fffffff, 0x7fffffff}, hi[2] = {(int)0x80000000, (int)0x80000000};
 #pragma unroll
+        for (int u = 0; u < 8; u++) {
+            const int64_t i = first + 32 * u + lane;
+            const bool on = i < M;
+            const int v = on ? lab[i] : 0;
+            const bool big = on && v > pivot;
+            const unsigned b = __ballot_sync(FULL, big);
+            if (lane == u) word = b;
+            if (on) {
+                lo[0] = big ? lo[0] : min(lo[0], v);
+                hi[0] = big ? hi[0] : max(hi[0], v);
+                lo[1] = big ? min(lo[1], v) : lo[1];
+                hi[1] = big ? max(hi[1], v) : hi[1];
+            }
+        }
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int a = __reduce_min_sync(FULL, lo[h]), b = __reduce_max_sync(FULL, hi[h]);
+            if (lane == 0 && whole) {
+                part[w][2 * h] = a;
+                part[w][2 * h + 1] = b;
+            } else if (lane == 0 && a <= b) {
+                atomicMin(&range[4 * a0 + 2 * h], a);
+                atomicMax(&range[4 * a0 + 2 * h + 1], b);
+            }
+        }
+    } else if (a0 == -2) {
+        for (int u = 0; u < 8; u++) {
+            const int64_t i = first + 32 * u + lane;
+            const int a = i < M ? owner[i] : -1;
+            bool big = false;
+            if (a >= 0) {
+                const int v = lab[i];
+                big = v > act[a].pivot;
+                atomicMin(&range[4 * a + (big ? 2 : 0)], v);
+                atomicMax(&range[4 * a + (big ? 3 : 1)], v);
+            }
+            const unsigned b = __ballot_sync(FULL, big);
+            if (lane == u) word = b;
+        }
+    }
+    rank_store(R, blockIdx.x, word);  // holds a block barrier after the loop above
+    if (whole && threadIdx.x < 4) {
+        int v = part[0][threadIdx.x];
+        for (int q = 1; q < 8; q++)
+            v = (threadIdx.x & 1) ? max(v, part[q][threadIdx.x]) : min(v, part[q][threadIdx.x]);
+        if (threadIdx.x & 1) atomicMax(&range[4 * a0 + threadIdx.x], v);
+        else atomicMin(&range[4 * a0 + threadIdx.x], v);
+    }
+}
+// Counts of a round's segments, and where each half goes: one of several
+// labels above RSG_LS_SUB elements to the next round, up to there to the
+// block lists; one of equal labels is finished, and copied (by a block, or as
+// a segment) when the round leaves it in the scratch buffer (dst 1).
+static __global__ void k_ls_nodes(LsNode *act, LsNode *nxt, const int32_t *range, int32_t *rnext,
+                                  LsState *st, RankBits R, int32_t round, int dst, LsSub *subs,
+                                  int32_t nsubs, int2 *copies) {
+    int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= st->ns[round]) return;
+    LsNode &A = act[k];
+    const int s = A.start, n = A.n, rs = R.rank(s);
+    const int m = n - (R.rank((int64_t)s + n) - rs);
+    A.m = m;
+    A.q = R.rank((int64_t)s + m) - rs;
+    A.rs = rs;
     for (int h = 0; h < 2; h++) {
         const int hs = h ? s + m : s, hn = h ? n - m : m;
-        hflag[2 * k + h] = split && hn > RSG_LS_SUB;
-        if (split && hn >= 2 && hn <= RSG_LS_SUB) {
+        const int32_t lo = range[4 * k + 2 * h], hi = range[4 * k + 2 * h + 1];
+        A.next[h] = -1;
+        if (hn > RSG_LS_SUB) {
+            if (lo != hi) {
+                const int j = atomicAdd(&st->ns[round + 1], 1);
+                A.next[h] = j;
+                LsNode x = {};
+                x.start = hs;
+                x.n = hn;
+                x.pivot = ls_pivot(lo, hi);
+                nxt[j] = x;
+                for (int g = 0; g < 2; g++) {
+                    rnext[4 * j + 2 * g] = 0x7fffffff;
+                    rnext[4 * j + 2 * g + 1] = (int32_t)0x80000000;
+                }
+            } else if (dst) {
+                copies[atomicAdd(&st->ncopy, 1)] = make_int2(hs, hn);
+            }
+        } else if (hn > 0 && (lo != hi || dst)) {
             const int c = hn > RSG_LS_SUB0;
             const int at = atomicAdd(&st->nsub[c], 1);
-            subs[c ? nsubs - 1 - at : at] = make_int2(hs, hn);
+            subs[c ? nsubs - 1 - at : at] = LsSub{hs, hn, dst, 0};
         }
     }
 }
-static __global__ void k_ls_tables(int64_t M, const int32_t *owner, LSeg S, const int32_t *flag,
-                            const int32_t *rank, int32_t *fb, int32_t *bs) {
-    int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= M) return;
-    int a = owner[i];
-    if (a < 0) return;
-    int s = S.start[a];
-    int l = (int)(i - s);
-    int br = rank[i] - rank[s];
-    int sr = l - br;
-    int m = S.m[a];
-    if (flag[i] && l < m) fb[s + br] = l;
-    if (!flag[i] && l >= m) bs[s + (m - 1 - sr)] = l;
+static __global__ void __launch_bounds__(256) k_ls_tables(int64_t M, const int32_t *owner,
+                                                          const LsNode *act, RankBits R,
+                                                          int32_t *fb, int32_t *bs) {
+    const int lane = threadIdx.x & 31;
+    const int64_t first = blockIdx.x * (int64_t)RSG_TILE + (threadIdx.x >> 5) * RSG_STRETCH;
+    const int a0 = stretch_owner(owner, first, M, true);
+    if (a0 == -1) return;
+#pragma unroll 1
+    for (int u = 0; u < 8; u++) {
+        const int64_t i = first + 32 * u + lane;
+        if (i >= M) return;
+        const int k = a0 >= 0 ? a0 : owner[i];
+        if (k < 0) continue;
+        const LsNode &A = act[k];
+        swap_tables((int)(i - A.start), R.big(i), R.rank(i) - A.rs, A.m, fb + A.start,
+                    bs + A.start);
+    }
 }
+// Elements to their places; a place then belongs to the half it lies in.
 template <class T>
-__global__ void k_ls_scatter(int64_t M, const int32_t *owner, LSeg S, const int32_t *flag,
-                             const int32_t *rank, const int32_t *fb, const int32_t *bs,
-                             const T *src, T *dst, const int32_t *lsrc, int32_t *ldst) {
-    int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= M) return;
-    int a = owner[i];
-    if (a < 0) return;
-    int s = S.start[a], n = S.n[a];
-    int l = (int)(i - s);
-    int br = rank[i] - rank[s];
-    int sr = l - br;
-    int m = S.m[a], q = S.q[a];
-    int big = flag[i];
-    int d;
-    if (!big && l < m) d = l;
-    else if (big && l < m) d = (br == 0) ? n - 1 : bs[s + br - 1] - 1;
-    else if (!big) d = fb[s + (m - 1 - sr)];
-    else {
-        int pos_last = (q > 0) ? bs[s + q - 1] : n;
-        if (l > pos_last) d = l - 1;
-        else if (pos_last - m >= 2) d = (l == m) ? pos_last - 1 : l - 1;
-        else d = l;
+__global__ void __launch_bounds__(256) k_ls_scatter(int64_t M, int32_t *owner, const LsNode *act,
+                                                    RankBits R, const int32_t *fb,
+                                                    const int32_t *bs, const T *src, T *dst,
+                                                    const int32_t *lsrc, int32_t *ldst) {
+    const int lane = threadIdx.x & 31;
+    const int64_t first = blockIdx.x * (int64_t)RSG_TILE + (threadIdx.x >> 5) * RSG_STRETCH;
+    const int a0 = stretch_owner(owner, first, M, true);
+    __syncwarp();  // every lane has read the owners that are written below
+    if (a0 == -1) return;
+    LsNode A;
+    if (a0 >= 0) A = act[a0];
+#pragma unroll 2
+    for (int u = 0; u < 8; u++) {
+        const int64_t i = first + 32 * u + lane;
+        if (i >= M) return;
+        if (a0 < 0) {
+            const int k = owner[i];
+            if (k < 0) continue;
+            A = act[k];
+        }
+        const T r = src[i];
+        const int v = lsrc[i], l = (int)(i - A.start);
+        const int d = swap_dest(l, A.n, R.big(i), R.rank(i) - A.rs, A.m, A.q, fb + A.start,
+                                bs + A.start);
+        dst[A.start + d] = r;
+        ldst[A.start + d] = v;
+        owner[i] = A.next[l >= A.m];
     }
-    dst[s + d] = src[i];
-    ldst[s + d] = lsrc[i];
-}
-// After a round: every element moves to the half of its segment it now
-// lies in; a half of the next round (hflag) has its compacted index (hidx),
-// and the elements of the other halves are copied from the buffer the round
-// wrote (src) to the output arrays when they differ: they are final, or a
-// block's to finish in place.
-template <class T>
-__global__ void k_ls_owner_next(int64_t M, int32_t *owner, LSeg S, const int32_t *hflag,
-                                const int32_t *hidx, const T *src, T *dst, const int32_t *lsrc,
-                                int32_t *ldst) {
-    int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= M) return;
-    int a = owner[i];
-    if (a < 0) return;
-    int h = 2 * a + ((i - S.start[a]) < S.m[a] ? 0 : 1);
-    if (hflag[h]) {
-        owner[i] = hidx[h];
-        return;
-    }
-    owner[i] = -1;
-    if (src != dst) {
-        dst[i] = src[i];
-        ldst[i] = lsrc[i];
-    }
-}
-// The next round's segments, with their label ranges cleared.
-static __global__ void k_ls_next(LSeg S, LsState *st, int32_t ub, const int32_t *hflag,
-                                 const int32_t *hidx, LSeg R) {
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= ub || k >= st->ns) return;
-    for (int h = 0; h < 2; h++) {
-        if (!hflag[2 * k + h]) continue;
-        const int j = hidx[2 * k + h];
-        R.start[j] = h ? S.start[k] + S.m[k] : S.start[k];
-        R.n[j] = h ? S.n[k] - S.m[k] : S.m[k];
-        R.mn[j] = 0x7fffffff;
-        R.mx[j] = (int32_t)0x80000000;
-    }
-}
-static __global__ void k_ls_advance(LsState *st, int32_t ub, const int32_t *hidx) {
-    if (threadIdx.x || blockIdx.x) return;
-    st->ns = hidx[2 * ub];
 }
 
 // One block's storage for a segment of at most S elements (at most S / 2
@@ -265,16 +270,21 @@ __device__ __forceinline__ void ls_range(int32_t (*mn)[2], int32_t (*mx)[2], int
 }
 // Finishes one listed segment per block, all its levels in shared memory, as
 // k_sub_build does a subtree: flags as bits, ranks by population counts,
-// 2-byte places, the records and labels moved once at the end.  A level costs
-// the chain of six block barriers, where a round of the loop below costs ten
-// launches and passes over all the call's elements: the sorts of one level of
-// a 64^3 snapshot were 79 rounds of the loop, 3 ms of launches.
+// 2-byte places, the records and labels moved once at the end (from the
+// scratch buffer where the rounds left them there).  A level costs the chain
+// of six block barriers, where a round of the loop below costs five launches
+// and passes over all the call's elements: with every level a round, the sorts
+// of a 64^3 snapshot were 79 rounds.
 template <class R, int S, int T>
-__global__ void __launch_bounds__(T) k_ls_sub(R *W, int32_t *lab, const int2 *segs) {
+__global__ void __launch_bounds__(T) k_ls_sub(R *W, int32_t *lab, const R *sw, const int32_t *sl,
+                                              const LsSub *segs) {
     extern __shared__ __align__(16) unsigned char ls_sm[];
     LsShared<S> &h = *reinterpret_cast<LsShared<S> *>(ls_sm);
     const int t = threadIdx.x, lane = t & 31;
-    const int g0 = segs[blockIdx.x].x, n = segs[blockIdx.x].y;
+    const LsSub seg = segs[blockIdx.x];
+    const int g0 = seg.start, n = seg.n;
+    const R *from = seg.src ? sw : W;
+    const int32_t *lfrom = seg.src ? sl : lab;
     const int nw = (n + 31) >> 5;
     const int span = ((n + T - 1) / T) * T;  // whole warps take part in every pass
     if (t == 0) {
@@ -285,7 +295,7 @@ __global__ void __launch_bounds__(T) k_ls_sub(R *W, int32_t *lab, const int2 *se
     __syncthreads();
     for (int i = t; i < span; i += T) {
         const bool ok = i < n;
-        const int v = ok ? lab[g0 + i] : 0;
+        const int v = ok ? lfrom[g0 + i] : 0;
         if (ok) {
             h.lab[i] = v;
             h.idx[0][i] = (uint16_t)i;
@@ -294,12 +304,13 @@ __global__ void __launch_bounds__(T) k_ls_sub(R *W, int32_t *lab, const int2 *se
         ls_range(h.mn, h.mx, v, ok ? 0 : RSG_LS_NONE, false);
     }
     __syncthreads();
-    if (h.mn[0][0] == h.mx[0][0]) return;  // nothing moves
+    const bool moves = h.mn[0][0] != h.mx[0][0];
+    if (!moves && !seg.src) return;
     if (t == 0) {
         h.s[0][0] = 0;
         h.n[0][0] = (uint16_t)n;
         h.pivot[0][0] = ls_pivot(h.mn[0][0], h.mx[0][0]);
-        h.nact[0] = 1;
+        h.nact[0] = moves;
     }
     auto rank = [&](int x) {
         return h.wpre[x >> 5] + __popc(h.bits[x >> 5] & ((1u << (x & 31)) - 1u));
@@ -407,31 +418,33 @@ __global__ void __launch_bounds__(T) k_ls_sub(R *W, int32_t *lab, const int2 *se
     }
     constexpr int V = sizeof(R) / 16, PER = S / T;
     static_assert(sizeof(R) % 16 == 0 && S % T == 0, "record vectors");
-    uint4 *rv = reinterpret_cast<uint4 *>(W + g0);
+    const uint4 *sv = reinterpret_cast<const uint4 *>(from + g0);
+    uint4 *dv = reinterpret_cast<uint4 *>(W + g0);
 #pragma unroll 1
     for (int v = 0; v < V; v++) {
         uint4 r[PER];
 #pragma unroll
         for (int u = 0; u < PER; u++) {
             const int i = t + u * T;
-            if (i < n) r[u] = rv[(int)h.idx[cur][i] * V + v];
+            if (i < n) r[u] = sv[(int)h.idx[cur][i] * V + v];
         }
         __syncthreads();
 #pragma unroll
         for (int u = 0; u < PER; u++) {
             const int i = t + u * T;
-            if (i < n) rv[i * V + v] = r[u];
+            if (i < n) dv[i * V + v] = r[u];
         }
     }
     for (int i = t; i < n; i += T) lab[g0 + i] = h.lab[h.idx[cur][i]];
 }
 template <class R, int S, int T>
-void launch_ls_sub(int32_t count, R *W, int32_t *lab, const int2 *segs, cudaStream_t st) {
+void launch_ls_sub(int32_t count, R *W, int32_t *lab, const R *sw, const int32_t *sl,
+                   const LsSub *segs, cudaStream_t st) {
     if (count == 0) return;
     const size_t sm = sizeof(LsShared<S>);
     RSG_CUDA(cudaFuncSetAttribute(k_ls_sub<R, S, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)sm));
-    launch(k_ls_sub<R, S, T>, count, T, sm, st, W, lab, segs);
+    launch(k_ls_sub<R, S, T>, count, T, sm, st, W, lab, sw, sl, segs);
 }
 
 // Sorts W (and its labels) inside every segment (host arrays hs/hn) the way
@@ -441,111 +454,104 @@ template <class T>
 void partition_sort_labels(Arena &ar, T *W, int32_t *lab, int64_t M,
                            const std::vector<int32_t> &hs, const std::vector<int32_t> &hn,
                            cudaStream_t st) {
-    std::vector<int32_t> s0, n0;  // the segments of the round loop
-    std::vector<int2> c0, c1;     // those the blocks finish
+    std::vector<int2> roots;    // the segments of the round loop
+    std::vector<LsSub> c0, c1;  // those the blocks finish
     for (size_t k = 0; k < hs.size(); k++) {
-        if (hn[k] > RSG_LS_SUB) {
-            s0.push_back(hs[k]);
-            n0.push_back(hn[k]);
-        } else if (hn[k] >= 2) {
-            (hn[k] > RSG_LS_SUB0 ? c1 : c0).push_back(make_int2(hs[k], hn[k]));
-        }
+        if (hn[k] > RSG_LS_SUB) roots.push_back(make_int2(hs[k], hn[k]));
+        else if (hn[k] >= 2) (hn[k] > RSG_LS_SUB0 ? c1 : c0).push_back(LsSub{hs[k], hn[k], 0, 0});
     }
-    const int32_t ns = (int32_t)s0.size();
+    const int32_t ns = (int32_t)roots.size();
     if (ns == 0 && c0.empty() && c1.empty()) return;
-    const int T_ = 256;
     size_t mark = ar.used;
-    LsState h = {};
-    h.ns = ns;
-    h.nsub[0] = (int32_t)c0.size();
-    h.nsub[1] = (int32_t)c1.size();
-    // listed segments are disjoint, of two elements or more
-    const int32_t nsubs = (int32_t)(M / 2 + 1);
-    int2 *subs = ar.get<int2>(nsubs);
+    struct Head {  // the fields of LsState before ns[]
+        int32_t nsub[2], ncopy, pad;
+    } h = {{(int32_t)c0.size(), (int32_t)c1.size()}, 0, 0};
+    static_assert(offsetof(LsState, ns) == sizeof(Head), "LsState layout");
+    // listed segments are disjoint
+    const int32_t nsubs = (int32_t)(ns > 0 ? M : (int64_t)(c0.size() + c1.size()));
+    LsSub *subs = ar.get<LsSub>(nsubs);
     if (!c0.empty())
-        RSG_CUDA(cudaMemcpyAsync(subs, c0.data(), sizeof(int2) * c0.size(),
+        RSG_CUDA(cudaMemcpyAsync(subs, c0.data(), sizeof(LsSub) * c0.size(),
                                  cudaMemcpyHostToDevice, st));
     if (!c1.empty())
-        RSG_CUDA(cudaMemcpyAsync(subs + (nsubs - c1.size()), c1.data(), sizeof(int2) * c1.size(),
+        RSG_CUDA(cudaMemcpyAsync(subs + (nsubs - c1.size()), c1.data(), sizeof(LsSub) * c1.size(),
                                  cudaMemcpyHostToDevice, st));
+    // rounds scatter back and forth between these
+    T *wb[2] = {W, nullptr};
+    int32_t *lb[2] = {lab, nullptr};
     if (ns > 0) {
         const int64_t cap = M / (RSG_LS_SUB + 1) + 1;  // segments of a round
-        LSeg S[2];
+        LsNode *act[2];
+        int32_t *range[2];
         for (int b = 0; b < 2; b++) {
-            S[b].start = ar.get<int32_t>(cap); S[b].n = ar.get<int32_t>(cap);
-            S[b].mn = ar.get<int32_t>(cap); S[b].mx = ar.get<int32_t>(cap);
-            S[b].m = ar.get<int32_t>(cap); S[b].q = ar.get<int32_t>(cap);
+            act[b] = ar.get<LsNode>(cap);
+            range[b] = ar.get<int32_t>(4 * cap);
         }
-        int32_t *hflag = ar.get<int32_t>(2 * cap + 1), *hidx = ar.get<int32_t>(2 * cap + 1);
-        int32_t *owner = ar.get<int32_t>(M), *flag = ar.get<int32_t>(M + 1);
-        int32_t *rank = ar.get<int32_t>(M + 1);
-        int32_t *fb = ar.get<int32_t>(M), *bs = ar.get<int32_t>(M);
-        T *tw = ar.get<T>(M);
-        int32_t *tl = ar.get<int32_t>(M);
+        int2 *copies = ar.get<int2>(cap), *d_roots = ar.get<int2>(ns);
+        int32_t *owner = ar.get<int32_t>(M), *fb = ar.get<int32_t>(M), *bs = ar.get<int32_t>(M);
+        wb[1] = ar.get<T>(M);
+        lb[1] = ar.get<int32_t>(M);
         LsState *ls = ar.get<LsState>(1);
-        size_t b1 = 0, b3 = 0;
-        cub::DeviceScan::ExclusiveSum(nullptr, b1, flag, rank, (int)(M + 1), st);
-        cub::DeviceScan::ExclusiveSum(nullptr, b3, hflag, hidx, (int)(2 * cap + 1), st);
-        if (b3 > b1) b1 = b3;
-        void *tmp = ar.take(b1 + 256);
-        size_t tb = b1 + 256;
-        RSG_CUDA(cudaMemcpyAsync(S[0].start, s0.data(), 4 * ns, cudaMemcpyHostToDevice, st));
-        RSG_CUDA(cudaMemcpyAsync(S[0].n, n0.data(), 4 * ns, cudaMemcpyHostToDevice, st));
+        const RankBits R = rank_alloc(ar, M, st);
+        const int32_t nt = (int32_t)rank_tiles(M);
+        RSG_CUDA(cudaMemcpyAsync(d_roots, roots.data(), sizeof(int2) * ns, cudaMemcpyHostToDevice, st));
+        RSG_CUDA(cudaMemsetAsync(ls, 0, sizeof(LsState), st));
         RSG_CUDA(cudaMemcpyAsync(ls, &h, sizeof(h), cudaMemcpyHostToDevice, st));
-        // rounds scatter back and forth between (W, lab) and (tw, tl); an
-        // element is copied to (W, lab) once, when its segment leaves the loop
-        T *wb[2] = {W, tw};
-        int32_t *lb[2] = {lab, tl};
-        int cur = 0;
-        launch(k_ls_owner, nblk(M, T_), T_, 0, st, (const int32_t *)S[0].start,
-               (const int32_t *)S[0].n, ns, M, owner);
-        launch(k_ls_init, nblk(ns, T_), T_, 0, st, S[0], ns);
+        RSG_CUDA(cudaMemcpyAsync(&ls->ns[0], &ns, sizeof(ns), cudaMemcpyHostToDevice, st));
+        RSG_CUDA(cudaMemsetAsync(owner, 0xff, sizeof(int32_t) * M, st));
+        launch(k_ls_roots, nblk(ns, 64), 64, 0, st, (const int2 *)d_roots, ns, act[0], range[0]);
+        const int64_t y = M / ns / 2048;
+        launch(k_ls_owner, dim3(ns, (unsigned)(y < 1 ? 1 : (y > 4096 ? 4096 : y))), 256, 0, st,
+               (const LsNode *)act[0], owner);
+        launch(k_ls_flags, nt, 256, 0, st, (const int32_t *)lab, M, (const int32_t *)owner,
+               (const LsNode *)act[0], range[0], R);
+        launch(k_ls_root_pivot, nblk(ns, 64), 64, 0, st, act[0], ns, range[0]);
         // Rounds run back to back with their counts on the device; grids are
         // sized by an upper bound of the segments (ub).  A round past the last
-        // costs passes over M elements (0.2 ms at 33M) against the 12 us of a
-        // read, so large calls read after every round.
+        // costs passes over M elements against the 12 us of a read, so large
+        // calls read after every round.
         const int batch = M > (1 << 22) ? 1 : RSG_LS_BATCH;
         int64_t ub = ns;
-        for (int round = 0; h.ns > 0;) {
+        int32_t now = ns;
+        int cur = 0;
+        for (int round = 0; now > 0;) {
             for (int b = 0; b < batch; b++, round++) {
-                if (round > 200) {
+                if (round > RSG_LS_ROUNDS) {
                     set_error(RSG_ERR_LIMIT, "label partition sort did not terminate");
                     throw Failure();
                 }
-                const LSeg &A = S[round & 1], &B = S[1 - (round & 1)];
-                const int32_t u = (int32_t)ub;
-                launch(k_ls_minmax<8>, nblk((M + 7) / 8, T_), T_, 0, st, (const int32_t *)lb[cur],
-                       M, (const int32_t *)owner, A);
-                launch(k_ls_flags, nblk(M + 1, T_), T_, 0, st, (const int32_t *)lb[cur], M,
-                       (const int32_t *)owner, A, flag);
-                cub::DeviceScan::ExclusiveSum(tmp, tb, flag, rank, (int)(M + 1), st);
-                launch(k_ls_counts, nblk(u + 1, T_), T_, 0, st, A, ls, u, (const int32_t *)rank,
-                       hflag, subs, nsubs);
-                launch(k_ls_tables, nblk(M, T_), T_, 0, st, M, (const int32_t *)owner, A,
-                       (const int32_t *)flag, (const int32_t *)rank, fb, bs);
-                launch(k_ls_scatter<T>, nblk(M, T_), T_, 0, st, M, (const int32_t *)owner, A,
-                       (const int32_t *)flag, (const int32_t *)rank, (const int32_t *)fb,
-                       (const int32_t *)bs, (const T *)wb[cur], wb[1 - cur],
+                const int x = round & 1;
+                launch(k_ls_flags, nt, 256, 0, st, (const int32_t *)lb[cur], M,
+                       (const int32_t *)owner, (const LsNode *)act[x], range[x], R);
+                launch(k_rank_scan, 1, 1024, 0, st, R.tpre, nt);
+                launch(k_ls_nodes, nblk(ub, 64), 64, 0, st, act[x], act[1 - x],
+                       (const int32_t *)range[x], range[1 - x], ls, R, round, 1 - cur, subs, nsubs,
+                       copies);
+                launch(k_ls_tables, nt, 256, 0, st, M, (const int32_t *)owner,
+                       (const LsNode *)act[x], R, fb, bs);
+                launch(k_ls_scatter<T>, nt, 256, 0, st, M, owner, (const LsNode *)act[x], R,
+                       (const int32_t *)fb, (const int32_t *)bs, (const T *)wb[cur], wb[1 - cur],
                        (const int32_t *)lb[cur], lb[1 - cur]);
-                cur ^= 1;
-                cub::DeviceScan::ExclusiveSum(tmp, tb, hflag, hidx, 2 * u + 1, st);
-                launch(k_ls_owner_next<T>, nblk(M, T_), T_, 0, st, M, owner, A,
-                       (const int32_t *)hflag, (const int32_t *)hidx, (const T *)wb[cur], W,
-                       (const int32_t *)lb[cur], lab);
-                launch(k_ls_next, nblk(u, T_), T_, 0, st, A, ls, u, (const int32_t *)hflag,
-                       (const int32_t *)hidx, B);
-                launch(k_ls_advance, 1, 1, 0, st, ls, u, (const int32_t *)hidx);
                 RSG_CHECK_LAUNCH();
+                cur ^= 1;
                 ub = std::min<int64_t>(2 * ub, cap);
             }
+            RSG_CUDA(cudaMemcpyAsync(&now, &ls->ns[round], sizeof(now), cudaMemcpyDeviceToHost, st));
             RSG_CUDA(cudaMemcpyAsync(&h, ls, sizeof(h), cudaMemcpyDeviceToHost, st));
             RSG_CUDA(cudaStreamSynchronize(st));
-            ub = h.ns;
+            ub = now;
+        }
+        if (h.ncopy) {
+            launch(k_copy_segs<T>, dim3(h.ncopy, 64), 256, 0, st, (const int2 *)copies,
+                   (const T *)wb[1], W);
+            launch(k_copy_segs<int32_t>, dim3(h.ncopy, 64), 256, 0, st, (const int2 *)copies,
+                   (const int32_t *)lb[1], lab);
         }
     }
-    launch_ls_sub<T, RSG_LS_SUB, 512>(h.nsub[1], W, lab, (const int2 *)subs + (nsubs - h.nsub[1]),
-                                      st);
-    launch_ls_sub<T, RSG_LS_SUB0, 64>(h.nsub[0], W, lab, (const int2 *)subs, st);
+    launch_ls_sub<T, RSG_LS_SUB, 512>(h.nsub[1], W, lab, (const T *)wb[1], (const int32_t *)lb[1],
+                                      (const LsSub *)subs + (nsubs - h.nsub[1]), st);
+    launch_ls_sub<T, RSG_LS_SUB0, 64>(h.nsub[0], W, lab, (const T *)wb[1], (const int32_t *)lb[1],
+                                      (const LsSub *)subs, st);
     RSG_CHECK_LAUNCH();
     ar.used = mark;
 }
