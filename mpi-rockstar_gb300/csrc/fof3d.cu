@@ -148,7 +148,7 @@ __device__ void sphere3_warp(const KNode<3> *nodes, const Rec *recs, const float
         const int xi = sn[sp];
         const unsigned m = sm[sp] & live;
         if (!m) continue;
-        const KNode<3> &nd = nodes[xi];
+        const KNode<3> nd = nodes[xi];  // three 16-byte loads
         int kind = 0;  // 1 out, 2 inside, 3 leaf points, 4 descend
         if (m & bit) {
             kind = 1;

@@ -163,8 +163,8 @@ __device__ __forceinline__ double d2d(const float *a, const float *b) {
 // Internal potential-tree nodes above this size are reduced by a block.
 #define RSG_BH_BIG 4096
 
-struct BHNode {
-    float mc[3], m, dmin;
+struct __align__(16) BHNode {  // the centre and mass in one 16-byte load
+    float mc[3], m, dmin, pad[3];
 };
 
 // src/potential.c:71-82 over the node's points
@@ -468,7 +468,9 @@ __global__ void __launch_bounds__(32 * RSG_BH_WPB) k_bh_walk(const KNode<3> *nod
         while (sp) {
             const int b = st[--sp];
             __syncwarp(hm);  // every lane has read before lane 0 pushes over the slot
-            const KNode<3> &n2 = nodes[b];
+            const KNode<3> n2 = nodes[b];  // three 16-byte loads
+            const float4 c4 = *reinterpret_cast<const float4 *>(&B[b]);
+            const float mc[3] = {c4.x, c4.y, c4.z};
             if (b == a) {
                 if (n.n > 20) continue;  // degenerate leaf
                 for (int qi = 0; qi < n.n; qi++) {
@@ -491,8 +493,8 @@ __global__ void __launch_bounds__(32 * RSG_BH_WPB) k_bh_walk(const KNode<3> *nod
                     // within 2.4e-7 of it (relative); outside a 2e-6 band around
                     // dmin^2 the FP32 value decides the same way, inside it the
                     // FP64 sum decides (GB300's FP64 pipe is narrow).
-                    float dx = fsub(bn.mc[0], B[b].mc[0]), dy = fsub(bn.mc[1], B[b].mc[1]),
-                          dz = fsub(bn.mc[2], B[b].mc[2]);
+                    float dx = fsub(bn.mc[0], mc[0]), dy = fsub(bn.mc[1], mc[1]),
+                          dz = fsub(bn.mc[2], mc[2]);
                     float sf = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, fmul(dx, dx)));
                     if (sf > 1e-30f && sf < 1e30f && dm2 > 1e-30f && dm2 < 1e30f) {
                         if (sf > fmul(dm2, 1.000002f)) dec = 0;
@@ -500,7 +502,7 @@ __global__ void __launch_bounds__(32 * RSG_BH_WPB) k_bh_walk(const KNode<3> *nod
                     }
                 }
                 if (dec < 0) {
-                    float r2 = (float)d2d(bn.mc, B[b].mc);
+                    float r2 = (float)d2d(bn.mc, mc);
                     open = !(r2 > dm2);
                 } else {
                     open = dec == 1;
@@ -526,14 +528,13 @@ __global__ void __launch_bounds__(32 * RSG_BH_WPB) k_bh_walk(const KNode<3> *nod
                     __syncwarp(hm);
                 }
             } else if (act) {
-                const BHNode &m = B[b];
                 if (F32) {
-                    float dx = px[0] - m.mc[0], dy = px[1] - m.mc[1], dz = px[2] - m.mc[2];
+                    float dx = px[0] - mc[0], dy = px[1] - mc[1], dz = px[2] - mc[2];
                     float r2 = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, dx * dx));
-                    add(0.0, m.m * rsqrtf(r2));
+                    add(0.0, c4.w * rsqrtf(r2));
                 } else {
-                    float r = (float)sqrt(d2d(px, m.mc));
-                    add((double)__fdiv_rn(m.m, r), 0.f);
+                    float r = (float)sqrt(d2d(px, mc));
+                    add((double)__fdiv_rn(c4.w, r), 0.f);
                 }
             }
         }
