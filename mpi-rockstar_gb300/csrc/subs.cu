@@ -498,7 +498,8 @@ __device__ __forceinline__ bool box_out6(const KNode<6> &nd, const float *c, flo
     return false;
 }
 
-// The first 48 bytes of a node, its box, as three 16-byte loads.
+// The first 48 bytes of a node, its box, as three 16-byte loads: a warp whose
+// lanes read different nodes pays for each load instruction by the lane.
 __device__ __forceinline__ float box_near6(const KNode<6> *nd, const float *c) {
     const float4 *v = reinterpret_cast<const float4 *>(nd);
     const float4 a = v[0], b = v[1], e = v[2];
@@ -870,15 +871,15 @@ __global__ void k_fill_eln(HierNodes N, int32_t base, int32_t *eln) {
 // monotone, so the sum of their squares in the same order bounds the lane's
 // distance.  With one node at a time for the whole warp and every point of a
 // leaf tested by every lane the searches of a quarter of the 512^3 volume
-// took 136 ms, 77% of the issue slots busy; now 83 ms (149, 109 and 85 ms for
-// runs of 0.5, 1 and 4 linking lengths: short runs repeat the walk, wide
-// boxes admit more points).
+// took 136 ms, 77% of the issue slots busy; now 70 ms.  (Without the lanes'
+// test of a leaf before its points, 83 ms at best, with runs of 2 linking
+// lengths: short runs repeat the walk, wide boxes admit more points.)
 // MODE 2 counts every list, keeps its first RSG_SLOT6 entries in a fixed slot
 // per particle and the rest in chunks of RSG_SLOT6 entries taken from a pool
 // and chained per particle (Chains); a particle whose chunk the pool could
 // not give is flagged (Chains::redo) and MODE 1 fills its CSR list with a
 // second search.
-#define RSG_REACH6 2.0f
+#define RSG_REACH6 6.0f
 #define RSG_STK6G 512
 #define RSG_SLOT6 32
 struct Chains {
@@ -1003,9 +1004,17 @@ __global__ void __launch_bounds__(128) k_fof6_w(const KNode<6> *nodes, const Rec
                 }
             }
             sp += total2;
-            // the points after imin of the leaves before the first node to descend
+            // the leaves before the first node to descend, by the lanes' own box
+            // tests: the run's box has room for nodes that no particle reaches
+            unsigned lm = __ballot_sync(FULL, kind == 1 && lane < f);
+            for (unsigned todo = lm; todo; todo &= todo - 1) {
+                const int b = __ffs(todo) - 1;
+                const int xb = __shfl_sync(FULL, xi, b);
+                if (!__any_sync(FULL, mine && box_near6(nodes + xb, c) < r2)) lm &= ~(1u << b);
+            }
+            // their points after imin
             const int a0 = max(s0, imin + 1);
-            const int pn = kind == 1 && lane < f ? max(0, s0 + m0 - a0) : 0;
+            const int pn = (lm >> lane) & 1u ? max(0, s0 + m0 - a0) : 0;
             int incl = pn;
 #pragma unroll
             for (int q = 1; q < 32; q <<= 1) {
