@@ -524,96 +524,128 @@ __device__ __forceinline__ float box_near6(const KNode<6> *nd, const float *c) {
 // 2015), so a point or node left out, its square at or above r * r, could not
 // have lowered r, and the result is the rounded root of the least square over
 // the own node (0 excepted) and every other point.
-// So the walk here climbs from the own node, where the near points are, and
-// takes each sibling on the way nearest child first, with both children
-// tested at their parent; the distance stays squared.  Each lane walks on to
-// its next leaf, then the lanes holding a leaf test their leaves together.
+// So the walk here climbs from the own node, where the near points are, with
+// the distances kept squared, and RSG_NN_G lanes share a query: a lane per point of
+// a leaf, per child of the nodes opened (the eight nearest the top of the stack),
+// and per sibling on the way up.  The searches of a warp differ in length by
+// more than ten: with a lane per query 3.8 of 32 lanes were active, and the
+// last warps ran alone.  At 33.5M particles (11 levels) a lane per query took 53 ms, 4 lanes
+// 66, 8 lanes 41, 16 lanes 38.5 and 32 lanes 53 (more boxes tested than
+// pruned); at 262,144 particles 2.8, 2.0, 1.3, 1.06 and 1.26 ms.
+#define RSG_NN_G 16
+#define RSG_NN_T 128
+// entries of a query's stack: above RSG_NN_STK - RSG_STACK6 - G nodes are opened one by one,
+// which needs an entry per level
+#define RSG_NN_STK 192
+template <int G>
 __device__ float next_closest(const KNode<6> *nodes, int root, const Rec *W, const float *c,
-                              bool valid, int *err) {
+                              bool valid, int *S, float *D, int *err) {
     const unsigned FULL = 0xffffffffu;
-    int nd = root;
-    float best = 0.f;
-    int stack[RSG_STACK6];
-    float far[RSG_STACK6];
-    int sp = 0;
+    const int lane = threadIdx.x & 31, gl = lane & (G - 1), g0 = lane & ~(G - 1);
+    const unsigned gmask = 0xffffffffu >> (32 - G);
+    const float INF = __int_as_float(0x7f800000);
     const unsigned long long c2[3] = {f2_pack(c[0], c[1]), f2_pack(c[2], c[3]),
                                       f2_pack(c[4], c[5])};
-    if (valid) {
-        while (nodes[nd].div >= 0) {
-            const KNode<6> &x = nodes[nd];
-            nd = (c[x.div] <= nodes[x.left].mx[x.div]) ? x.left : x.left + 1;
-        }
-        while (nd != root) {
-            int pdv = nodes[nodes[nd].parent].div;
-            if (nodes[nd].mn[pdv] == nodes[nd].mx[pdv]) nd = nodes[nd].parent;
-            else break;
-        }
-        const KNode<6> &o = nodes[nd];
-        for (int j = 0; j < 6; j++) {
-            float dx = fsub(o.mx[j], o.mn[j]);
-            best = fadd(best, fmul(dx, dx));
-        }
-        for (int i = 0; i < o.n; i++) {
+    auto scan = [&](int s, int n, bool own, float best) {
+        for (int i = gl; i < n; i += G) {
             unsigned long long q2[3];
-            rec_pairs(W + o.start + i, q2);
-            float d = dist6_p(c2, q2);
-            if (d && d < best) best = d;
+            rec_pairs(W + s + i, q2);
+            const float d = dist6_p(c2, q2);
+            if (d < best && !(own && d == 0.f)) best = d;
         }
+        __syncwarp();
+#pragma unroll
+        for (int o = G / 2; o; o >>= 1) best = fminf(best, __shfl_xor_sync(FULL, best, o));
+        return best;
+    };
+    int nd = root, sp = 0;
+    float best = 0.f;
+    {
+        int s = 0, n = 0;
+        if (valid) {
+            while (nodes[nd].div >= 0) {
+                const KNode<6> &x = nodes[nd];
+                nd = (c[x.div] <= nodes[x.left].mx[x.div]) ? x.left : x.left + 1;
+            }
+            while (nd != root) {
+                int pdv = nodes[nodes[nd].parent].div;
+                if (nodes[nd].mn[pdv] == nodes[nd].mx[pdv]) nd = nodes[nd].parent;
+                else break;
+            }
+            const KNode<6> &o = nodes[nd];
+            for (int j = 0; j < 6; j++) {
+                float dx = fsub(o.mx[j], o.mn[j]);
+                best = fadd(best, fmul(dx, dx));
+            }
+            s = o.start;
+            n = o.n;
+        }
+        __syncwarp();
+        best = scan(s, n, true, best);
     }
-    bool go = valid;
+    bool go = valid;  // the same in a query's lanes, as are sp, nd and best
     while (__any_sync(FULL, go)) {
-        int leaf = -1;
-        while (go && leaf < 0) {
-            int ni;
-            if (sp > 0) {
-                if (far[--sp] >= best) continue;
-                ni = stack[sp];
-            } else {  // climb: the next sibling on the way to the root
-                if (nd == root) {
-                    go = false;
-                    break;
+        const bool climb = go && sp == 0;
+        if (__any_sync(FULL, climb)) {  // the next G siblings on the way to the root
+            int sib = -1;
+            float d = INF;
+            if (climb) {
+                if (nd == root) go = false;
+                for (int i = 0; i < G && nd != root; i++) {
+                    const int p = nodes[nd].parent, l = nodes[p].left;
+                    if (gl == i) sib = l == nd ? l + 1 : l;
+                    nd = p;
                 }
-                const int p = nodes[nd].parent, l = nodes[p].left;
-                ni = l == nd ? l + 1 : l;
-                nd = p;
-                if (box_near6(nodes + ni, c) >= best) continue;
+                if (sib >= 0) d = box_near6(nodes + sib, c);
             }
-            for (;;) {
-                const int4 t = reinterpret_cast<const int4 *>(nodes + ni)[3];
-                if (t.z < 0) {  // div
-                    leaf = ni;
-                    break;
-                }
-                int a = t.w, b = t.w + 1;
-                float da = box_near6(nodes + a, c), db = box_near6(nodes + b, c);
-                if (db < da) {
-                    a = t.w + 1;
-                    b = t.w;
-                    const float w = da;
-                    da = db;
-                    db = w;
-                }
-                if (da >= best) break;
-                if (db < best) {
-                    if (sp >= RSG_STACK6) {
-                        atomicExch(err, 1);
-                        go = false;
-                        break;
-                    }
-                    stack[sp] = b;
-                    far[sp++] = db;
-                }
-                ni = a;
+            __syncwarp();
+            const unsigned b = (__ballot_sync(FULL, d < best) >> g0) & gmask;
+            if (d < best) {
+                const int q = __popc(b >> gl >> 1);  // the lowest sibling on top
+                S[q] = sib;
+                D[q] = d;
             }
+            if (climb) sp = __popc(b);
+            __syncwarp();
         }
-        if (leaf >= 0) {
-            const int s = nodes[leaf].start, n = nodes[leaf].n;
-            for (int i = 0; i < n; i++) {
-                unsigned long long q2[3];
-                rec_pairs(W + s + i, q2);
-                const float d = dist6_p(c2, q2);
-                if (d < best) best = d;
+        // open the top entries, a lane per child
+        const int take = (sp + G <= RSG_NN_STK - RSG_STACK6) ? min(sp, G / 2) : min(sp, 1);
+        const int pr = gl >> 1;
+        float far = INF, dc = INF;
+        int4 t = make_int4(0, 0, -1, 0);
+        if (pr < take) far = D[sp - 1 - pr];
+        const bool act = far < best;
+        if (act) {
+            t = reinterpret_cast<const int4 *>(nodes + S[sp - 1 - pr])[3];
+            if (t.z >= 0) dc = box_near6(nodes + t.w + (gl & 1), c);
+        }
+        sp -= take;
+        __syncwarp();
+        const float od = __shfl_xor_sync(FULL, dc, 1);
+        const unsigned b = (__ballot_sync(FULL, dc < best) >> g0) & gmask;
+        const int add = __popc(b);
+        if (sp + add > RSG_NN_STK) {
+            atomicExch(err, 1);
+            go = false;
+            sp = 0;
+        } else {
+            if (dc < best) {  // nearest child on top, the pairs in their order
+                const bool top = od < best && (dc < od || (dc == od && !(gl & 1)));
+                const int q = sp + __popc(b >> (2 * pr + 1) >> 1) + top;
+                S[q] = t.w + (gl & 1);
+                D[q] = dc;
             }
+            sp += add;
+        }
+        __syncwarp();
+        // the leaves among them, one after the other, a lane per point
+        unsigned lb = (__ballot_sync(FULL, act && t.z < 0 && !(gl & 1)) >> g0) & gmask;
+        while (__any_sync(FULL, lb != 0)) {
+            const int src = g0 + (lb ? __ffs(lb) - 1 : 0);
+            const int s = __shfl_sync(FULL, t.x, src), n = __shfl_sync(FULL, t.y, src);
+            const float fd = __shfl_sync(FULL, far, src);
+            best = scan(s, lb && fd < best ? n : 0, false, best);
+            lb &= lb - 1;
         }
     }
     return sqrt_fd(best);
@@ -642,10 +674,14 @@ __global__ void k_nn_keys(HierNodes N, int32_t base, int32_t count, const int32_
 }
 // The next-closest distance of every sample, queries taken in `order`
 // (sample indices; null: as stored), results stored by sample index.
-__global__ void k_nn(const KNode<6> *nodes, const Rec *W, HierNodes N, int32_t base,
-                     int32_t count, const int32_t *soff, const int32_t *sidx, float *prad,
-                     int64_t total, int exact, int *err, const uint32_t *order) {
-    int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(RSG_NN_T)
+    k_nn(const KNode<6> *nodes, const Rec *W, HierNodes N, int32_t base, int32_t count,
+         const int32_t *soff, const int32_t *sidx, float *prad, int64_t total, int exact, int *err,
+         const uint32_t *order) {
+    __shared__ int stk[RSG_NN_T / RSG_NN_G][RSG_NN_STK];
+    __shared__ float far[RSG_NN_T / RSG_NN_G][RSG_NN_STK];
+    const int w = threadIdx.x / RSG_NN_G;
+    int64_t q = blockIdx.x * (int64_t)(RSG_NN_T / RSG_NN_G) + w;
     // lanes past the end stay (next_closest synchronises the warp)
     const bool valid = q < total;
     if (!valid) q = total - 1;
@@ -666,8 +702,9 @@ __global__ void k_nn(const KNode<6> *nodes, const Rec *W, HierNodes N, int32_t b
     float c[6];
 #pragma unroll
     for (int d = 0; d < 6; d++) c[d] = W[s + j].pos[d];
-    const float rr = next_closest(nodes, k, W, c, valid, err);
-    if (valid) prad[g] = rr;
+    __syncwarp();
+    const float rr = next_closest<RSG_NN_G>(nodes, k, W, c, valid, stk[w], far[w], err);
+    if (valid && threadIdx.x % RSG_NN_G == 0) prad[g] = rr;
 }
 
 // find_median_r / rad_partition (src/groupies.c:735-786), run as is on the
@@ -2745,7 +2782,7 @@ SubsOut find_subs_device(Arena &ar, rsg_particle *d_p, int64_t num_p, const int6
                 while (bits < 64 && ((int64_t)1 << (bits - 32)) < cnt) bits++;
                 sort_pairs(ar, k1, k2, v1, order, tot, bits, st);
             }
-            launch(k_nn, nblk(tot, 128), 128, 0, st, F.nodes, W, N, base, cnt, soff, sidx, prad,
+            launch(k_nn, nblk((int64_t)tot * RSG_NN_G, RSG_NN_T), RSG_NN_T, 0, st, F.nodes, W, N, base, cnt, soff, sidx, prad,
                    (int64_t)tot, (int)cfg.exact_ll_calc, err, (const uint32_t *)order);
             ar.used = m0;
         }
