@@ -49,6 +49,12 @@ __device__ __forceinline__ float dist3_p(unsigned long long cxy, float cz, const
     const float dz = fsub(cz, q.pos[2]);
     return fadd(fadd(p0, p1), fmul(dz, dz));
 }
+__device__ __forceinline__ float dist3_q(unsigned long long cxy, float cz, const float4 &q) {
+    float p0, p1;
+    f2_split(f2_sqr(f2_sub(cxy, f2_pack(q.x, q.y))), p0, p1);
+    const float dz = fsub(cz, q.z);
+    return fadd(fadd(p0, p1), fmul(dz, dz));
+}
 // The reference's two box tests, in its operation order:
 // _fast3tree_box_not_intersect_sphere and _fast3tree_box_inside_sphere
 // (src/fast3tree.c:293-330).
@@ -340,17 +346,39 @@ __device__ __forceinline__ bool warp_query(const int *list, int nq, int *q) {
 __device__ __forceinline__ bool warp_idle(int nq) {
     return (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u) >= nq;
 }
-// |S_r(i)| capped at 17 (the reference only asks whether it exceeds 16)
-__global__ void __launch_bounds__(128) k_count_w(const KNode<3> *nodes, const Rec *recs, int n,
-                                                 float r, uint8_t *cnt, int *err) {
+// |S_r(i)| capped at 17 (the reference only asks whether it exceeds 16).
+// Half the particles of a volume are dense, and most of those have 17 of
+// their neighbours in the sphere among the RSG_CNT_WIN particles on either
+// side of them in tree order, so these are tried first, from shared memory: a
+// point nearer than r is in S_r by whichever way the walk meets it (no box that
+// holds it is out, its offsets being no more than the point's).  The lanes left
+// walk the tree from the root.  The walk is what the kernel waits for (83% of the issue
+// slots, 18 lanes active): 17.6 -> 10.2 ms at 33.5M particles, 4.45 -> 2.64 at
+// 8.4M, 3.9 -> 1.8 on the cluster; the window costs at most 65 tests a lane.
+#define RSG_CNT_T 128
+#define RSG_CNT_WIN 32
+__global__ void __launch_bounds__(RSG_CNT_T) k_count_w(const KNode<3> *nodes, const Rec *recs,
+                                                       int n, float r, uint8_t *cnt, int *err) {
+    __shared__ float4 tile[RSG_CNT_T + 2 * RSG_CNT_WIN];
+    const int b0 = blockIdx.x * RSG_CNT_T - RSG_CNT_WIN;
+    const float INF = __int_as_float(0x7f800000);
+    for (int e = threadIdx.x; e < RSG_CNT_T + 2 * RSG_CNT_WIN; e += RSG_CNT_T)
+        tile[e] = b0 + e >= 0 && b0 + e < n ? *reinterpret_cast<const float4 *>(recs + b0 + e)
+                                            : make_float4(INF, INF, INF, 0.f);
+    __syncthreads();
     if (warp_idle(n)) return;
     int i;
-    bool act = warp_query(nullptr, n, &i);
-    float c[3] = {0, 0, 0};
-    if (act) { c[0] = recs[i].pos[0]; c[1] = recs[i].pos[1]; c[2] = recs[i].pos[2]; }
-    int k = 0;
+    const bool act = warp_query(nullptr, n, &i);
+    const float4 q = tile[threadIdx.x + RSG_CNT_WIN];
+    const float c[3] = {q.x, q.y, q.z}, r2 = fmul(r, r);
+    const unsigned long long cxy = f2_pack(c[0], c[1]);
+    int k = act ? 0 : 17;
+    for (int e = 0; e <= 2 * RSG_CNT_WIN && __any_sync(0xffffffffu, k < 17); e++)
+        k += dist3_q(cxy, c[2], tile[threadIdx.x + e]) < r2;
+    const bool walk = k < 17;
+    if (walk) k = 0;
     sphere3_warp(
-        nodes, recs, c, act, r, -1, err,
+        nodes, recs, c, walk, r, -1, err,
         [&](int s, int m) { k += m; return k <= 16; },
         [&](int j) { k++; return k <= 16; });
     if (act) cnt[i] = (uint8_t)(k > 17 ? 17 : k);
@@ -1448,8 +1476,7 @@ FofOut fof3d_device(Arena &ar, const rsg_particle *d_in, int64_t n64, const rsg_
 
     uint8_t *cnt = ar.get<uint8_t>(n);
     phase_mark(st, "fof.tree3d");
-    const int TW = 128;
-    launch(k_count_w, nblk(n, TW), TW, 0, st, F.nodes, recs, n, r, cnt, err);
+    launch(k_count_w, nblk(n, RSG_CNT_T), RSG_CNT_T, 0, st, F.nodes, recs, n, r, cnt, err);
     phase_mark(st, "fof.count");
     // dense particles (more than 16 neighbours), in tree order
     int *dense = ar.get<int>(n);
