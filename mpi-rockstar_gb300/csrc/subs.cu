@@ -1380,6 +1380,30 @@ __device__ __forceinline__ float asc_x(const AscHalo &h, const float *pos) {
     float b = __fdiv_rn(v2, fmul(h.vrms, h.vrms));
     return fadd(a, b);
 }
+// asc_x below `cut`, without its two divisions when one of the two terms alone
+// reaches cut: r2 >= cut * r^2 rounded up gives a quotient of at least cut, and the
+// other term, not negative, does not lower the sum.  The assignment's scans are bound
+// by their instructions: 15.9 -> 11.8 ms on the
+// cluster of 5M particles, 8.8 -> 6.7 at 33.5M.
+__device__ __forceinline__ bool asc_below(const AscHalo &h, const float *pos, float cut,
+                                          float *x) {
+    float r2 = 0.f, v2 = 0.f;
+    const float rr = fmul(h.r, h.r), vv = fmul(h.vrms, h.vrms);
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        float dx = fsub(h.pos[i], pos[i]);
+        r2 = fadd(r2, fmul(dx, dx));
+    }
+    if (r2 >= __fmul_ru(cut, rr)) return false;
+#pragma unroll
+    for (int i = 3; i < 6; i++) {
+        float dx = fsub(h.pos[i], pos[i]);
+        v2 = fadd(v2, fmul(dx, dx));
+    }
+    if (v2 >= __fmul_ru(cut, vv)) return false;
+    *x = fadd(__fdiv_rn(r2, rr), __fdiv_rn(v2, vv));
+    return !(*x >= cut);
+}
 // Buckets of 32 consecutive candidates (k_asc_buckets_s) for nodes with more
 // than Tuning::asc_bucket_min (bmin) of them: the box of their centres and the largest
 // radius over the valid ones (inv: the bucket holds an invalid halo).  For a
@@ -1390,7 +1414,7 @@ struct AscBucket {
     int32_t inv;  // holds a halo without a valid metric
 };
 // lower bound of x over a bucket's valid halos
-__device__ __forceinline__ float asc_bucket_lb(const AscBucket &B, const float *pos) {
+__device__ __forceinline__ float asc_bucket_d2(const AscBucket &B, const float *pos) {
     float d2 = 0.f;
 #pragma unroll
     for (int i = 0; i < 3; i++) {
@@ -1399,7 +1423,14 @@ __device__ __forceinline__ float asc_bucket_lb(const AscBucket &B, const float *
         else if (pos[i] > B.mx[i]) gap = fsub(pos[i], B.mx[i]);
         d2 = fadd(d2, fmul(gap, gap));
     }
-    return __fdiv_rn(d2, fmul(B.rmax, B.rmax));
+    return d2;
+}
+__device__ __forceinline__ float asc_bucket_lb(const AscBucket &B, const float *pos) {
+    return __fdiv_rn(asc_bucket_d2(B, pos), fmul(B.rmax, B.rmax));
+}
+// The lower bound reaches cut (undivided, as in asc_below).
+__device__ __forceinline__ bool asc_bucket_out(const AscBucket &B, const float *pos, float cut) {
+    return asc_bucket_d2(B, pos) >= __fmul_ru(cut, fmul(B.rmax, B.rmax));
 }
 // Nodes with more than bmin growing halos also get their halos in
 // Morton order of position (within the node's box of halo centres), so that
@@ -1620,14 +1651,14 @@ __global__ void k_asc_assign_p(const Rec *W, int64_t M, const int32_t *eln, Hier
         for (int j = 0; j < ng;) {
             if ((j & 1023) == 0) {
                 const AscBucket &S = bk2[h0 + (j >> 10)];
-                if ((!S.inv || best < 1e20f) && asc_bucket_lb(S, pos) >= cut) {
+                if ((!S.inv || best < 1e20f) && asc_bucket_out(S, pos, cut)) {
                     j += 1024;
                     continue;
                 }
             }
             if ((j & 31) == 0) {
                 const AscBucket &B = bk[h0 + (j >> 5)];
-                if ((!B.inv || best < 1e20f) && asc_bucket_lb(B, pos) >= cut) {
+                if ((!B.inv || best < 1e20f) && asc_bucket_out(B, pos, cut)) {
                     j += 32;
                     continue;
                 }
@@ -1637,8 +1668,8 @@ __global__ void k_asc_assign_p(const Rec *W, int64_t M, const int32_t *eln, Hier
             if (!asc_valid(c)) {
                 m = 1e20f;
             } else {
-                float x = asc_x(c, pos);
-                if (x >= cut) {
+                float x;
+                if (!asc_below(c, pos, cut, &x)) {
                     j++;
                     continue;
                 }
