@@ -58,16 +58,10 @@ ALGO_BYTES = {
     "k_basic_props": lambda st, L: 48.0 * st["items_6d"] / max(L, 1),
     # norm_sd: positions read and written back
     "k_norm_par": lambda st, L: 48.0 * st["items_6d"] / max(L, 1),
-    "k_norm_warp": lambda st, L: 48.0 * st["items_6d"] / max(L, 1),
     # next-closest search: sample position read, distance written
     "k_nn": lambda st, L: 28.0 * st["samples_6d"] / max(L, 1),
     # median selection: every sample distance read once
     "k_target_par": lambda st, L: 4.0 * st["samples_6d"] / max(L, 1),
-    # later-dense lists: positions of the dense particles in both launches,
-    # every entry (one per dense pair) written once
-    "k_llist_w": lambda st, L: (32.0 * st["dense"] + 4.0 * st["dense_pairs"]) / max(L, 1),
-    # seed frontiers: every list entry read, its pending count updated
-    "k_kahn": lambda st, L: 12.0 * st["dense_pairs"] / max(L, 1),
     # potentials: record read (48 B), potential written (8 B)
     "k_bh_walk": lambda st, L: 56.0 * st["pot_records"] / max(L, 1),
     # property scans: record read, kinetic energy written
@@ -80,7 +74,7 @@ ALGO_BYTES = {
 # dram__bytes_write.sum of the captured launch over the units it processed),
 # scaled to the timed launches by their units
 NCU_TRAFFIC = {
-    "k_fof6_w": ((137.976064e6 + 95.008e6) / 2309888.0, "items_6d",
+    "k_fof6_w": ((142.594048e6 + 132.396032e6) / 2309888.0, "items_6d",
                  "one ncu capture of the level-0 launch on workload 4 at 1/32 scale, "
                  "scaled by particles"),
 }
@@ -89,11 +83,8 @@ NCU_TRAFFIC = {
 # a tree walk their product -- the share of the SM's lane-issue capacity
 # doing work -- says more than an HBM fraction.
 NCU_ISSUE = {
-    "k_fof6_w": (0.774138, 27.75),
-    "k_nn": (0.662851, 4.62),
-    "k_bh_walk": (0.698618, 19.11),
-    "k_llist_w": (0.642338, 14.73),
-    "k_kahn": (0.219013, 27.52),
+    "k_fof6_w": (0.647406, 29.52),
+    "k_nn": (0.687077, 23.33),
 }
 NCU_ISSUE_SOURCE = "ncu, workload 4 at 1/32 scale, one launch per kernel"
 
