@@ -1833,24 +1833,27 @@ __device__ __forceinline__ int vmax_bin(float ds, float rsc) {
                                                   : (int64_t)bf;
     return (b < 50) ? (int)b : -1;
 }
-// Vmax and Rvmax from the 50-bin mass histogram (src/properties.c:39-69), then
-// the final radius and vrms of calc_basic_halo_props.
-__device__ void basic_vmax(rsg_halo &hh, const int *bins, int do_bins, float rsc_s,
-                           const DevCfg *C) {
+// Vmax and Rvmax from the 50-bin mass histogram (src/properties.c:39-69): the
+// largest of the bins' mass over radius, then the fields, and the final radius
+// and vrms of calc_basic_halo_props.
+__device__ float vmax_peak(const int *bins, float rsc, const DevCfg *C) {
+    float vm = 0.f;
+    int64_t tp = 0;
+    for (int i = 0; i < 50; i++) {
+        // (float)((i + 1.0) / (double)rsc), src/properties.c:58, as one FP32
+        // division: the exact quotient of a small integer by a float lies
+        // either on a float rounding midpoint or more than 2^-48 (relative)
+        // from every one, so the FP64 quotient rounds to the same float
+        float r = __fdiv_rn((float)(i + 1), rsc);
+        if ((double)r < C->force_res) r = (float)C->force_res;
+        tp += bins[i];
+        float vc = __fdiv_rn(__ll2float_rn(tp), r);
+        if (vc > vm) vm = vc;
+    }
+    return vm;
+}
+__device__ void basic_vmax(rsg_halo &hh, float vm, int do_bins, const DevCfg *C) {
     if (do_bins) {
-        float rsc = rsc_s, vm = 0.f;
-        int64_t tp = 0;
-        for (int i = 0; i < 50; i++) {
-            // (float)((i + 1.0) / (double)rsc), src/properties.c:58, as one FP32
-            // division: the exact quotient of a small integer by a float lies
-            // either on a float rounding midpoint or more than 2^-48 (relative)
-            // from every one, so the FP64 quotient rounds to the same float
-            float r = __fdiv_rn((float)(i + 1), rsc);
-            if ((double)r < C->force_res) r = (float)C->force_res;
-            tp += bins[i];
-            float vc = __fdiv_rn(__ll2float_rn(tp), r);
-            if (vc > vm) vm = vc;
-        }
         float sn = (float)C->scale_now;
         float v = (float)sqrt(RSG_GC * (double)vm * C->particle_mass / (double)sn);
         hh.vmax = v;
@@ -1858,6 +1861,82 @@ __device__ void basic_vmax(rsg_halo &hh, const int *bins, int do_bins, float rsc
     }
     if (hh.vmax_r) hh.r = hh.vmax_r;
     hh.vrms = sqrt_fd(hh.vrms);
+}
+
+// basic_decide and basic_vmax by a whole warp: the FP64 divisions, cube roots and
+// bins that do not depend on one another go one to a lane.  On one lane a halo's
+// decisions are some 400 FP64 instructions, each holding the pipe as long as one of
+// 32 lanes, and a small halo's sums are less: k_basic_props_w 14.7 -> 7.9 ms at 33.5M
+// particles, 2.3 -> 1.3 on 6,000 groups; k_basic_props, bound by its sums, 7.6 -> 7.0.
+// Lane d < 6 brings coordinate d's mean and summed squared deviations.
+__device__ void basic_decide_w(rsg_halo &hh, double mean, double p2, int np, const DevCfg *C,
+                               int *do_bins, float *rsc_out) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const double q = p2 / (double)np;
+    const int64_t num = hh.num_p, nch = hh.num_child_particles ? hh.num_child_particles : num;
+    const float rad = (float)cbrt((double)(lane == 1 ? nch : num) /
+                                  ((4.0 * M_PI / 3.0) * C->rvir_dens));
+    float r = 0, vr = 0;
+#pragma unroll
+    for (int k = 0; k < 3; k++) r = (float)((double)r + __shfl_sync(FULL, q, k));
+#pragma unroll
+    for (int k = 3; k < 6; k++) vr = (float)((double)vr + __shfl_sync(FULL, q, k));
+    const double e = (double)(lane == 1 ? vr : r) / (double)np;
+    const double pe = __shfl_sync(FULL, e, 0), ve = __shfl_sync(FULL, e, 1);
+    const bool at = (!hh.min_pos_err) || ((double)hh.min_pos_err > pe);
+    const bool av = (!hh.min_vel_err) || ((double)hh.min_vel_err > ve);
+    const float hr = __shfl_sync(FULL, rad, 0), cr = __shfl_sync(FULL, rad, 1);
+    __syncwarp();  // the reads above before the writes
+    if (lane < 3) {
+        if (at) hh.pos[lane] = (float)mean;
+    } else if (lane < 6) {
+        if (av) hh.pos[lane] = (float)mean;
+        hh.bulkvel[lane - 3] = (float)mean;
+    }
+    if (lane == 0) {
+        if (at) {
+            hh.min_pos_err = (float)pe;
+            hh.n_core = num;
+        }
+        if (av) hh.min_vel_err = (float)ve;
+        hh.m = (float)num;
+        hh.num_child_particles = nch;
+        hh.r = hr;
+        hh.vrms = vr;
+        hh.child_r = cr;
+        hh.vmax = hh.vmax_r = 0;
+    }
+    __syncwarp();
+    *do_bins = cr > 0;
+    *rsc_out = (float)(50.0 / (double)cr);
+}
+// The warp's form of the loop over the bins; the largest of 50 values does not
+// depend on the order.
+__device__ float vmax_peak_w(const int *bins, float rsc, const DevCfg *C) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    float vm = 0.f;
+    int before = 0;
+#pragma unroll
+    for (int b = 0; b < 64; b += 32) {
+        const int i = b + lane;
+        int tp = i < 50 ? bins[i] : 0;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(FULL, tp, o);
+            if (lane >= o) tp += v;
+        }
+        tp += before;
+        before = __shfl_sync(FULL, tp, 31);
+        float r = __fdiv_rn((float)(i + 1), rsc);
+        if ((double)r < C->force_res) r = (float)C->force_res;
+        const float vc = __fdiv_rn(__int2float_rn(tp), r);
+        if (i < 50 && vc > vm) vm = vc;
+    }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) vm = fmaxf(vm, __shfl_xor_sync(FULL, vm, o));
+    return vm;
 }
 
 // calc_basic_halo_props + estimate_vmax (src/properties.c:39-125); one
@@ -1933,12 +2012,15 @@ __global__ void k_basic_props(const Rec *W, rsg_halo *H, const int32_t *list, co
     __shared__ float rsc_s;
     __shared__ int do_bins;
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (threadIdx.x < 32) {
+        const int d = min((int)threadIdx.x, 5);
         int db;
         float rs;
-        basic_decide(hh, mean, p2, np, C, &db, &rs);
-        do_bins = db;
-        rsc_s = rs;
+        basic_decide_w(hh, mean[d], p2[d], np, C, &db, &rs);
+        if (threadIdx.x == 0) {
+            do_bins = db;
+            rsc_s = rs;
+        }
     }
     __syncthreads();
     if (do_bins) {
@@ -1957,7 +2039,10 @@ __global__ void k_basic_props(const Rec *W, rsg_halo *H, const int32_t *list, co
         }
     }
     __syncthreads();
-    if (threadIdx.x == 0) basic_vmax(hh, bins, do_bins, rsc_s, C);
+    if (threadIdx.x < 32) {
+        const float vm = do_bins ? vmax_peak_w(bins, rsc_s, C) : 0.f;
+        if (threadIdx.x == 0) basic_vmax(hh, vm, do_bins, C);
+    }
 }
 
 // Batched form, halos of at most RSG_BP_WARP particles: the same steps with
@@ -1965,7 +2050,7 @@ __global__ void k_basic_props(const Rec *W, rsg_halo *H, const int32_t *list, co
 // its threads idle and spends its time in barriers).  Each lane sums in
 // double-float on the FP32 pipe (df64.cuh; the FP64 pipe bound the FP64
 // form), the lanes' sums are added in FP64 (the batched form's sums are not
-// in the reference's order anyway); lane 0 takes the decisions.
+// in the reference's order anyway).
 #define RSG_BP_WARP 1024
 __global__ void __launch_bounds__(256) k_basic_props_w(const Rec *W, rsg_halo *H,
                                                        const int32_t *list, int32_t nl,
@@ -1978,7 +2063,7 @@ __global__ void __launch_bounds__(256) k_basic_props_w(const Rec *W, rsg_halo *H
     const int ps = (int)hh.p_start, np = (int)hh.num_p;
     if (np > RSG_BP_WARP) return;  // the block kernel's
     DF acc[6];
-    double mean[6], p2[6];
+    double mean = 0, p2 = 0;  // lane d's: coordinate d's
 #pragma unroll
     for (int d = 0; d < 6; d++) acc[d] = DF{0.f, 0.f};
     for (int i = lane; i < np; i += 32)
@@ -1987,25 +2072,29 @@ __global__ void __launch_bounds__(256) k_basic_props_w(const Rec *W, rsg_halo *H
     DF md[6];
 #pragma unroll
     for (int d = 0; d < 6; d++) {
-        // warp_sum_d leaves the total in lane 0; every lane needs the mean
-        mean[d] = __shfl_sync(0xffffffffu, warp_sum_d(df_to_double(acc[d])), 0) / (double)np;
-        md[d] = df_from_double(mean[d]);
+        // warp_sum_d leaves the total in lane 0
+        const double t = __shfl_sync(0xffffffffu, warp_sum_d(df_to_double(acc[d])), 0);
+        if (lane == d) mean = t;
         acc[d] = DF{0.f, 0.f};
     }
+    mean /= (double)np;
+#pragma unroll
+    for (int d = 0; d < 6; d++) md[d] = df_from_double(__shfl_sync(0xffffffffu, mean, d));
     for (int i = lane; i < np; i += 32)
 #pragma unroll
         for (int d = 0; d < 6; d++)
             acc[d] = df_add(acc[d], df_sqr(df_sub_from_f(W[ps + i].pos[d], md[d])));
 #pragma unroll
-    for (int d = 0; d < 6; d++) p2[d] = warp_sum_d(df_to_double(acc[d]));  // lane 0's are used
-    int db = 0;
-    float rs = 0.f;
-    if (lane == 0) basic_decide(hh, mean, p2, np, C, &db, &rs);
-    db = __shfl_sync(0xffffffffu, db, 0);
-    rs = __shfl_sync(0xffffffffu, rs, 0);
+    for (int d = 0; d < 6; d++) {
+        const double t = __shfl_sync(0xffffffffu, warp_sum_d(df_to_double(acc[d])), 0);
+        if (lane == d) p2 = t;
+    }
+    int db;
+    float rs;
+    basic_decide_w(hh, mean, p2, np, C, &db, &rs);
     int *bins = bins_s[w];
     for (int k = lane; k < 50; k += 32) bins[k] = 0;
-    __syncwarp();  // also orders lane 0's halo writes before the reads below
+    __syncwarp();
     if (db) {
         const float c0 = hh.pos[0], c1 = hh.pos[1], c2 = hh.pos[2];
         for (int i = lane; i < np; i += 32) {
@@ -2018,7 +2107,8 @@ __global__ void __launch_bounds__(256) k_basic_props_w(const Rec *W, rsg_halo *H
         }
     }
     __syncwarp();
-    if (lane == 0) basic_vmax(hh, bins, db, rs, C);
+    const float vm = db ? vmax_peak_w(bins, rs, C) : 0.f;
+    if (lane == 0) basic_vmax(hh, vm, db, C);
 }
 
 // Batched form, halos above Tuning::bp_big particles: calc_basic_halo_props
@@ -2125,7 +2215,7 @@ __global__ void k_bp_vmax(rsg_halo *H, const int32_t *list, int32_t nl, const in
     for (int b = 0; b < 50; b++) bins[b] = 0;
     for (int c = c0[t]; c < c0[t] + nch[t]; c++)
         for (int b = 0; b < 50; b++) bins[b] += P[c].bins[b];
-    basic_vmax(H[list[t]], bins, dob[t], rsc[t], C);
+    basic_vmax(H[list[t]], dob[t] ? vmax_peak(bins, rsc[t], C) : 0.f, dob[t], C);
 }
 
 // growing-halo list of a level: node glist entries concatenated
