@@ -1939,109 +1939,155 @@ __device__ float vmax_peak_w(const int *bins, float rsc, const DevCfg *C) {
     return vm;
 }
 
+// Batched form, halos of RSG_BP_WARP to Tuning::bp_big particles: their list, and
+// their means and summed squared deviations, a block per halo and coordinate.  The
+// FP64 pipe bounds these sums; a level has few such halos, and with all six
+// coordinates on one block its SM was the launch's time (with the decisions 76 us at
+// 262,144 particles and 139 on 6,000 groups, now 47 and 70; over 33.5M 7.0 -> 5.3 ms).
+__global__ void k_bp_mid(const rsg_halo *H, const int32_t *list, int32_t nl, int big, int small,
+                         int32_t *mid, int *nmid) {
+    int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= nl) return;
+    const int64_t np = H[list[t]].num_p;
+    if (np > small && np <= big) mid[atomicAdd(nmid, 1)] = list[t];
+}
+__global__ void __launch_bounds__(256) k_bp_dims(const Rec *W, const rsg_halo *H,
+                                                 const int32_t *mid, const int *nmid,
+                                                 double2 *sums) {
+    __shared__ double sm[40];
+    __shared__ double mean_s;
+    for (int e = blockIdx.x; e < 6 * *nmid; e += gridDim.x) {
+        const rsg_halo &hh = H[mid[e / 6]];
+        const int d = e % 6, ps = (int)hh.p_start, np = (int)hh.num_p;
+        double a = 0;
+        for (int i = threadIdx.x; i < np; i += blockDim.x) a += (double)W[ps + i].pos[d];
+        double t = block_sum_d(a, sm);
+        if (threadIdx.x == 0) mean_s = t / (double)np;
+        __syncthreads();
+        const double mean = mean_s;
+        a = 0;
+        for (int i = threadIdx.x; i < np; i += blockDim.x) {
+            double x = (double)W[ps + i].pos[d] - mean;
+            a += x * x;
+        }
+        t = block_sum_d(a, sm);
+        if (threadIdx.x == 0) sums[e] = make_double2(mean, t);
+        __syncthreads();
+    }
+}
 // calc_basic_halo_props + estimate_vmax (src/properties.c:39-125); one
-// block per listed halo.
-__global__ void k_basic_props(const Rec *W, rsg_halo *H, const int32_t *list, const DevCfg *C,
-                              int seq_max, int big, int small) {
+// block per listed halo (the batched form's medium ones: MID, sums by
+// k_bp_dims; all of the plain form's).  Halos emptied by the assignment
+// (num_p 0) are still processed, as the reference processes them.
+template <bool MID>
+__global__ void k_basic_props(const Rec *W, rsg_halo *H, const int32_t *list, const int *nlist,
+                              const DevCfg *C, int seq_max, const double2 *sums) {
     __shared__ double sm[40];
     __shared__ double mean[6], p2[6];
     __shared__ int bins[50];
-    int h = list[blockIdx.x];
-    rsg_halo &hh = H[h];
-    int ps = (int)hh.p_start, np = (int)hh.num_p;
-    // chunked and warp paths (batched form); halos emptied by the assignment
-    // (num_p 0) are still processed, as the reference processes them
-    if (np > big || np <= small) return;
-    if (np <= seq_max) {
-        // in array order (src/properties.c:76-87): the block stages values,
-        // thread 0 adds them
-        __shared__ double stage[256][6];
-        double a = 0, b = 0;  // lane d of warp 0 owns coordinate d
-        for (int b0 = 0; b0 < np; b0 += blockDim.x) {
-            int i = b0 + threadIdx.x;
-            if (i < np)
-                for (int d = 0; d < 6; d++) stage[threadIdx.x][d] = (double)W[ps + i].pos[d];
-            __syncthreads();
+    for (int e = blockIdx.x; e < (MID ? *nlist : (int)gridDim.x); e += gridDim.x) {
+        int h = list[e];
+        rsg_halo &hh = H[h];
+        int ps = (int)hh.p_start, np = (int)hh.num_p;
+        if (MID) {
             if (threadIdx.x < 6) {
-                int m = min((int)blockDim.x, np - b0), d = threadIdx.x;
-                for (int t = 0; t < m; t++) a += stage[t][d];
+                const double2 v = sums[6 * e + threadIdx.x];
+                mean[threadIdx.x] = v.x;
+                p2[threadIdx.x] = v.y;
+            }
+        } else if (np <= seq_max) {
+            // in array order (src/properties.c:76-87): the block stages values,
+            // thread 0 adds them
+            __shared__ double stage[256][6];
+            double a = 0, b = 0;  // lane d of warp 0 owns coordinate d
+            for (int b0 = 0; b0 < np; b0 += blockDim.x) {
+                int i = b0 + threadIdx.x;
+                if (i < np)
+                    for (int d = 0; d < 6; d++) stage[threadIdx.x][d] = (double)W[ps + i].pos[d];
+                __syncthreads();
+                if (threadIdx.x < 6) {
+                    int m = min((int)blockDim.x, np - b0), d = threadIdx.x;
+                    for (int t = 0; t < m; t++) a += stage[t][d];
+                }
+                __syncthreads();
+            }
+            if (threadIdx.x < 6) mean[threadIdx.x] = a / (double)np;
+            __syncthreads();
+            for (int b0 = 0; b0 < np; b0 += blockDim.x) {
+                int i = b0 + threadIdx.x;
+                if (i < np)
+                    for (int d = 0; d < 6; d++) {
+                        double x = (double)W[ps + i].pos[d] - mean[d];
+                        stage[threadIdx.x][d] = x * x;
+                    }
+                __syncthreads();
+                if (threadIdx.x < 6) {
+                    int m = min((int)blockDim.x, np - b0), d = threadIdx.x;
+                    for (int t = 0; t < m; t++) b += stage[t][d];
+                }
+                __syncthreads();
+            }
+            if (threadIdx.x < 6) p2[threadIdx.x] = b;
+            __syncthreads();
+        } else {
+            double acc[6] = {0, 0, 0, 0, 0, 0};
+            for (int i = threadIdx.x; i < np; i += blockDim.x)
+#pragma unroll
+                for (int d = 0; d < 6; d++) acc[d] += (double)W[ps + i].pos[d];
+            for (int d = 0; d < 6; d++) {
+                double t = block_sum_d(acc[d], sm);
+                if (threadIdx.x == 0) mean[d] = t / (double)np;
             }
             __syncthreads();
-        }
-        if (threadIdx.x < 6) mean[threadIdx.x] = a / (double)np;
-        __syncthreads();
-        for (int b0 = 0; b0 < np; b0 += blockDim.x) {
-            int i = b0 + threadIdx.x;
-            if (i < np)
+            for (int d = 0; d < 6; d++) acc[d] = 0;
+            for (int i = threadIdx.x; i < np; i += blockDim.x)
+#pragma unroll
                 for (int d = 0; d < 6; d++) {
                     double x = (double)W[ps + i].pos[d] - mean[d];
-                    stage[threadIdx.x][d] = x * x;
+                    acc[d] += x * x;
                 }
-            __syncthreads();
-            if (threadIdx.x < 6) {
-                int m = min((int)blockDim.x, np - b0), d = threadIdx.x;
-                for (int t = 0; t < m; t++) b += stage[t][d];
+            for (int d = 0; d < 6; d++) {
+                double t = block_sum_d(acc[d], sm);
+                if (threadIdx.x == 0) p2[d] = t;
             }
-            __syncthreads();
         }
-        if (threadIdx.x < 6) p2[threadIdx.x] = b;
+        if (threadIdx.x < 50) bins[threadIdx.x] = 0;
+        __shared__ float rsc_s;
+        __shared__ int do_bins;
         __syncthreads();
-    } else {
-    double acc[6] = {0, 0, 0, 0, 0, 0};
-    for (int i = threadIdx.x; i < np; i += blockDim.x)
-#pragma unroll
-        for (int d = 0; d < 6; d++) acc[d] += (double)W[ps + i].pos[d];
-    for (int d = 0; d < 6; d++) {
-        double t = block_sum_d(acc[d], sm);
-        if (threadIdx.x == 0) mean[d] = t / (double)np;
-    }
-    __syncthreads();
-    for (int d = 0; d < 6; d++) acc[d] = 0;
-    for (int i = threadIdx.x; i < np; i += blockDim.x)
-#pragma unroll
-        for (int d = 0; d < 6; d++) {
-            double x = (double)W[ps + i].pos[d] - mean[d];
-            acc[d] += x * x;
+        if (threadIdx.x < 32) {
+            const int d = min((int)threadIdx.x, 5);
+            int db;
+            float rs;
+            basic_decide_w(hh, mean[d], p2[d], np, C, &db, &rs);
+            if (threadIdx.x == 0) {
+                do_bins = db;
+                rsc_s = rs;
+            }
         }
-    for (int d = 0; d < 6; d++) {
-        double t = block_sum_d(acc[d], sm);
-        if (threadIdx.x == 0) p2[d] = t;
-    }
-    }
-    if (threadIdx.x < 50) bins[threadIdx.x] = 0;
-    __shared__ float rsc_s;
-    __shared__ int do_bins;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        const int d = min((int)threadIdx.x, 5);
-        int db;
-        float rs;
-        basic_decide_w(hh, mean[d], p2[d], np, C, &db, &rs);
-        if (threadIdx.x == 0) {
-            do_bins = db;
-            rsc_s = rs;
+        __syncthreads();
+        if (do_bins) {
+            float rsc = rsc_s;
+            float c0 = hh.pos[0], c1 = hh.pos[1], c2 = hh.pos[2];
+            for (int i = threadIdx.x; i < np; i += blockDim.x) {
+                float dx, ds = 0.f;
+                dx = fsub(c0, W[ps + i].pos[0]); ds = fadd(ds, fmul(dx, dx));
+                dx = fsub(c1, W[ps + i].pos[1]); ds = fadd(ds, fmul(dx, dx));
+                dx = fsub(c2, W[ps + i].pos[2]); ds = fadd(ds, fmul(dx, dx));
+                int key = vmax_bin(ds, rsc);
+                // lanes with the same bin add once (shared-memory atomics on 50 bins
+                // would otherwise serialise)
+                unsigned peers = __match_any_sync(__activemask(), key);
+                if (key >= 0 && (threadIdx.x & 31) == __ffs(peers) - 1)
+                    atomicAdd(&bins[key], __popc(peers));
+            }
         }
-    }
-    __syncthreads();
-    if (do_bins) {
-        float rsc = rsc_s;
-        float c0 = hh.pos[0], c1 = hh.pos[1], c2 = hh.pos[2];
-        for (int i = threadIdx.x; i < np; i += blockDim.x) {
-            float dx, ds = 0.f;
-            dx = fsub(c0, W[ps + i].pos[0]); ds = fadd(ds, fmul(dx, dx));
-            dx = fsub(c1, W[ps + i].pos[1]); ds = fadd(ds, fmul(dx, dx));
-            dx = fsub(c2, W[ps + i].pos[2]); ds = fadd(ds, fmul(dx, dx));
-            int key = vmax_bin(ds, rsc);
-            // lanes with the same bin add once (shared-memory atomics on 50 bins
-            // would otherwise serialise)
-            unsigned peers = __match_any_sync(__activemask(), key);
-            if (key >= 0 && (threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(&bins[key], __popc(peers));
+        __syncthreads();
+        if (threadIdx.x < 32) {
+            const float vm = do_bins ? vmax_peak_w(bins, rsc_s, C) : 0.f;
+            if (threadIdx.x == 0) basic_vmax(hh, vm, do_bins, C);
         }
-    }
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        const float vm = do_bins ? vmax_peak_w(bins, rsc_s, C) : 0.f;
-        if (threadIdx.x == 0) basic_vmax(hh, vm, do_bins, C);
+        __syncthreads();
     }
 }
 
@@ -2571,11 +2617,26 @@ static void basic_props(Arena &ar, const Rec *W, rsg_halo *H, const int32_t *lis
                         const DevCfg *d_dc, int seq_max, int exact, cudaStream_t st) {
     const int T = 256;
     if (nl <= 0) return;
-    launch(k_basic_props, nl, T, 0, st, W, H, list, d_dc, exact ? seq_max : 0,
-           exact ? 0x7fffffff : tuning().bp_big, exact ? -1 : RSG_BP_WARP);
-    if (exact) return;
-    launch(k_basic_props_w, nblk(nl, 8), 256, 0, st, W, H, list, nl, d_dc);
+    if (exact) {
+        launch(k_basic_props<false>, nl, T, 0, st, W, H, list, (const int *)nullptr, d_dc, seq_max,
+               (const double2 *)nullptr);
+        return;
+    }
     size_t mark = ar.used;
+    {
+        int32_t *mid = ar.get<int32_t>(nl);
+        int *nmid = ar.get<int>(1);
+        double2 *sums = ar.get<double2>((size_t)6 * nl);
+        RSG_CUDA(cudaMemsetAsync(nmid, 0, sizeof(int), st));
+        launch(k_bp_mid, nblk(nl, T), T, 0, st, (const rsg_halo *)H, list, nl, tuning().bp_big,
+               RSG_BP_WARP, mid, nmid);
+        launch(k_bp_dims, (int)std::min<int64_t>(6 * (int64_t)nl, 1216), T, 0, st, W,
+               (const rsg_halo *)H, (const int32_t *)mid, (const int *)nmid, sums);
+        launch(k_basic_props<true>, std::min<int>(nl, 1216), T, 0, st, W, H, (const int32_t *)mid,
+               (const int *)nmid, d_dc, 0, (const double2 *)sums);
+        ar.used = mark;
+    }
+    launch(k_basic_props_w, nblk(nl, 8), 256, 0, st, W, H, list, nl, d_dc);
     int32_t *nch = ar.get<int32_t>(nl + 1), *c0 = ar.get<int32_t>(nl + 1);
     const int bpbig = tuning().bp_big, bpch = tuning().bp_chunk;
     launch(k_bp_nch, nblk(nl + 1, T), T, 0, st, (const rsg_halo *)H, list, nl, bpbig, bpch, nch);
