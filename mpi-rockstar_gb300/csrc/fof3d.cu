@@ -407,7 +407,9 @@ __global__ void __launch_bounds__(RSG_CNT_T) k_count_w(const KNode<3> *nodes, co
 // rounding is monotone, so the sums of their squares in the same order bound
 // the lane's sums.  A point is in S_r(k) when its distance is below r^2, or
 // equal to it when the walk takes one of the point's nodes whole
-// (glist_whole); the bounds used are strict, so equality is always tested.
+// (glist_whole).  So nodes and points whose near bound equals r^2 are kept (a
+// node at r of its particles can lie in the far corner of one taken whole), and
+// only those whose far bound is below it are taken without a test.
 #define RSG_REACH 2.0f
 #define RSG_GE 128           // entries per chunk of a group's list
 #define RSG_GSTK 512
@@ -536,7 +538,7 @@ __global__ void __launch_bounds__(128) k_glist(const KNode<3> *nodes, const Rec 
             float near, far;
             group_bounds(lo, hi, ch.mn, ch.mx, near, far);
             const unsigned in =
-                __ballot_sync(FULL, ch.start + ch.n > kmin + 1 && near < r2) & 3u;
+                __ballot_sync(FULL, ch.start + ch.n > kmin + 1 && near <= r2) & 3u;
             if (in == 3u) break;
             if (in == 0u) {
                 x = -1;
@@ -557,7 +559,7 @@ __global__ void __launch_bounds__(128) k_glist(const KNode<3> *nodes, const Rec 
                 const KNode<3> nd3 = nodes[xi];
                 float near, far;
                 group_bounds(lo, hi, nd3.mn, nd3.mx, near, far);
-                if (nd3.start + nd3.n > kmin + 1 && near < r2) {
+                if (nd3.start + nd3.n > kmin + 1 && near <= r2) {
                     kind = far < r2 ? 1 : (nd3.div < 0 ? 2 : 3);
                     s0 = nd3.start;
                     m0 = nd3.n;
