@@ -466,7 +466,7 @@ __global__ void __launch_bounds__(128) k_glist(const KNode<3> *nodes, const Rec 
     const int g = g0 + ((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     if (g >= g1) return;
     const unsigned below = (1u << lane) - 1u;
-    const float r2 = fmul(r, r), reach = RSG_REACH * r;
+    const float r2 = fmul(r, r), reach = RSG_REACH * fabsf(r);
     int *S = stk[w];
     uint2 *buf = stage[w];
     const bool act = 32 * g + lane < nd;
@@ -484,8 +484,10 @@ __global__ void __launch_bounds__(128) k_glist(const KNode<3> *nodes, const Rec 
         bool mine = (pending >> lane) & 1u;
         float lo[3], hi[3];
 #pragma unroll
-        for (int d = 0; d < 3; d++)
-            mine &= fabsf(fsub(c[d], __shfl_sync(FULL, c[d], lead))) <= reach;
+        for (int d = 0; d < 3; d++) {
+            const float cl = __shfl_sync(FULL, c[d], lead);
+            mine &= lane == lead || fabsf(fsub(c[d], cl)) <= reach;
+        }
 #pragma unroll
         for (int d = 0; d < 3; d++) {
             lo[d] = ord2f(__reduce_min_sync(FULL, mine ? f2ord(c[d]) : 0xffffffffu));
@@ -538,7 +540,7 @@ __global__ void __launch_bounds__(128) k_glist(const KNode<3> *nodes, const Rec 
             float near, far;
             group_bounds(lo, hi, ch.mn, ch.mx, near, far);
             const unsigned in =
-                __ballot_sync(FULL, ch.start + ch.n > kmin + 1 && near <= r2) & 3u;
+                __ballot_sync(FULL, ch.start + ch.n > kmin + 1 && !(near > r2)) & 3u;
             if (in == 3u) break;
             if (in == 0u) {
                 x = -1;
@@ -559,7 +561,7 @@ __global__ void __launch_bounds__(128) k_glist(const KNode<3> *nodes, const Rec 
                 const KNode<3> nd3 = nodes[xi];
                 float near, far;
                 group_bounds(lo, hi, nd3.mn, nd3.mx, near, far);
-                if (nd3.start + nd3.n > kmin + 1 && near <= r2) {
+                if (nd3.start + nd3.n > kmin + 1 && !(near > r2)) {
                     kind = far < r2 ? 1 : (nd3.div < 0 ? 2 : 3);
                     s0 = nd3.start;
                     m0 = nd3.n;
@@ -630,7 +632,7 @@ __global__ void __launch_bounds__(128) k_glist(const KNode<3> *nodes, const Rec 
                             float near, far;
                             group_bounds(lo, hi, p, p, near, far);
                             all = far < r2;
-                            some = !all && near <= r2;
+                            some = !all && !(near > r2);
                         }
                     }
                 }
@@ -649,7 +651,7 @@ __global__ void __launch_bounds__(128) k_glist(const KNode<3> *nodes, const Rec 
                     bool hit = false;
                     if (mine && k < jb) {
                         const float d = dist3_p(cxy, c[2], recs[jb]);
-                        hit = d < r2 || (d == r2 && glist_whole(nodes, xb, c, r, r2));
+                        hit = d < r2 || (!(d > r2) && glist_whole(nodes, xb, c, r, r2));
                     }
                     const unsigned hm = __ballot_sync(FULL, hit);
                     if (lane == b) mask = hm;
