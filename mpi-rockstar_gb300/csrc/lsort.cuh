@@ -5,6 +5,7 @@
 // level-synchronously, many at once; what is left of a segment at or below
 // that size is finished by one block in shared memory.
 #pragma once
+#include "hosttables.cuh"
 #include "kdtree.cuh"
 
 namespace rsg {
@@ -468,14 +469,12 @@ void partition_sort_labels(Arena &ar, T *W, int32_t *lab, int64_t M,
     } h = {{(int32_t)c0.size(), (int32_t)c1.size()}, 0, 0};
     static_assert(offsetof(LsState, ns) == sizeof(Head), "LsState layout");
     // listed segments are disjoint
-    const int32_t nsubs = (int32_t)(ns > 0 ? M : (int64_t)(c0.size() + c1.size()));
+    const int32_t nsubs = ns > 0 ? (int32_t)M : h.nsub[0] + h.nsub[1];
     LsSub *subs = ar.get<LsSub>(nsubs);
-    if (!c0.empty())
-        RSG_CUDA(cudaMemcpyAsync(subs, c0.data(), sizeof(LsSub) * c0.size(),
-                                 cudaMemcpyHostToDevice, st));
-    if (!c1.empty())
-        RSG_CUDA(cudaMemcpyAsync(subs + (nsubs - c1.size()), c1.data(), sizeof(LsSub) * c1.size(),
-                                 cudaMemcpyHostToDevice, st));
+    // with no segment for the rounds nothing below waits for the stream
+    HostTables tables(st);
+    RSG_CUDA(tables.copy(subs, std::move(c0)));
+    RSG_CUDA(tables.copy(subs + (nsubs - h.nsub[1]), std::move(c1)));
     // rounds scatter back and forth between these
     T *wb[2] = {W, nullptr};
     int32_t *lb[2] = {lab, nullptr};
@@ -494,10 +493,11 @@ void partition_sort_labels(Arena &ar, T *W, int32_t *lab, int64_t M,
         LsState *ls = ar.get<LsState>(1);
         const RankBits R = rank_alloc(ar, M, st);
         const int32_t nt = (int32_t)rank_tiles(M);
-        RSG_CUDA(cudaMemcpyAsync(d_roots, roots.data(), sizeof(int2) * ns, cudaMemcpyHostToDevice, st));
+        RSG_CUDA(tables.copy(d_roots, std::move(roots)));
         RSG_CUDA(cudaMemsetAsync(ls, 0, sizeof(LsState), st));
-        RSG_CUDA(cudaMemcpyAsync(ls, &h, sizeof(h), cudaMemcpyHostToDevice, st));
-        RSG_CUDA(cudaMemcpyAsync(&ls->ns[0], &ns, sizeof(ns), cudaMemcpyHostToDevice, st));
+        // Head and ns[0]
+        RSG_CUDA(tables.copy((int32_t *)ls,
+                             std::vector<int32_t>{h.nsub[0], h.nsub[1], 0, 0, ns}));
         RSG_CUDA(cudaMemsetAsync(owner, 0xff, sizeof(int32_t) * M, st));
         launch(k_ls_roots, nblk(ns, 64), 64, 0, st, (const int2 *)d_roots, ns, act[0], range[0]);
         const int64_t y = M / ns / 2048;

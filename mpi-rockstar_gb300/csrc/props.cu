@@ -18,6 +18,7 @@
 #include <cub/cub.cuh>
 
 #include "halo_math.cuh"
+#include "hosttables.cuh"
 #include "kdtree_impl.cuh"
 
 namespace rsg {
@@ -2067,6 +2068,7 @@ void bh_potential(Arena &ar, PotRec *PO, int64_t npo, const int32_t *rs, const i
     }
     BHNode *B = ar.get<BHNode>(F.nnodes);
     int32_t *big = ar.get<int32_t>(F.nnodes);
+    HostTables tables(st);  // to the end: the list of leaves below waits for the stream anyway
     {
         int32_t *arrived = ar.get<int32_t>(F.nnodes);
         RSG_CUDA(cudaMemsetAsync(arrived, 0, sizeof(int32_t) * F.nnodes, st));
@@ -2103,23 +2105,19 @@ void bh_potential(Arena &ar, PotRec *PO, int64_t npo, const int32_t *rs, const i
                 hfirst.push_back((int32_t)hitem.size());
             }
             if (!mid.empty()) {
-                RSG_CUDA(cudaMemcpyAsync(big, mid.data(), 4 * mid.size(), cudaMemcpyHostToDevice,
-                                         st));
-                launch(k_bh_dmin_big, (unsigned)mid.size(), 256, 0, st, F.nodes,
-                       (const int32_t *)big, PO, B, 0);
+                const unsigned nm = (unsigned)mid.size();
+                RSG_CUDA(tables.copy(big, std::move(mid)));
+                launch(k_bh_dmin_big, nm, 256, 0, st, F.nodes, (const int32_t *)big, PO, B, 0);
             }
             if (!hnode.empty()) {
-                const int32_t nh = (int32_t)hnode.size();
-                int2 *d_item = ar.get<int2>(hitem.size());
-                double2 *d_part = ar.get<double2>(hitem.size());
+                const int32_t nh = (int32_t)hnode.size(), ni = (int32_t)hitem.size();
+                int2 *d_item = ar.get<int2>(ni);
+                double2 *d_part = ar.get<double2>(ni);
                 int32_t *d_hnode = ar.get<int32_t>(nh), *d_hfirst = ar.get<int32_t>(nh + 1);
-                RSG_CUDA(cudaMemcpyAsync(d_item, hitem.data(), sizeof(int2) * hitem.size(),
-                                         cudaMemcpyHostToDevice, st));
-                RSG_CUDA(cudaMemcpyAsync(d_hnode, hnode.data(), 4 * nh, cudaMemcpyHostToDevice,
-                                         st));
-                RSG_CUDA(cudaMemcpyAsync(d_hfirst, hfirst.data(), 4 * (nh + 1),
-                                         cudaMemcpyHostToDevice, st));
-                launch(k_bh_huge_part, (unsigned)hitem.size(), 256, 0, st, F.nodes,
+                RSG_CUDA(tables.copy(d_item, std::move(hitem)));
+                RSG_CUDA(tables.copy(d_hnode, std::move(hnode)));
+                RSG_CUDA(tables.copy(d_hfirst, std::move(hfirst)));
+                launch(k_bh_huge_part, (unsigned)ni, 256, 0, st, F.nodes,
                        (const int2 *)d_item, chunk, PO, (const BHNode *)B, d_part);
                 launch(k_bh_huge_fin, nblk(nh, 64), 64, 0, st, F.nodes, (const int32_t *)d_hnode,
                        (const int32_t *)d_hfirst, nh, (const double2 *)d_part, B);
