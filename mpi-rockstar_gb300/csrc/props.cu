@@ -20,6 +20,7 @@
 #include "halo_math.cuh"
 #include "hosttables.cuh"
 #include "kdtree_impl.cuh"
+#include "widths.cuh"
 
 namespace rsg {
 
@@ -235,7 +236,8 @@ __global__ void k_bh_climb(const KNode<3> *nodes, int32_t nn, const PotRec *PO, 
 template <int EXACT>
 __global__ void __launch_bounds__(256) k_bh_dmin(const KNode<3> *nodes, int32_t nn,
                                                  const PotRec *PO, BHNode *B) {
-    const int a = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    const int64_t a = warp_index(blockIdx.x, blockDim.x, threadIdx.x);
+    const int lane = threadIdx.x & 31;
     if (a >= nn) return;
     const KNode<3> &x = nodes[a];
     if (x.div < 0 || x.n > RSG_BH_BIG) return;
