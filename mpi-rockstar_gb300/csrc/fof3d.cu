@@ -32,6 +32,7 @@
 #include "kdtree_impl.cuh"
 #include "lsort.cuh"
 #include "uflabels.cuh"
+#include "widths.cuh"
 
 namespace rsg {
 
@@ -423,7 +424,8 @@ struct __align__(16) GChunk {
 struct GLists {
     GChunk *pool;
     int cap;                 // chunks of the pool
-    int *cursor;             // chunks asked for (more than cap: lists are cut)
+    unsigned *cursor;        // hands the chunks out; those asked for beyond cap are not
+                             // kept, so it may pass any width (see has_place)
     int *nch;                // chunks per group
 };
 // Whether the reference's walk takes a node holding leaf x whole for the
@@ -500,10 +502,10 @@ __global__ void __launch_bounds__(128) k_glist(const KNode<3> *nodes, const Rec 
         int ne = 0, ns = 0, chunk = -1;  // entries in the chunk, staged; the chunk
         auto flush = [&](int m) {        // the first m <= 32 staged entries
             if (ne == RSG_GE || ne == 0) {
-                int nc = 0;
-                if (lane == 0) nc = atomicAdd(G.cursor, 1);
+                unsigned nc = 0;
+                if (lane == 0) nc = atomicAdd(G.cursor, 1u);
                 nc = __shfl_sync(FULL, nc, 0);
-                lost |= nc >= G.cap;
+                lost |= !has_place(nc, G.cap);
                 if (lane == 0 && !lost) {
                     if (ne == RSG_GE) G.pool[chunk].n = RSG_GE;
                     G.pool[nc].mask = run;
@@ -511,7 +513,7 @@ __global__ void __launch_bounds__(128) k_glist(const KNode<3> *nodes, const Rec 
                     G.pool[nc].ord = nch;
                 }
                 nch++;
-                chunk = nc;
+                chunk = (int)nc;
                 ne = 0;
             }
             if (!lost && lane < m) G.pool[chunk].e[ne + lane] = buf[lane];
@@ -1517,10 +1519,10 @@ FofOut fof3d_device(Arena &ar, const rsg_particle *d_in, int64_t n64, const rsg_
     cub::DeviceReduce::Max(nullptr, mb, gn, gm, ng + 1, st);
     const size_t gtb = (sb > mb ? sb : mb) + 256;
     void *gtmp = ar.take(gtb);
-    // {chunks asked for, pairs}
+    // {cursor, pairs}
     unsigned long long *tot = ar.get<unsigned long long>(2);
     RSG_CUDA(cudaMemsetAsync(tot, 0, 2 * sizeof(*tot), st));
-    KL.G.cursor = (int *)tot;
+    KL.G.cursor = (unsigned *)tot;
     // The lists go to the arena beside what the rest of the FOF takes from it
     // (< 256 B per particle: the label derivation and the partition sort).
     // Lists that do not fit (very dense snapshots) get an allocation of
@@ -1547,14 +1549,13 @@ FofOut fof3d_device(Arena &ar, const rsg_particle *d_in, int64_t n64, const rsg_
            (const uint8_t *)cnt, (const int *)dpfx, KL.G, skip, diff, tot + 1, err);
     if (nd > 0) cub::DeviceScan::InclusiveSum(dst_tmp, dsb, diff, diff, nd + 1, st);
     launch(k_kahn_init, nblk(nd, T), T, 0, st, nd, (const int *)diff, skip, KL.und);
-    unsigned long long htot[2] = {0, 0};
-    RSG_CUDA(cudaMemcpyAsync(htot, tot, sizeof(htot), cudaMemcpyDeviceToHost, st));
-    RSG_CUDA(cudaStreamSynchronize(st));
-    const int64_t nch = (int64_t)(uint32_t)htot[0];  // chunks the lists take
-    const int64_t ne = (int64_t)htot[1];
     launch(k_gchunks, nblk(ng + 1, T), T, 0, st, (const int *)KL.G.nch, ng, gn);
     sb = mb = gtb;
     cub::DeviceScan::ExclusiveSum(gtmp, sb, gn, go, ng + 1, st);
+    int64_t nch = 0, ne = 0;  // chunks that the lists take, pairs
+    RSG_CUDA(cudaMemcpyAsync(&nch, go + ng, sizeof(nch), cudaMemcpyDeviceToHost, st));
+    RSG_CUDA(cudaMemcpyAsync(&ne, tot + 1, sizeof(ne), cudaMemcpyDeviceToHost, st));
+    RSG_CUDA(cudaStreamSynchronize(st));
     // chunk boundaries: groups c[t] .. c[t+1], the chunks of their lists
     std::vector<int> cb_h(2, 0);
     std::vector<int64_t> lb_h(2, 0);

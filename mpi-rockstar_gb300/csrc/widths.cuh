@@ -14,4 +14,11 @@ __host__ __device__ __forceinline__ int64_t warp_index(unsigned block, unsigned 
     return ((int64_t)block * threads + thread) >> 5;
 }
 
+// Whether a place that a counter handed out lies in a pool of `cap`.  The
+// counter also counts what finds no room, past 2^31 for the lists of very dense
+// snapshots: as an int such a place is negative and below every cap.
+__host__ __device__ __forceinline__ bool has_place(unsigned place, int cap) {
+    return cap > 0 && place < (unsigned)cap;
+}
+
 }  // namespace rsg
