@@ -17,8 +17,8 @@
 //     rotated down by one (the front pointer stops at m and swaps it with
 //     each tail element in turn).
 // Every element's destination is therefore a function of per-node prefix
-// counts of the "big" flag, which one global scan provides for all nodes of
-// a level at once.  Degenerate nodes (max == min on the split dimension) get
+// counts of the "big" flag, which are kept as bits with the counts before
+// every word and tile (RankBits) for all nodes of a level at once.  Degenerate nodes (max == min on the split dimension) get
 // lim = +inf so nothing moves, as in the reference's early return.
 #pragma once
 #include <cub/cub.cuh>

@@ -95,8 +95,8 @@ __device__ __forceinline__ void sub_box(unsigned (*cbox)[2][2 * D], const float 
 // moved once at the end.  Its cost is the chain of a level's six block
 // barriers (about 1 us a level), hidden by the other blocks of the SM; a
 // level of the loop below reads and writes every record of the call and
-// costs at least fourteen launches, and the levels below 2048 records are
-// half or more of a build's.  2048 records are what leaves room for three
+// costs five launches, and the levels below 2048 records are half or more of a
+// build's.  2048 records are what leaves room for three
 // blocks an SM in 3D (70 KB) and two in 6D (83 KB); 256-record subtrees, the
 // bulk of the 6D forests, run sixteen to an SM.
 // Children are numbered in the order the blocks allocate them: a node's two
@@ -155,7 +155,7 @@ __global__ void __launch_bounds__(T) k_sub_build(RecT *out, const RecT *scratch,
         const int nact = h.nact;
         if (nact == 0) break;
         level++;
-        // split dimension and limit (src/fast3tree.c:736-757), as k_prep
+        // split dimension and limit (src/fast3tree.c:736-757), as split_of
         for (int k = t; k < nact; k += T) {
             const float *bx = h.box[cur][k];
             int dim = D - 1;
